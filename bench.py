@@ -344,7 +344,7 @@ def main():
     launches = sum(sum(int(x) for x in s.kernel_launches) + int(s.step_launches) + 2 for s in stats)
     # roofline of the dominant kernel: one more step of the same workload with CUDA events
     # between the kernels of every iteration (event nodes inside the captured graphs); the tail
-    # iterations run k_steps ("steps" in the shares), the others the six queue kernels
+    # iterations run k_block ("steps" in the shares), the others the six queue kernels
     flush.zero_()
     prof = [step(prec, profile=1)]
     torch.cuda.synchronize()

@@ -1,0 +1,342 @@
+// cm_block.cuh -- the resident-steps kernel (included by cm_engine.cu).
+//
+// k_block holds each block's electrons in shared memory and takes them through many steps per launch.  An
+// iteration is one list of tasks of up to 32 electrons each, which the block's warps take one after
+// another: the flights, by wave segment (one material and energy band per warp), each with the elastic
+// event it ends in, and the inelastic and misc events queued by the iteration before.  What an iteration
+// appends is the next one's lists, so a warp runs one kind of work at a time although a thread sees every
+// kind, and secondaries start at once in the slots of electrons that ended.
+//
+// It runs where few electrons are left: there the queue kernels cost ~55 us an iteration (six launches and
+// their serial latency) however few electrons they move, and one electron per thread through whole steps
+// leaves a warp's lanes in different events (measured before this kernel: 26 M steps of a 3 keV scan with
+// phonons 61 ms, now 20 ms; the last 256 k electrons of a 500 eV line scan 12.3 -> 7.7 ms in FP32, 42 ->
+// 23 ms in FP64).  With the GPU full the queue kernels move 3.8 G electron-steps/s and this kernel 2.3 G
+// (16 warps per SM against their 24 and more), so they keep the full waves.
+//
+#pragma once
+
+namespace cm {
+
+#ifndef CM_BLOCK_THREADS
+#define CM_BLOCK_THREADS 512
+#endif
+#ifndef CM_BLOCK_MINB
+#define CM_BLOCK_MINB 1
+#endif
+#ifndef CM_BLOCK_SLOTS
+#define CM_BLOCK_SLOTS 1024
+#endif
+
+constexpr int kBlockThreads = CM_BLOCK_THREADS;
+constexpr int kBlockSlots = CM_BLOCK_SLOTS;
+constexpr int kBlockPerSm = CM_BLOCK_MINB;
+// lists a slot can be in: the flights of each wave segment, the inelastic and the misc events
+constexpr int kListTab = kSegments, kListMisc = kSegments + 1, kListDead = kSegments + 2, kLists = kSegments + 3;
+constexpr int kListNone = kLists;
+// iterations after which a block passes what is left of the wave on to the next one instead of taking it
+constexpr int kBlockHardLimit = 4096;
+
+// control words of a block
+struct BlockCtl {
+  int cnt[2][kLists];  // entries of each list, this iteration's and the next one's
+  int nfree;           // free slots (free_slot[0..nfree))
+  int taken;           // of which secondaries have taken, from the top
+  int task;            // next task of the iteration
+  int claim_base, claim_n;
+  int exhausted;       // the wave has no electron left to take
+};
+
+// The block's electrons: structure of arrays over its slots, in shared memory.
+template <typename R>
+struct BlockMem {
+  double *px, *py, *pz;
+  unsigned long long* key;
+  R *dx, *dy, *dz, *E, *Ep, *hx, *hy, *hz;
+  int *region, *pixel, *aux;
+  uint32_t* step;
+  unsigned short* list[2];  // [kLists][kBlockSlots] each
+  unsigned short* free_slot;
+  unsigned char* born;      // the slot holds a secondary started in this launch
+  BlockCtl* ctl;
+
+  static constexpr size_t bytes() {
+    return (size_t)kBlockSlots * (4 * 8 + 8 * sizeof(R) + 4 * 4 + 2 * kLists * 2 + 2 + 1) + sizeof(BlockCtl) + 64;
+  }
+  __device__ __forceinline__ explicit BlockMem(unsigned char* p) {
+    constexpr size_t n = kBlockSlots;
+    px = (double*)p; py = px + n; pz = py + n;
+    key = (unsigned long long*)(pz + n);
+    dx = (R*)(key + n); dy = dx + n; dz = dy + n; E = dz + n; Ep = E + n; hx = Ep + n; hy = hx + n; hz = hy + n;
+    region = (int*)(hz + n); pixel = region + n; aux = pixel + n;
+    step = (uint32_t*)(aux + n);
+    ctl = (BlockCtl*)(step + n);
+    list[0] = (unsigned short*)(ctl + 1);
+    list[1] = list[0] + kLists * n;
+    free_slot = list[1] + kLists * n;
+    born = (unsigned char*)(free_slot + n);
+  }
+  __device__ __forceinline__ El<R> load(int i) const {
+    El<R> e;
+    e.p[0] = px[i]; e.p[1] = py[i]; e.p[2] = pz[i];
+    e.d[0] = dx[i]; e.d[1] = dy[i]; e.d[2] = dz[i];
+    e.E = E[i];
+    e.region = region[i]; e.pixel = pixel[i];
+    e.step = step[i]; e.key = key[i];
+    return e;
+  }
+  __device__ __forceinline__ void store(int i, const El<R>& e) const {
+    px[i] = e.p[0]; py[i] = e.p[1]; pz[i] = e.p[2];
+    dx[i] = e.d[0]; dy[i] = e.d[1]; dz[i] = e.d[2];
+    E[i] = e.E;
+    region[i] = e.region; pixel[i] = e.pixel;
+    step[i] = e.step; key[i] = e.key;
+  }
+  __device__ __forceinline__ void put(int par, int l, int slot) const {
+    list[par][l * kBlockSlots + atomicAdd(&ctl->cnt[par][l], 1)] = (unsigned short)slot;
+  }
+};
+
+// secondaries take a free slot of the block, or go to the run's pool when there is none
+template <typename R>
+struct BlockSink : DeviceSink {
+  const BlockMem<R>& b;
+  int par;  // parity of the lists being filled
+  __device__ __forceinline__ BlockSink(const BlockMem<R>& m, int p) : b(m), par(p) {}
+  __device__ __forceinline__ bool put_secondary(const RunView<R>& v, const El<R>& se) {
+    const int k = atomicAdd(&b.ctl->taken, 1), avail = b.ctl->nfree;
+    if (k >= avail) return pool_push(v, se, *this);
+    const int slot = b.free_slot[avail - 1 - k];
+    b.store(slot, se);
+    b.born[slot] = 1;
+    b.put(par, wave_segment(v.s, se.region, se.E), slot);
+    return true;
+  }
+};
+
+// One task: up to 32 electrons of one list through their flight (with the elastic event it ends in) or
+// their queued event.  Every lane of the warp calls it; lanes without an electron have slot < 0.
+template <typename R, int D>
+__device__ __forceinline__ void block_task(const RunView<R>& v, const BlockMem<R>& b, int l, int slot, BlockSink<R>& sink,
+                                           StepCounts& sc) {
+  int dest = kListNone;
+  if (slot >= 0) {
+    El<R> e = b.load(slot);
+    bool alive;
+    dest = kListDead;
+    if (l < kSegments) {
+      const int q = flight_apply<R, D>(v, e, sink, sc);
+      alive = q >= 0;
+      if (q == Q_EL) alive = elastic_apply(v, e);
+      if (alive) {
+        b.px[slot] = e.p[0]; b.py[slot] = e.p[1]; b.pz[slot] = e.p[2];
+        b.E[slot] = e.E;
+        b.region[slot] = e.region;
+        b.step[slot] = e.step;
+        if (q == Q_EL) {
+          b.dx[slot] = e.d[0]; b.dy[slot] = e.d[1]; b.dz[slot] = e.d[2];
+        } else {
+          b.Ep[slot] = e.Ep;
+          b.aux[slot] = e.aux;
+          if (aux_kind(e.aux) == AUX_BARRIER) { b.hx[slot] = e.h[0]; b.hy[slot] = e.h[1]; b.hz[slot] = e.h[2]; }
+        }
+        dest = q == Q_EL ? wave_segment(v.s, e.region, e.E) : q == Q_TAB ? kListTab : kListMisc;
+      }
+    } else {
+      e.Ep = b.Ep[slot];
+      e.aux = b.aux[slot];
+      if (l == kListTab) {
+        alive = inelastic_apply(v, e, sink, sc);
+      } else {
+        e.h[0] = b.hx[slot]; e.h[1] = b.hy[slot]; e.h[2] = b.hz[slot];
+        alive = misc_apply<R, D>(v, e, sink, sc);
+        if (alive) {
+          b.px[slot] = e.p[0]; b.py[slot] = e.p[1]; b.pz[slot] = e.p[2];
+          b.region[slot] = e.region;
+        }
+      }
+      if (alive) {
+        b.dx[slot] = e.d[0]; b.dy[slot] = e.d[1]; b.dz[slot] = e.d[2];
+        b.E[slot] = e.E;
+        dest = wave_segment(v.s, e.region, e.E);
+      }
+    }
+    if (!alive) job_end(v, e.pixel, e.step, sink);
+  }
+  // append the slots to their lists: one shared-memory atomic per list and warp
+  __syncwarp();
+  const unsigned same = __match_any_sync(0xffffffffu, dest);
+  const int lane = threadIdx.x & 31, leader = __ffs(same) - 1;
+  int base = 0;
+  if (dest != kListNone && lane == leader) base = atomicAdd(&b.ctl->cnt[sink.par][dest], __popc(same));
+  base = __shfl_sync(0xffffffffu, base, leader);
+  if (dest != kListNone)
+    b.list[sink.par][dest * kBlockSlots + base + __popc(same & ((1u << lane) - 1))] = (unsigned short)slot;
+}
+
+// The tasks of an iteration: 32 entries of one list each, events first (they take longest).  events_only:
+// the flights stay in their lists.
+template <typename R, int D>
+__device__ __forceinline__ void block_stage(const RunView<R>& v, const BlockMem<R>& b, int par, bool events_only,
+                                            BlockSink<R>& sink, StepCounts& sc) {
+  const int lane = threadIdx.x & 31;
+  for (;;) {
+    int t = 0;
+    if (lane == 0) t = atomicAdd(&b.ctl->task, 1);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    int l = kListTab, n;
+    for (;;) {  // the list this task falls in: inelastic, misc, then the segments
+      n = b.ctl->cnt[par][l];
+      const int k = (n + 31) >> 5;
+      if (t < k) break;
+      t -= k;
+      if (l == kListTab) l = kListMisc;
+      else if (l == kListMisc) {
+        if (events_only) return;
+        l = 0;
+      } else if (++l == kSegments) return;
+    }
+    const int i = 32 * t + lane;
+    const int slot = i < n ? (int)b.list[par][l * kBlockSlots + i] : -1;
+    block_task<R, D>(v, b, l, slot, sink, sc);
+  }
+}
+
+// Electrons of wave `cur` through about `iters` iterations (a flight with its elastic event, or a queued
+// event, per electron and iteration), survivors kept in the next wave.  cap: slots a block may use.
+template <typename R, int D>
+__global__ void __launch_bounds__(kBlockThreads, kBlockPerSm) k_block(RunView<R> v, int cur, int iters, int cap) {
+  const BlockMem<R> b(cm_stage_smem);
+  BlockCtl* c = b.ctl;
+  const int n = v.c->n[cur];
+  const int grid = gridDim.x, tid = threadIdx.x, T = kBlockThreads;
+  if (n == 0) return;
+  __shared__ int first[kSegments + 1];
+  segment_starts(v.c, cur, first);
+  // The first share: every block takes the same number of electrons, in runs of `run` from all over the
+  // wave, so that the blocks get like mixes of materials and energies
+  const int reserve = cap / 8;
+  int quota = (n + grid - 1) / grid;
+  const int run = quota >= 64 ? 8 : 1;
+  quota = (quota + run - 1) / run * run;
+  if (quota > cap - reserve) quota = (cap - reserve) / run * run;
+  const long long dealt = (long long)quota * grid;
+  for (int i = tid; i < cap; i += T) b.free_slot[i] = (unsigned short)(cap - 1 - i);
+  for (int i = tid; i < 2 * kLists; i += T) (&c->cnt[0][0])[i] = 0;
+  __syncthreads();
+  int mine = 0;  // electrons of the share that exist
+  {
+    // slots [0, quota) of the share; slot j holds electron (j / run * grid + block) * run + j % run
+    const int whole = n / (run * grid) * run;
+    const int rest = n - n / (run * grid) * (run * grid) - (int)blockIdx.x * run;
+    mine = whole + (rest < 0 ? 0 : rest > run ? run : rest);
+    if (mine > quota) mine = quota;
+  }
+  auto take = [&](int i, int slot, int par) {
+    const int k = segment_of(first, i);
+    const El<R> e = load_live(v.w[cur], k * v.W + (i - first[k]));
+    b.store(slot, e);
+    b.born[slot] = 0;
+    b.put(par, wave_segment(v.s, e.region, e.E), slot);
+  };
+  for (int j = tid; j < mine; j += T) take((j / run * grid + (int)blockIdx.x) * run + j % run, j, 0);
+  if (tid == 0) {
+    c->nfree = cap - mine;
+    c->taken = 0;
+    c->task = 0;
+    c->claim_n = 0;
+    c->exhausted = dealt >= n;
+  }
+  __syncthreads();
+  StepCounts sc;
+  int par = 0, it = 0;
+  for (;; ++it) {
+    // the last iteration runs the queued events only, so that every electron ends between two steps
+    const bool out = c->exhausted != 0;
+    const bool last = (c->nfree == cap && out) || (it >= iters && out) || it >= kBlockHardLimit;
+    BlockSink<R> sink(b, par ^ 1);
+    block_stage<R, D>(v, b, par, last, sink, sc);
+    __syncthreads();
+    if (last) break;
+    // free slots: those the secondaries took are gone, those of the electrons that ended come back
+    const int avail = c->nfree, tk = c->taken < avail ? c->taken : avail, nd = c->cnt[par ^ 1][kListDead];
+    for (int i = tid; i < nd; i += T) b.free_slot[avail - tk + i] = b.list[par ^ 1][kListDead * kBlockSlots + i];
+    __syncthreads();
+    if (tid < kLists) c->cnt[par][tid] = 0;
+    if (tid == 0) {
+      const int nf = avail - tk + nd, want = nf - reserve;
+      int m = 0;
+      if (!out && (want >= 32 || nf == cap)) {
+        const long long base = dealt + atomicAdd(&v.c->claim, want);
+        m = base >= n ? 0 : (n - base < want ? (int)(n - base) : want);
+        c->claim_base = (int)base;
+        if (base + want >= n) c->exhausted = 1;
+      }
+      c->claim_n = m;
+      c->nfree = nf - m;
+      c->taken = 0;
+      c->task = 0;
+      c->cnt[par ^ 1][kListDead] = 0;
+    }
+    __syncthreads();
+    const int m = c->claim_n;
+    if (m > 0) {
+      for (int i = tid; i < m; i += T) take(c->claim_base + i, b.free_slot[c->nfree + i], par ^ 1);
+      __syncthreads();
+    }
+    par ^= 1;
+  }
+  // every electron that is left goes to the next wave (secondaries started here to the pool, whose refill
+  // keeps the wave within its bound)
+  {
+    DeviceSink sink;
+    for (int h = 0; h < 2; ++h)
+      for (int l = 0; l < kSegments; ++l) {
+        const int p = par ^ h, k = c->cnt[p][l];
+        for (int i = tid; i < k; i += T) {
+          const int slot = b.list[p][l * kBlockSlots + i];
+          const El<R> e = b.load(slot);
+          if (b.born[slot]) pool_push(v, e, sink);
+          else keep(v, cur ^ 1, e, sink);
+        }
+      }
+    // a wave this launch did not get through is passed on as it is
+    while (!c->exhausted) {
+      __syncthreads();
+      if (tid == 0) {
+        const long long base = dealt + atomicAdd(&v.c->claim, 4096);
+        c->claim_n = base >= n ? 0 : (n - base < 4096 ? (int)(n - base) : 4096);
+        c->claim_base = (int)base;
+        if (base + 4096 >= n) c->exhausted = 1;
+      }
+      __syncthreads();
+      for (int i = tid; i < c->claim_n; i += T) {
+        const int w = c->claim_base + i, k = segment_of(first, w);
+        keep(v, cur ^ 1, load_live(v.w[cur], k * v.W + (w - first[k])), sink);
+      }
+      __syncthreads();
+    }
+  }
+  flush_counts(v.c, sc);
+}
+
+// Slots per block: all of them, or fewer for a small wave, so that the blocks together hold about a wave of
+// electrons at most: the secondary pool is sized by the wave, and what the blocks hold may end in it.
+static int block_cap(int W, int grid) {
+  const int cap = W / grid;
+  return cap > kBlockSlots ? kBlockSlots : cap < 1 ? 1 : cap;
+}
+
+template <typename R, int D> static void launch_block_d(const RunView<R>& v, int cur, int nsm, int iters, cudaStream_t s) {
+  const int grid = nsm * kBlockPerSm;
+  cudaFuncSetAttribute(k_block<R, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BlockMem<R>::bytes());
+  k_block<R, D><<<grid, kBlockThreads, BlockMem<R>::bytes(), s>>>(v, cur, iters, block_cap(v.W, grid));
+}
+
+template <typename R> static void launch_block(const RunView<R>& v, int cur, int nsm, int iters, cudaStream_t s) {
+  if (v.s.depth == 0) launch_block_d<R, 0>(v, cur, nsm, iters, s);
+  else if (v.s.depth <= 2) launch_block_d<R, 2>(v, cur, nsm, iters, s);
+  else launch_block_d<R, kMaxShapeDepth>(v, cur, nsm, iters, s);
+}
+
+}  // namespace cm

@@ -826,6 +826,10 @@ struct DeviceSink {
     const unsigned long long sum = cg::reduce(part, value, cg::plus<unsigned long long>());
     if (part.thread_rank() == 0) atomicAdd(counters + idx, sum);
   }
+  // secondaries go to the run's pool
+  template <typename R> __device__ __forceinline__ bool put_secondary(const RunView<R>& v, const El<R>& se) {
+    return pool_push(v, se, *this);
+  }
   __device__ __forceinline__ unsigned long long ticket(unsigned long long* c) { return atomicAdd(c, 1ull); }
   __device__ __forceinline__ void error(int* e, int code) { atomicExch(e, code); }
 };
@@ -869,23 +873,15 @@ template <typename R> __device__ __forceinline__ bool stage_tables(const RunView
 }
 
 __device__ __forceinline__ void flush_counts(Counters* c, StepCounts& sc) {
-  for (int off = 16; off > 0; off >>= 1) {
-    sc.steps += __shfl_down_sync(0xffffffffu, sc.steps, off);
-    sc.scat += __shfl_down_sync(0xffffffffu, sc.scat, off);
-    sc.bar += __shfl_down_sync(0xffffffffu, sc.bar, off);
-    sc.esc += __shfl_down_sync(0xffffffffu, sc.esc, off);
-    sc.sec += __shfl_down_sync(0xffffffffu, sc.sec, off);
-    sc.zero += __shfl_down_sync(0xffffffffu, sc.zero, off);
-    sc.limit += __shfl_down_sync(0xffffffffu, sc.limit, off);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    if (sc.steps) atomicAdd(&c->steps, sc.steps);
-    if (sc.scat) atomicAdd(&c->scatters, sc.scat);
-    if (sc.bar) atomicAdd(&c->barriers, sc.bar);
-    if (sc.esc) atomicAdd(&c->escapes, sc.esc);
-    if (sc.sec) atomicAdd(&c->secondaries, sc.sec);
-    if (sc.zero) atomicAdd(&c->ended_zero, sc.zero);
-    if (sc.limit) atomicAdd(&c->ended_limit, sc.limit);
+  // a thread counts one launch's steps in 32 bits; the warp's sums and the run's totals are 64-bit
+  const unsigned int mine[7] = {sc.steps, sc.scat, sc.bar, sc.esc, sc.sec, sc.zero, sc.limit};
+  unsigned long long* const total[7] = {&c->steps,       &c->scatters,   &c->barriers,   &c->escapes,
+                                        &c->secondaries, &c->ended_zero, &c->ended_limit};
+#pragma unroll
+  for (int k = 0; k < 7; ++k) {
+    unsigned long long sum = mine[k];
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, off);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(total[k], sum);
   }
 }
 
@@ -929,7 +925,7 @@ template <typename R, int D> __global__ void __launch_bounds__(256) k_flight(Run
   flight_loop<R, D>(v, cur);
 }
 
-// Kernels that stage the small tables into shared memory (1 flight, 2 elastic, 4 inelastic, 8 steps) and
+// Kernels that stage the small tables into shared memory (1 flight, 2 elastic, 4 inelastic) and
 // the inelastic grid in blocks per SM when it stages.  k_inelastic gathers ~130 table values per event
 // (cubic interpolation in the 2-D energy-loss and SE tables and the 3-D angle table); staged into the
 // shared memory of a grid of 2 resident blocks per SM it gains 1 % on the linescan.  Staging in the
@@ -1011,41 +1007,18 @@ static void launch_flight(const RunView<float>& v, int cur, int grid, cudaStream
   else k_flight<float, kMaxShapeDepth><<<grid, 256, smem, s>>>(v, cur);
 }
 
-// The tail of a run: once fewer electrons are left than fill the GPU, each thread takes one electron
-// through CM_TAIL_STEPS whole steps per iteration (k_steps) instead of one step through the queue
+// The tail of a run: once fewer electrons are left than fill the GPU, the blocks of k_block take them
+// through CM_TAIL_STEPS iterations per launch in shared memory instead of one step through the queue
 // kernels, whose launches and queue traffic then cost more than the steps themselves.
 #ifndef CM_TAIL_BELOW
 #define CM_TAIL_BELOW 262144
 #endif
 #ifndef CM_TAIL_STEPS
-#define CM_TAIL_STEPS 32
+#define CM_TAIL_STEPS 64
 #endif
-#if defined(CM_MINB_STEPS)
-#define CM_LB_STEPS __launch_bounds__(256, CM_MINB_STEPS)
-#else
-#define CM_LB_STEPS __launch_bounds__(256)
-#endif
-
-template <typename R, int D> __global__ void CM_LB_STEPS k_steps(RunView<R> v, int cur, int nsteps) {
-  DeviceSink sink;
-  StepCounts sc;
-  const int n = v.c->n[cur];
-  if ((int)(blockIdx.x * blockDim.x) >= n || !stage_tables(v)) return;
-  __shared__ int first[kSegments + 1];
-  segment_starts(v.c, cur, first);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int k = segment_of(first, i);
-    steps_one<R, D>(v, cur, k * v.W + (i - first[k]), nsteps, sink, sc);
-  }
-  flush_counts(v.c, sc);
-}
-
-template <typename R>
-static void launch_steps(const RunView<R>& v, int cur, int grid, int nsteps, cudaStream_t s, size_t smem) {
-  if (v.s.depth == 0) k_steps<R, 0><<<grid, 256, smem, s>>>(v, cur, nsteps);
-  else if (v.s.depth <= 2) k_steps<R, 2><<<grid, 256, smem, s>>>(v, cur, nsteps);
-  else k_steps<R, kMaxShapeDepth><<<grid, 256, smem, s>>>(v, cur, nsteps);
-}
+}  // namespace cm
+#include "cm_block.cuh"
+namespace cm {
 
 // the launch settings a run uses: the context's tuning, built-in defaults where it holds 0
 template <typename R> static cm_tuning resolved_tuning(const cm_context* ctx) {
@@ -1090,7 +1063,7 @@ __global__ void k_tail(RunView<R> v, int cur, int steps) {
 // does and then sets the condition of the conditional node it runs under: another iteration, or not when
 // the run is done or failed (a device error, the iteration limit, a cancel flag set by the host), and for
 // the queue loop also once every primary has started and fewer electrons are left than io.tail_below
-// (the tail loop of whole steps per thread takes over).  Iterations of a loop body after its end do no
+// (the tail loop of k_block takes over).  Iterations of a loop body after its end do no
 // work: their kernels find no electrons.
 template <typename R>
 __global__ void k_loop(RunView<R> v, int cur, int steps, cudaGraphConditionalHandle h) {
@@ -1232,10 +1205,9 @@ static void launch_queue_iteration(const cm_context* ctx, const RunView<R>& v, c
 }
 
 template <typename R>
-static void launch_tail_iteration(const RunView<R>& v, const RunView<R>& vs, int cur, int grid, int tail_steps,
-                                  size_t smem, cudaStream_t s, cudaGraphConditionalHandle* h, cudaEvent_t* ev) {
-  if (CM_STAGE_KERNELS & 8) launch_steps(vs, cur, grid, tail_steps, s, smem);
-  else launch_steps(v, cur, grid, tail_steps, s, 0);
+static void launch_tail_iteration(const cm_context* ctx, const RunView<R>& v, int cur, int grid, int tail_steps,
+                                  cudaStream_t s, cudaGraphConditionalHandle* h, cudaEvent_t* ev) {
+  launch_block(v, cur, ctx->nsm, tail_steps, s);
   if (ev) cudaEventRecordWithFlags(ev[0], s, cudaEventRecordExternal);
   launch_spawn<R>(v, cur, grid, s);
   if (ev) cudaEventRecordWithFlags(ev[1], s, cudaEventRecordExternal);
@@ -1290,7 +1262,7 @@ static int build_loop_graph(cm_context* ctx, RunBuffers<R>& rb, const RunView<R>
       return bail(e, "cudaStreamBeginCaptureToGraph");
     for (int it = 0; it < kLoopBody; ++it) {
       if (loop == 0) launch_queue_iteration<R>(ctx, v, vs, it & 1, grid, smem, ctx->cap_stream, &hh, nullptr);
-      else launch_tail_iteration<R>(v, vs, it & 1, grid, tail_steps, smem, ctx->cap_stream, &hh, nullptr);
+      else launch_tail_iteration<R>(ctx, v, it & 1, grid, tail_steps, ctx->cap_stream, &hh, nullptr);
     }
     cudaGraph_t captured = nullptr;
     if ((e = cudaStreamEndCapture(ctx->cap_stream, &captured)) != cudaSuccess) return bail(e, "cudaStreamEndCapture");
@@ -1454,7 +1426,7 @@ static int run_device_once(cm_context* ctx, const cm_run_desc* d, uint32_t* back
       cudaEventRecordWithFlags(ev[0], stream, cudaEventRecordExternal);
       for (int it = 0; it < K; ++it) {
         if (loop == 0) launch_queue_iteration<R>(ctx, v, vs, it & 1, grid, smem, stream, nullptr, &pev[(size_t)it * 6 + 1]);
-        else launch_tail_iteration<R>(v, vs, it & 1, grid, tu.tail_steps, smem, stream, nullptr, &tev[(size_t)it * 3 + 1]);
+        else launch_tail_iteration<R>(ctx, v, it & 1, grid, tu.tail_steps, stream, nullptr, &tev[(size_t)it * 3 + 1]);
       }
       CM_CUDA(cudaStreamEndCapture(stream, &graph[loop]));
       CM_CUDA(cudaGraphInstantiate(&exec[loop], graph[loop], 0));
@@ -2537,7 +2509,7 @@ int cm_autotune(cm_context* ctx, const cm_run_desc* d, cm_tuning* best) {
     return rc;
   }
   const int belows[] = {65536, 131072, 524288};
-  const int steps[] = {16, 64};
+  const int steps[] = {32, 128};
   auto sweep = [&](int cm_tuning::*field, const int* vals, int n) -> int {
     for (int k = 0; k < n; ++k) {
       if (vals[k] == cur.*field) continue;

@@ -17,7 +17,7 @@
 // on their own.
 //
 // The batcher replays captured rounds of transport iterations (the queue kernels while the wave is full,
-// the several-steps kernel in the tail) and between rounds admits jobs, reads the counters and finishes
+// the resident-steps kernel in the tail) and between rounds admits jobs, reads the counters and finishes
 // jobs.  When the batch runs empty its scene and tables are dropped, so memory stays bounded.
 #pragma once
 
@@ -429,7 +429,7 @@ static int batch_round(Batcher& b) {
     hc.total_primaries = b.total;
     hc.done = 0;
   }
-  // several whole steps per thread (the tail kernels) whenever fewer electrons are in the wave and pool than
+  // many steps per launch (the tail kernels) whenever fewer electrons are in the wave and pool than
   // fill the GPU, even with primaries still to start; the refill then fills the wave only up to that many,
   // so a light load runs at the latency of a job alone and a heavy one through the queue kernels
   const long long left = (long long)hc.n[0] + hc.n[1] + std::min(hc.pool, v.poolCap);
@@ -449,7 +449,7 @@ static int batch_round(Batcher& b) {
       CM_CUDA(cudaStreamBeginCapture(ctx->cap_stream, cudaStreamCaptureModeThreadLocal));
       for (int it = 0; it < kLoopBody; ++it) {
         if (loop == 0) launch_queue_iteration<R>(ctx, v, vs, it & 1, grid, smem, ctx->cap_stream, nullptr, nullptr);
-        else launch_tail_iteration<R>(v, vs, it & 1, grid, tu.tail_steps, smem, ctx->cap_stream, nullptr, nullptr);
+        else launch_tail_iteration<R>(ctx, v, it & 1, grid, tu.tail_steps, ctx->cap_stream, nullptr, nullptr);
       }
       CM_CUDA(cudaStreamEndCapture(ctx->cap_stream, &b.round_graph[loop]));
       CM_CUDA(cudaGraphInstantiate(&b.round_exec[loop], b.round_graph[loop], 0));

@@ -34,11 +34,12 @@ struct Counters {
   unsigned long long steps, scatters, barriers, escapes, secondaries;
   unsigned long long iterations;
   unsigned long long units[4];
-  unsigned long long step_units;  // electrons the several-steps kernel started with
+  unsigned long long step_units;  // electrons the resident-steps kernel started with
   unsigned long long logged;      // escapes offered to the escape log
   unsigned long long slots, tail_slots;  // iteration slots the device-driven loop ran (all, tail)
   unsigned long long ended_zero, ended_limit;  // electrons ended by the zero-energy cut, by the step limit
   int fill;  // the refill fills the wave up to this many electrons (0: W); set by the job server's tail rounds
+  int claim;  // wave electrons taken by the blocks of the resident-steps kernel beyond their first share
 };
 
 template <typename R>
@@ -163,7 +164,7 @@ struct RunView {
 
 // per-thread event counts, reduced once per warp by the kernels
 struct StepCounts {
-  unsigned long long steps = 0, scat = 0, bar = 0, esc = 0, sec = 0, zero = 0, limit = 0;
+  unsigned int steps = 0, scat = 0, bar = 0, esc = 0, sec = 0, zero = 0, limit = 0;
 };
 
 // Histogram::bin (Utility/Histogram.cu:73-80) over bins min + i*delta with
@@ -422,7 +423,18 @@ CM_D int survivors(const Counters* c, int nxt) {
   return n;
 }
 
-// push a secondary to the pool when MonteCarloSS::trackSecondaryElectron (:165-174) would track it
+// a record appended to the secondary pool; false (and CM_EOVERFLOW) when the pool is full
+template <typename R, typename Sink> CM_D bool pool_push(const RunView<R>& v, const El<R>& se, Sink& sink) {
+  const int slot = sink.append(&v.c->pool);
+  if (slot >= v.poolCap) {
+    sink.error(&v.c->error, -5 /* CM_EOVERFLOW */);
+    return false;
+  }
+  store_live(v.pool, slot, se);
+  return true;
+}
+
+// hand a secondary to the sink (the pool) when MonteCarloSS::trackSecondaryElectron (:165-174) would track it
 template <typename R, typename Sink>
 CM_D void push_secondary(const RunView<R>& v, const El<R>& pe, const R sd[3], R sE, Sink& sink, StepCounts& sc) {
   const Msm& m = v.s.msms[v.s.regions[pe.region].msm];
@@ -437,12 +449,7 @@ CM_D void push_secondary(const RunView<R>& v, const El<R>& pe, const R sd[3], R 
   se.step = 0;
   se.key = mix64(pe.key ^ (0x9E3779B97F4A7C15ULL * (unsigned long long)pe.step));
   se.h[0] = se.h[1] = se.h[2] = 0;
-  const int slot = sink.append(&v.c->pool);
-  if (slot >= v.poolCap) {
-    sink.error(&v.c->error, -5 /* CM_EOVERFLOW */);
-    return;
-  }
-  store_live(v.pool, slot, se);
+  if (!sink.put_secondary(v, se)) return;
   job_start(v, pe.pixel, sink);
   ++sc.sec;
 }
@@ -524,25 +531,6 @@ CM_D void misc_one(const RunView<R>& v, int cur, int j, Sink& sink, StepCounts& 
   else job_end(v, e.pixel, e.step, sink);
 }
 
-// Up to nsteps whole steps (flight and event) of wave slot i in one thread, the survivor kept.  The
-// tail of a run, when too few electrons are left to fill the GPU, goes this way: the same steps
-// with the same random streams as the queue kernels, without a launch and a queue per event.
-template <typename R, int D, typename Sink>
-CM_D void steps_one(const RunView<R>& v, int cur, int i, int nsteps, Sink& sink, StepCounts& sc) {
-  El<R> e = load_live(v.w[cur], i);
-  for (int k = 0; k < nsteps; ++k) {
-    const int q = flight_apply<R, D>(v, e, sink, sc);
-    const bool alive = q < 0 ? false
-                             : q == Q_EL ? elastic_apply(v, e)
-                                         : q == Q_TAB ? inelastic_apply(v, e, sink, sc) : misc_apply<R, D>(v, e, sink, sc);
-    if (!alive) {
-      job_end(v, e.pixel, e.step, sink);
-      return;
-    }
-  }
-  keep(v, cur ^ 1, e, sink);
-}
-
 // refill plan of the next wave: secondaries from the pool first; new primaries
 // only once the pool is empty, and at most W/32 per iteration so that the
 // cascades of one batch of primaries do not all peak together
@@ -604,7 +592,7 @@ CM_D void spawn_one(const RunView<R>& v, int nxt, int j, int take_se, int poolTo
   job_start(v, px, sink);
 }
 
-// end of an iteration: counters of the next wave, reset of this one (steps: the iteration ran k_steps)
+// end of an iteration: counters of the next wave, reset of this one (steps: the iteration ran k_block)
 CM_D void tail_update(Counters* c, int cur, int W, int poolCap, bool steps) {
   const int nxt = cur ^ 1;
   int nn, take_se, take_p;
@@ -631,6 +619,7 @@ CM_D void tail_update(Counters* c, int cur, int W, int poolCap, bool steps) {
   c->next_primary += (unsigned long long)take_p;
   c->n[cur] = 0;
   c->q[0] = c->q[1] = c->q[2] = 0;
+  c->claim = 0;
   c->done = (c->n[nxt] == 0 && c->pool == 0 && c->next_primary == c->total_primaries) ? 1 : 0;
 }
 

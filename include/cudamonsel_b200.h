@@ -50,8 +50,8 @@ extern "C" {
 #define CM_OPT_GLOBAL_TABLES 16 /* kernels read every table from global memory (through L1/L2); by default the small
                                    tables are staged into each block's shared memory by a bulk copy (same results) */
 #define CM_OPT_QUEUE_STEPS 8   /* one step per iteration through the queue kernels to the end of a run; by default
-                                  the tail of a run (fewer electrons left than fill the GPU) takes several whole
-                                  steps per thread (same results) */
+                                  the tail of a run (fewer electrons left than fill the GPU) takes many steps per
+                                  launch, its electrons held in shared memory (same results) */
 
 typedef struct cm_context cm_context;
 
@@ -68,8 +68,8 @@ int cm_set_options(cm_context* ctx, int options);
  * each electron's random stream is keyed by its lineage, so they change only the speed. */
 typedef struct {
   int wave;                    /* electrons per wave segment (default 2^21; 1024 .. 2^24) */
-  int tail_below;              /* k_steps runs the tail once fewer electrons are left (default 262144) */
-  int tail_steps;              /* whole steps per thread and launch in the tail (default 32) */
+  int tail_below;              /* k_block runs the tail once fewer electrons are left (default 262144) */
+  int tail_steps;              /* iterations per launch of the tail kernel (default 64) */
   int blocks_per_sm;           /* grid = SMs x blocks_per_sm blocks of 256 threads (default 8) */
   double ms;                   /* cm_autotune: device time of the transport loop under these settings */
   int pool;                    /* secondary-pool records per wave electron (default by the highest beam
@@ -221,7 +221,7 @@ typedef struct {
   double kernel_ms[6];         /* per kernel, summed over launches (profile != 0 only) */
   int64_t kernel_launches[6];
   int64_t units[4];            /* electrons handled by flight, elastic, inelastic, misc */
-  int64_t step_launches;       /* launches of the several-steps-per-thread kernel that runs the tail of a
+  int64_t step_launches;       /* launches of the resident-steps kernel (k_block) that runs the tail of a
                                   run (when fewer electrons are left than fill the GPU); the queue kernels
                                   flight .. misc do not run in those iterations */
   int64_t step_units;          /* electrons those launches started with */
