@@ -31,8 +31,10 @@ namespace cm {
 constexpr int kBlockThreads = CM_BLOCK_THREADS;
 constexpr int kBlockSlots = CM_BLOCK_SLOTS;
 constexpr int kBlockPerSm = CM_BLOCK_MINB;
-// lists a slot can be in: the flights of each wave segment, the inelastic and the misc events
-constexpr int kListTab = kSegments, kListMisc = kSegments + 1, kListDead = kSegments + 2, kLists = kSegments + 3;
+// lists a slot can be in: the flights of each wave segment, the inelastic and the misc events, the flights
+// that need the full form
+constexpr int kListSlow = kSlowSegment, kListTab = kWaveSegments, kListMisc = kWaveSegments + 1, kListDead = kWaveSegments + 2;
+constexpr int kLists = kWaveSegments + 3;
 constexpr int kListNone = kLists;
 // iterations after which a block passes what is left of the wave on to the next one instead of taking it
 constexpr int kBlockHardLimit = 4096;
@@ -124,11 +126,13 @@ __device__ __forceinline__ void block_task(const RunView<R>& v, const BlockMem<R
     El<R> e = b.load(slot);
     bool alive;
     dest = kListDead;
-    if (l < kSegments) {
-      const int q = flight_apply<R, D>(v, e, sink, sc);
+    if (l <= kListSlow) {
+      const int q = l == kListSlow ? flight_apply<R, D>(v, e, sink, sc) : flight_apply<R, 0, true>(v, e, sink, sc);
       alive = q >= 0;
       if (q == Q_EL) alive = elastic_apply(v, e);
-      if (alive) {
+      if (q == Q_SLOW) {
+        dest = kListSlow;
+      } else if (alive) {
         b.px[slot] = e.p[0]; b.py[slot] = e.p[1]; b.pz[slot] = e.p[2];
         b.E[slot] = e.E;
         b.region[slot] = e.region;
@@ -158,7 +162,7 @@ __device__ __forceinline__ void block_task(const RunView<R>& v, const BlockMem<R
       if (alive) {
         b.dx[slot] = e.d[0]; b.dy[slot] = e.d[1]; b.dz[slot] = e.d[2];
         b.E[slot] = e.E;
-        dest = wave_segment(v.s, e.region, e.E);
+        dest = l == kListTab ? wave_segment(v.s, e.region, e.E) : segment_after_misc(v, e);
       }
     }
     if (!alive) job_end(v, e.pixel, e.step, sink);
@@ -185,7 +189,7 @@ __device__ __forceinline__ void block_stage(const RunView<R>& v, const BlockMem<
     if (lane == 0) t = atomicAdd(&b.ctl->task, 1);
     t = __shfl_sync(0xffffffffu, t, 0);
     int l = kListTab, n;
-    for (;;) {  // the list this task falls in: inelastic, misc, then the segments
+    for (;;) {  // the list this task falls in: inelastic, misc, full flights, then the segments
       n = b.ctl->cnt[par][l];
       const int k = (n + 31) >> 5;
       if (t < k) break;
@@ -193,6 +197,8 @@ __device__ __forceinline__ void block_stage(const RunView<R>& v, const BlockMem<
       if (l == kListTab) l = kListMisc;
       else if (l == kListMisc) {
         if (events_only) return;
+        l = kListSlow;
+      } else if (l == kListSlow) {
         l = 0;
       } else if (++l == kSegments) return;
     }
@@ -211,7 +217,7 @@ __global__ void __launch_bounds__(kBlockThreads, kBlockPerSm) k_block(RunView<R>
   const int n = v.c->n[cur];
   const int grid = gridDim.x, tid = threadIdx.x, T = kBlockThreads;
   if (n == 0) return;
-  __shared__ int first[kSegments + 1];
+  __shared__ int first[kWaveSegments + 1];
   segment_starts(v.c, cur, first);
   // The first share: every block takes the same number of electrons, in runs of `run` from all over the
   // wave, so that the blocks get like mixes of materials and energies
@@ -237,7 +243,7 @@ __global__ void __launch_bounds__(kBlockThreads, kBlockPerSm) k_block(RunView<R>
     const El<R> e = load_live(v.w[cur], k * v.W + (i - first[k]));
     b.store(slot, e);
     b.born[slot] = 0;
-    b.put(par, wave_segment(v.s, e.region, e.E), slot);
+    b.put(par, k, slot);
   };
   for (int j = tid; j < mine; j += T) take((j / run * grid + (int)blockIdx.x) * run + j % run, j, 0);
   if (tid == 0) {
@@ -291,13 +297,13 @@ __global__ void __launch_bounds__(kBlockThreads, kBlockPerSm) k_block(RunView<R>
   {
     DeviceSink sink;
     for (int h = 0; h < 2; ++h)
-      for (int l = 0; l < kSegments; ++l) {
+      for (int l = 0; l < kWaveSegments; ++l) {
         const int p = par ^ h, k = c->cnt[p][l];
         for (int i = tid; i < k; i += T) {
           const int slot = b.list[p][l * kBlockSlots + i];
           const El<R> e = b.load(slot);
           if (b.born[slot]) pool_push(v, e, sink);
-          else keep(v, cur ^ 1, e, sink);
+          else keep(v, cur ^ 1, e, l, sink);
         }
       }
     // a wave this launch did not get through is passed on as it is
@@ -312,7 +318,7 @@ __global__ void __launch_bounds__(kBlockThreads, kBlockPerSm) k_block(RunView<R>
       __syncthreads();
       for (int i = tid; i < c->claim_n; i += T) {
         const int w = c->claim_base + i, k = segment_of(first, w);
-        keep(v, cur ^ 1, load_live(v.w[cur], k * v.W + (w - first[k])), sink);
+        keep(v, cur ^ 1, load_live(v.w[cur], k * v.W + (w - first[k])), k, sink);
       }
       __syncthreads();
     }

@@ -1146,6 +1146,26 @@ template <typename R> CM_D bool is_containing_region(const SceneView<R>& s, int 
   return false;
 }
 
+// both ends of a step lie strictly inside a region described by f (see FastRegion)
+template <typename R> CM_D bool step_inside(const SceneView<R>& s, const FastRegion& f, const double* p0, const double* p1) {
+  for (int i = 0; i < f.np; ++i) {
+    const FastPlane& P = s.fast_planes[f.plane0 + i];
+    const double a = P.n[0] * p0[0] + P.n[1] * p0[1] + P.n[2] * p0[2];
+    const double b = P.n[0] * p1[0] + P.n[1] * p1[1] + P.n[2] * p1[2];
+    if (!(a < P.d && b < P.d)) return false;
+  }
+  if (f.cyl < 0) return true;
+  const FastCyl& c = s.fast_cyls[f.cyl];
+  const double* const ends[2] = {p0, p1};
+  for (int k = 0; k < 2; ++k) {
+    const double q[3] = {ends[k][0] - c.e0[0], ends[k][1] - c.e0[1], ends[k][2] - c.e0[2]};
+    const double a = q[0] * c.ax[0] + q[1] * c.ax[1] + q[2] * c.ax[2];
+    const double r[3] = {q[0] - a * c.ax[0], q[1] - a * c.ax[1], q[2] - a * c.ax[2]};
+    if (!(r[0] * r[0] + r[1] * r[1] + r[2] * r[2] < c.rad2)) return false;
+  }
+  return true;
+}
+
 // RegionBase.cu:74-119.  p1 is clipped to the boundary; returns the region just
 // over it (-1: outside the chamber) and the struck boundary's normal.
 template <typename R, int D = kMaxShapeDepth>

@@ -197,6 +197,9 @@ struct cm_context {
   RunIO* io_host = nullptr;        // pinned staging of the run's RunIO
   cudaStream_t stream = nullptr;
   cudaStream_t cap_stream = nullptr;  // stream the launch graphs are captured on
+  // branches of a captured iteration: kernels that do not depend on one another run side by side
+  cudaStream_t side[2] = {nullptr, nullptr};
+  cudaEvent_t fork_ev = nullptr, join_ev[2] = {nullptr, nullptr};
   const std::atomic<int>* cancel = nullptr;  // set by a job server for the running job
   int* cancel_host = nullptr;      // mapped host flag the device loop reads (the server sets it on cancel)
   const int* cancel_dev = nullptr; // its device address
@@ -440,6 +443,54 @@ static Box shape_box(cm_context* ctx, int id) {
     }
   }
   return box_world();
+}
+
+// The half-spaces and cylinders whose common part lies strictly (by kFastMarginNm) inside a shape,
+// appended to fp and fc; false when the shape has no such description.  A step with both ends in there
+// crosses nothing as the boundary search sees it: its plane solves find u outside (0, 1] by a margin far
+// above rounding, and an intersection or a union of shapes (one part of it holding the step) reports none.
+static bool inside_of(const std::vector<Shape>& shapes, const std::vector<Plane>& planes, int id,
+                      std::vector<FastPlane>& fp, std::vector<FastCyl>& fc) {
+  const Shape& sh = shapes[id];
+  auto half_space = [&](const double* n, double d) {
+    const double len = sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+    if (!(len > 0) || !std::isfinite(len) || !std::isfinite(d)) return false;
+    fp.push_back(FastPlane{{n[0] / len, n[1] / len, n[2] / len}, d / len - kFastMarginNm});
+    return true;
+  };
+  switch (sh.kind) {
+    case SHAPE_PLANES:
+      for (int i = 0; i < sh.np; ++i) {
+        const Plane& p = planes[sh.plane0 + i];
+        if (!half_space(p.n, p.n[0] * p.p[0] + p.n[1] * p.p[1] + p.n[2] * p.p[2])) return false;
+      }
+      return true;
+    case SHAPE_INTERSECTION:
+      return inside_of(shapes, planes, sh.a, fp, fc) && inside_of(shapes, planes, sh.b, fp, fc);
+    case SHAPE_UNION: {
+      const size_t np = fp.size(), nc = fc.size();
+      if (inside_of(shapes, planes, sh.a, fp, fc) && fc.size() == nc) return true;
+      fp.resize(np);
+      fc.resize(nc);
+      if (inside_of(shapes, planes, sh.b, fp, fc)) return true;
+      fp.resize(np);
+      fc.resize(nc);
+      return false;
+    }
+    case SHAPE_CYLINDER: {
+      // only a cylinder whose axis is normalised is ever struck (see cm_shape_cylinder)
+      const double u = sh.nax[0] * sh.nax[0] + sh.nax[1] * sh.nax[1] + sh.nax[2] * sh.nax[2];
+      const double rad = sqrt(sh.rad2), m = 1e-3 + 1e-9 * sh.len;
+      if (!(fabs(u - 1.0) < 1e-9) || !(rad > 2 * m) || !(sh.len > 4 * m)) return false;
+      const double back[3] = {-sh.nax[0], -sh.nax[1], -sh.nax[2]};
+      const double a0 = sh.nax[0] * sh.e0[0] + sh.nax[1] * sh.e0[1] + sh.nax[2] * sh.e0[2];
+      if (!half_space(sh.nax, a0 + sh.len - m) || !half_space(back, -a0 - m)) return false;
+      fc.push_back(FastCyl{{sh.e0[0], sh.e0[1], sh.e0[2]}, {sh.nax[0], sh.nax[1], sh.nax[2]}, (rad - m) * (rad - m)});
+      return true;
+    }
+    default:
+      return false;  // spheres: the full form
+  }
 }
 
 template <typename R>
@@ -767,6 +818,25 @@ static int build_scene(cm_context* ctx, DevScene<R>& ds) {
     r.grid = (int)grids.size();
     grids.push_back(g);
   }
+  // what lies strictly inside each childless region (FastRegion): its shape's half-spaces and at most one
+  // cylinder; of a union one part is enough
+  std::vector<FastRegion> fast;
+  std::vector<FastPlane> fplanes;
+  std::vector<FastCyl> fcyls;
+  for (const Region& r : regions) {
+    FastRegion f{r.msm, r.cls, (int)fplanes.size(), -1, -1};
+    if (r.nchild == 0) {
+      const size_t c0 = fcyls.size();
+      if (inside_of(shapes, planes, r.shape, fplanes, fcyls) && fcyls.size() - c0 <= 1) {
+        f.np = (int)fplanes.size() - f.plane0;
+        if (fcyls.size() > c0) f.cyl = (int)c0;
+      } else {
+        fplanes.resize(f.plane0);
+        fcyls.resize(c0);
+      }
+    }
+    fast.push_back(f);
+  }
   SceneView<R>& v = ds.view;
   int rc = 0;
   const bool h = ds.host;
@@ -776,7 +846,8 @@ static int build_scene(cm_context* ctx, DevScene<R>& ds) {
       (rc = dev_copy(ds.allocs, motts, &v.mott, h)) || (rc = dev_copy(ds.allocs, tabs, &v.tables, h)) ||
       (rc = dev_copy(ds.allocs, blob, &v.blob, h)) || (rc = dev_copy(ds.allocs, dbl, &v.dbl, h)) ||
       (rc = dev_copy(ds.allocs, grids, &v.grids, h)) || (rc = dev_copy(ds.allocs, cell_start, &v.cell_start, h)) ||
-      (rc = dev_copy(ds.allocs, grid_items, &v.grid_items, h)))
+      (rc = dev_copy(ds.allocs, grid_items, &v.grid_items, h)) || (rc = dev_copy(ds.allocs, fast, &v.fast, h)) ||
+      (rc = dev_copy(ds.allocs, fplanes, &v.fast_planes, h)) || (rc = dev_copy(ds.allocs, fcyls, &v.fast_cyls, h)))
     return rc;
   v.chamber = 0;
   v.options = ctx->options;
@@ -891,41 +962,59 @@ __device__ __forceinline__ void flush_counts(Counters* c, StepCounts& sc) {
 __device__ __forceinline__ void segment_starts(const Counters* c, int cur, int* first) {
   if (threadIdx.x == 0) {
     int a = 0;
-    for (int k = 0; k < kSegments; ++k) {
+    for (int k = 0; k < kWaveSegments; ++k) {
       first[k] = a;
       a += c->nc[cur][k];
     }
-    first[kSegments] = a;
+    first[kWaveSegments] = a;
   }
   __syncthreads();
 }
 
 __device__ __forceinline__ int segment_of(const int* first, int i) {
   int k = 0;
-  while (k < kSegments - 1 && i >= first[k + 1]) ++k;
+  while (k < kWaveSegments - 1 && i >= first[k + 1]) ++k;
   return k;
 }
 
-template <typename R, int D> __device__ __forceinline__ void flight_loop(const RunView<R>& v, int cur) {
+// FAST flights of the wave's class segments
+template <typename R> __device__ __forceinline__ void flight_fast_loop(const RunView<R>& v, int cur) {
   DeviceSink sink;
   StepCounts sc;
-  const int n = v.c->n[cur];
-  if ((int)(blockIdx.x * blockDim.x) >= n || !stage_tables(v)) return;  // blocks without work stage nothing
-  __shared__ int first[kSegments + 1];
+  const int n = v.c->n[cur] - v.c->nc[cur][kSlowSegment];
+  if ((int)(blockIdx.x * blockDim.x) >= n) return;
+  __shared__ int first[kWaveSegments + 1];
   segment_starts(v.c, cur, first);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int k = segment_of(first, i);  // the i-th electron over the class segments in order
-    flight_one<R, D>(v, cur, k * v.W + (i - first[k]), sink, sc);
+    flight_one<R, 0, true>(v, cur, k * v.W + (i - first[k]), sink, sc);
   }
   flush_counts(v.c, sc);
 }
 
-// FP64 flight: register-hungry double geometry and physics, compiled without an occupancy target
-template <typename R, int D> __global__ void __launch_bounds__(256) k_flight(RunView<R> v, int cur) {
-  flight_loop<R, D>(v, cur);
+#ifndef CM_MINB_FLIGHT32
+#define CM_MINB_FLIGHT32 4
+#endif
+#ifndef CM_MINB_FLIGHT64
+#define CM_MINB_FLIGHT64 2
+#endif
+template <typename R>
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? CM_MINB_FLIGHT32 : CM_MINB_FLIGHT64) k_flight_fast(RunView<R> v, int cur) {
+  flight_fast_loop(v, cur);
 }
 
-// Kernels that stage the small tables into shared memory (1 flight, 2 elastic, 4 inelastic) and
+// the full form of the flights in the wave's slow segment
+template <typename R, int D> __global__ void __launch_bounds__(256) k_flight(RunView<R> v, int cur) {
+  DeviceSink sink;
+  StepCounts sc;
+  const int n = v.c->nc[cur][kSlowSegment];
+  if ((int)(blockIdx.x * blockDim.x) >= n) return;
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
+    flight_one<R, D, false>(v, cur, kSlowSegment * v.W + j, sink, sc);
+  flush_counts(v.c, sc);
+}
+
+// Kernels that stage the small tables into shared memory (2 elastic, 4 inelastic) and
 // the inelastic grid in blocks per SM when it stages.  k_inelastic gathers ~130 table values per event
 // (cubic interpolation in the 2-D energy-loss and SE tables and the 3-D angle table); staged into the
 // shared memory of a grid of 2 resident blocks per SM it gains 1 % on the linescan.  Staging in the
@@ -939,9 +1028,6 @@ template <typename R, int D> __global__ void __launch_bounds__(256) k_flight(Run
 
 // Resident CTAs per SM the kernels are compiled for (register caps 65536 / (256 x n)); a build may set
 // them with -DCM_MINB_FLIGHT32=n and so on.  CM_MINB_INELASTIC unset: the compiler chooses.
-#ifndef CM_MINB_FLIGHT32
-#define CM_MINB_FLIGHT32 3
-#endif
 #ifndef CM_MINB_ELASTIC
 #define CM_MINB_ELASTIC 4
 #endif
@@ -956,15 +1042,7 @@ template <typename R, int D> __global__ void __launch_bounds__(256) k_flight(Run
 #define CM_LB_INELASTIC __launch_bounds__(256)
 #endif
 
-// FP32 flight over leaf shapes compiled for 3 resident CTAs per SM (80 registers): the kernel is
-// latency-bound and the extra warps hide more than the spills cost (linescan +5 %, rough image +3 %
-// against 2 CTAs per SM; 4 CTAs spill twice as much and lose 7 % on the rough image).  Tree walks
-// (D > 0) spill too much under a cap and keep k_flight.  k_elastic runs at 4 CTAs per SM (64
-// registers, a few spills): linescan +2 %.
-__global__ void __launch_bounds__(256, CM_MINB_FLIGHT32) k_flight32_leaf(RunView<float> v, int cur) {
-  flight_loop<float, 0>(v, cur);
-}
-
+// k_elastic runs at 4 CTAs per SM (64 registers, a few spills): linescan +2 %.
 template <typename R>
 __global__ void CM_LB_ELASTIC k_elastic(RunView<R> v, int cur) {
   DeviceSink sink;
@@ -995,16 +1073,10 @@ __global__ void __launch_bounds__(256) k_misc(RunView<R> v, int cur) {
 
 // the kernels are compiled for the intersection nestings 0 (leaf shapes only), 2 and 4
 // smem: bytes of staged tables (v.s.nstaged elements), 0 when the view stages none
-static void launch_flight(const RunView<double>& v, int cur, int grid, cudaStream_t s, size_t smem = 0) {
-  if (v.s.depth == 0) k_flight<double, 0><<<grid, 256, smem, s>>>(v, cur);
-  else if (v.s.depth <= 2) k_flight<double, 2><<<grid, 256, smem, s>>>(v, cur);
-  else k_flight<double, kMaxShapeDepth><<<grid, 256, smem, s>>>(v, cur);
-}
-
-static void launch_flight(const RunView<float>& v, int cur, int grid, cudaStream_t s, size_t smem = 0) {
-  if (v.s.depth == 0) k_flight32_leaf<<<grid, 256, smem, s>>>(v, cur);
-  else if (v.s.depth <= 2) k_flight<float, 2><<<grid, 256, smem, s>>>(v, cur);
-  else k_flight<float, kMaxShapeDepth><<<grid, 256, smem, s>>>(v, cur);
+template <typename R> static void launch_flight(const RunView<R>& v, int cur, int grid, cudaStream_t s) {
+  if (v.s.depth == 0) k_flight<R, 0><<<grid, 256, 0, s>>>(v, cur);
+  else if (v.s.depth <= 2) k_flight<R, 2><<<grid, 256, 0, s>>>(v, cur);
+  else k_flight<R, kMaxShapeDepth><<<grid, 256, 0, s>>>(v, cur);
 }
 
 // The tail of a run: once fewer electrons are left than fill the GPU, the blocks of k_block take them
@@ -1136,9 +1208,9 @@ static int ensure_buffers(cm_context* ctx, int W, int poolCap) {
   if (rb.cap == W && rb.poolCap >= poolCap) return 0;
   NvtxRange range("cm run buffers");
   rb.release();
-  // two waves of kSegments segments, the pool, three queues: refused before any allocation when the
+  // two waves of kWaveSegments segments, the pool, three queues: refused before any allocation when the
   // device has not that much free memory (less a reserve for the run's other buffers)
-  const size_t need = ((size_t)2 * kSegments * W + (size_t)poolCap) * record_bytes<R>() + (size_t)3 * W * 4;
+  const size_t need = ((size_t)2 * kWaveSegments * W + (size_t)poolCap) * record_bytes<R>() + (size_t)3 * W * 4;
   size_t freeb = 0, totalb = 0;
   CM_CUDA(cudaMemGetInfo(&freeb, &totalb));
   if (need + ((size_t)256 << 20) > freeb) {
@@ -1148,7 +1220,8 @@ static int ensure_buffers(cm_context* ctx, int W, int poolCap) {
     return fail(CM_ENOMEM, msg);
   }
   int rc;
-  if ((rc = alloc_wave(rb.allocs, rb.w[0], kSegments * W)) || (rc = alloc_wave(rb.allocs, rb.w[1], kSegments * W)) ||
+  if ((rc = alloc_wave(rb.allocs, rb.w[0], kWaveSegments * W)) ||
+      (rc = alloc_wave(rb.allocs, rb.w[1], kWaveSegments * W)) ||
       (rc = alloc_wave(rb.allocs, rb.pool, poolCap))) {
     rb.release();  // nothing half-built stays behind: the next run allocates afresh
     return rc;
@@ -1186,16 +1259,37 @@ constexpr int kLoopBody = 16;
 template <typename R>
 static void launch_queue_iteration(const cm_context* ctx, const RunView<R>& v, const RunView<R>& vs, int cur, int grid,
                                    size_t smem, cudaStream_t s, cudaGraphConditionalHandle* h, cudaEvent_t* ev) {
-  if (CM_STAGE_KERNELS & 1) launch_flight(vs, cur, grid, s, smem);
-  else launch_flight(v, cur, grid, s);
+  // The full flights run beside the fast ones, and the inelastic and misc events beside the elastic ones:
+  // each is a few electrons whose serial latency (~50 us) would otherwise be added to every iteration.  A
+  // profiled run launches them one after another, with events between them.
+  const bool side = ev == nullptr;
+  auto fork = [&](int branches) {
+    if (!side) return;
+    cudaEventRecord(ctx->fork_ev, s);
+    for (int k = 0; k < branches; ++k) cudaStreamWaitEvent(ctx->side[k], ctx->fork_ev, 0);
+  };
+  auto join = [&](int branches) {
+    if (!side) return;
+    for (int k = 0; k < branches; ++k) {
+      cudaEventRecord(ctx->join_ev[k], ctx->side[k]);
+      cudaStreamWaitEvent(s, ctx->join_ev[k], 0);
+    }
+  };
+  const cudaStream_t s1 = side ? ctx->side[0] : s, s2 = side ? ctx->side[1] : s;
+  fork(1);
+  launch_flight(v, cur, grid, s1);
+  k_flight_fast<R><<<grid, 256, 0, s>>>(v, cur);
+  join(1);
   if (ev) cudaEventRecordWithFlags(ev[0], s, cudaEventRecordExternal);
+  fork(2);
+  if (CM_STAGE_KERNELS & 4) k_inelastic<R><<<ctx->nsm * CM_INEL_BLOCKS_PER_SM, 256, smem, s1>>>(vs, cur);
+  else k_inelastic<R><<<grid, 256, 0, s1>>>(v, cur);
+  if (ev) cudaEventRecordWithFlags(ev[1], s, cudaEventRecordExternal);
+  launch_misc<R>(v, cur, grid, s2);
+  if (ev) cudaEventRecordWithFlags(ev[2], s, cudaEventRecordExternal);
   if (CM_STAGE_KERNELS & 2) k_elastic<R><<<grid, 256, smem, s>>>(vs, cur);
   else k_elastic<R><<<grid, 256, 0, s>>>(v, cur);
-  if (ev) cudaEventRecordWithFlags(ev[1], s, cudaEventRecordExternal);
-  if (CM_STAGE_KERNELS & 4) k_inelastic<R><<<ctx->nsm * CM_INEL_BLOCKS_PER_SM, 256, smem, s>>>(vs, cur);
-  else k_inelastic<R><<<grid, 256, 0, s>>>(v, cur);
-  if (ev) cudaEventRecordWithFlags(ev[2], s, cudaEventRecordExternal);
-  launch_misc<R>(v, cur, grid, s);
+  join(2);
   if (ev) cudaEventRecordWithFlags(ev[3], s, cudaEventRecordExternal);
   launch_spawn<R>(v, cur, grid, s);
   if (ev) cudaEventRecordWithFlags(ev[4], s, cudaEventRecordExternal);
@@ -1442,7 +1536,8 @@ static int run_device_once(cm_context* ctx, const cm_run_desc* d, uint32_t* back
         float ms[6] = {0, 0, 0, 0, 0, 0};
         if (!tail) {
           for (int k = 0; k < 6; ++k) cudaEventElapsedTime(&ms[k], pev[(size_t)it * 6 + k], pev[(size_t)it * 6 + k + 1]);
-          for (int k = 0; k < 6; ++k) kms[k] += ms[k];
+          static const int order[6] = {CM_K_FLIGHT, CM_K_INELASTIC, CM_K_MISC, CM_K_ELASTIC, CM_K_SPAWN, CM_K_TAIL};
+          for (int k = 0; k < 6; ++k) kms[order[k]] += ms[k];
         } else {
           for (int k = 0; k < 3; ++k) cudaEventElapsedTime(&ms[k], tev[(size_t)it * 3 + k], tev[(size_t)it * 3 + k + 1]);
           step_ms += ms[0];
@@ -1748,6 +1843,11 @@ int cm_context_create(int device, cm_context** out) {
   if (stack < 8192) CM_CUDA(cudaDeviceSetLimit(cudaLimitStackSize, 8192));
   CM_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   CM_CUDA(cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking));
+  CM_CUDA(cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming));
+  for (int k = 0; k < 2; ++k) {
+    CM_CUDA(cudaStreamCreateWithFlags(&c->side[k], cudaStreamNonBlocking));
+    CM_CUDA(cudaEventCreateWithFlags(&c->join_ev[k], cudaEventDisableTiming));
+  }
   CM_CUDA(cudaMalloc(&c->counters, sizeof(Counters)));
   CM_CUDA(cudaMallocHost(&c->counters_host, sizeof(Counters)));
   CM_CUDA(cudaMallocHost(&c->io_host, sizeof(RunIO)));
@@ -1784,6 +1884,11 @@ int cm_context_destroy(cm_context* ctx) {
   cudaFreeHost(ctx->cancel_host);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->cap_stream) cudaStreamDestroy(ctx->cap_stream);
+  for (int k = 0; k < 2; ++k) {
+    if (ctx->side[k]) cudaStreamDestroy(ctx->side[k]);
+    if (ctx->join_ev[k]) cudaEventDestroy(ctx->join_ev[k]);
+  }
+  if (ctx->fork_ev) cudaEventDestroy(ctx->fork_ev);
   delete ctx;
   return 0;
 }
@@ -2848,7 +2953,7 @@ static int run_noalloc(cm_context* ctx, const cm_run_desc* d, uint32_t* back, ui
                            "allocates, so make one cm_run, cm_run_device or cm_eval_* call with this precision "
                            "after the last scene change first");
   const int n = d->npix;
-  // layout: counters | bad flag | run inputs | pixel tables | wave 0 | wave 1 (kSegments W each) | 3 queues |
+  // layout: counters | bad flag | run inputs | pixel tables | wave 0 | wave 1 (kWaveSegments W each) | 3 queues |
   // pool (8 W)
   Carve a{scratch};
   Counters* c = a.take<Counters>(1);
@@ -2863,7 +2968,7 @@ static int run_noalloc(cm_context* ctx, const cm_run_desc* d, uint32_t* back, ui
   const size_t rec = 3 * 8 + 8 * sizeof(R) + 4 * 4 + 8;
   const size_t pad = (3 * 16 + 3) * 256;  // worst-case rounding of the 51 pieces below
   const size_t left = kNoAllocScratchBytes - a.off;
-  long long W = (long long)((left > pad ? left - pad : 0) / ((2 * kSegments + 8) * rec + 3 * 4));
+  long long W = (long long)((left > pad ? left - pad : 0) / ((2 * kWaveSegments + 8) * rec + 3 * 4));
   if (d->wave > 0 && d->wave < W) W = d->wave;
   if (W < 1024) return fail(CM_EINVAL, "cm_run_noalloc: no room for a wave of 1024 electrons");
   const int poolCap = (int)(8 * W);
@@ -2875,8 +2980,8 @@ static int run_noalloc(cm_context* ctx, const cm_run_desc* d, uint32_t* back, ui
 #endif
   v.s = ds.view;
   v.s.chamber = d->chamber;
-  carve_wave(a, v.w[0], kSegments * (int)W);
-  carve_wave(a, v.w[1], kSegments * (int)W);
+  carve_wave(a, v.w[0], kWaveSegments * (int)W);
+  carve_wave(a, v.w[1], kWaveSegments * (int)W);
   for (int k = 0; k < 3; ++k) v.q[k] = a.take<int>(W);
   carve_wave(a, v.pool, poolCap);
   if (a.off > kNoAllocScratchBytes) return fail(CM_EINVAL, "cm_run_noalloc: scratch layout does not fit");
@@ -2912,6 +3017,7 @@ static int run_noalloc(cm_context* ctx, const cm_run_desc* d, uint32_t* back, ui
     for (int k = 0; k < 16; ++k, ++it) {
       const int cur = it & 1;
       launch_flight(v, cur, grid, s);
+      k_flight_fast<R><<<grid, 256, 0, s>>>(v, cur);
       k_elastic<R><<<grid, 256, 0, s>>>(v, cur);
       k_inelastic<R><<<grid, 256, 0, s>>>(v, cur);
       launch_misc<R>(v, cur, grid, s);

@@ -58,6 +58,24 @@ struct ChildGrid {
   int unb0, nunb;         // the unbounded children: grid_items[unb0 .. unb0 + nunb)
 };
 
+// The part of a childless region that lies strictly inside its shape, as half-spaces (FastPlane) and at
+// most one cylinder wall.  A step whose two ends are both in there meets no boundary, and the region test
+// and the boundary search need not run: kFastMarginNm is far above the rounding of either evaluation (at
+// most ~1e-6 nm for coordinates below 1e9 nm), so both decide alike.
+struct FastRegion {
+  int msm, cls;          // as the Region's
+  int plane0, np;        // half-spaces fast_planes[plane0, plane0 + np); np < 0: no such description
+  int cyl;               // fast_cyls index, -1: none
+};
+struct FastPlane {
+  double n[3], d;        // inside: n . p < d
+};
+struct FastCyl {
+  double e0[3], ax[3];   // a point of the axis and its unit vector
+  double rad2;           // inside: squared distance from the axis < rad2
+};
+constexpr double kFastMarginNm = 1e-4;
+
 // electrons are kept in one wave segment per material class, so that the
 // threads of a warp mostly run the same material's code
 constexpr int kClasses = 4;
@@ -66,7 +84,11 @@ constexpr int kClasses = 4;
 // a warp's threads mostly run the same branches
 constexpr int kSegments = 2 * kClasses;
 constexpr double kSegmentSplitEv = 50.0;
-constexpr int kMaxWave = 1 << 27;  // electrons per wave segment: kSegments x and 8 x (the pool) stay within int
+// and one more for the electrons whose next step may meet a boundary or needs no mechanism (those in regions
+// without a FastRegion description, at a boundary just met, or handed back by the fast flight): the full
+// flight takes these
+constexpr int kSlowSegment = kSegments, kWaveSegments = kSegments + 1;
+constexpr int kMaxWave = 1 << 27;  // electrons per wave segment: kWaveSegments x and 8 x (the pool) stay within int
 
 // JoyLuoNieminenCSD (JMONSEL/JoyLuoNieminenCSD.cu:42-121) in eV/nm units
 struct Jln {
@@ -155,6 +177,9 @@ struct SceneView {
   const ChildGrid* grids;
   const int* cell_start;
   const int* grid_items;
+  const FastRegion* fast;    // per region
+  const FastPlane* fast_planes;
+  const FastCyl* fast_cyls;
   const R* blob;             // table data in compute precision
   const double* dbl;         // double copies: NISTMott quantile tables (sampled angles within 1e-6 in FP32
                              // too), NU-table axes and 3-D table values

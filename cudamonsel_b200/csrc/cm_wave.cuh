@@ -24,10 +24,11 @@ struct Wave {
 
 struct Counters {
   int n[2];              // electrons in each wave
-  int nc[2][kSegments];  // of which in each segment (segment k holds slots [k W, k W + nc))
-  int ns[kSegments];     // electrons the refill appends after the survivors of each segment
+  int nc[2][kWaveSegments];  // of which in each segment (segment k holds slots [k W, k W + nc))
+  int ns[kWaveSegments];     // electrons the refill appends after the survivors of each segment
   int pool;
   int q[3];
+  int deferred;  // fast flights handed on to the next iteration's full flights
   int error;
   int done;
   unsigned long long next_primary, total_primaries;
@@ -93,7 +94,13 @@ template <typename R> CM_D El<R> load_event(const Wave<R>& w, int i) {
   return e;
 }
 
-enum { Q_EL = 0, Q_TAB = 1, Q_MISC = 2 };
+// wave segment of an electron in `region` at energy E: its material's class, split at kSegmentSplitEv
+template <typename R> CM_D int wave_segment(const SceneView<R>& s, int region, R E) {
+  if (region < 0 || s.fast[region].np < 0) return kSlowSegment;
+  return 2 * s.fast[region].cls + (E < (R)kSegmentSplitEv ? 1 : 0);
+}
+
+enum { Q_EL = 0, Q_TAB = 1, Q_MISC = 2, Q_SLOW = 3 };
 enum { AUX_MECH = 1, AUX_BARRIER = 2, AUX_PASS = 3 };
 CM_HD int aux_pack(int kind, int v) { return (kind << 24) | (v & 0xffffff); }
 CM_HD int aux_kind(int a) { return a >> 24; }
@@ -275,14 +282,20 @@ template <typename R> CM_D int mech_pick(const R* cum, int n, R r) {
 // One step's flight on a record held in registers (p, d, E, step, region and key valid; the pixel too,
 // or, when pixel_src is given, read from there if the electron escapes): the event queue of its end, or
 // -1 when the electron ended here (escaped and tallied, stopped, trapped).
-template <typename R, int D, typename Sink>
+//
+// FAST: the step of an electron that stays strictly inside a childless region, without the region test,
+// the boundary search, crossings and escapes; Q_SLOW, with nothing changed or counted, when this step may
+// need them (the full form then takes it from the start: the random stream is keyed by the step).
+template <typename R, int D, bool FAST = false, typename Sink>
 CM_D int flight_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc, const int* pixel_src = nullptr) {
   const SceneView<R>& s = v.s;
   int reg = e.region;
-  if (reg < 0 || !shape_contains<R, D>(s, s.regions[reg].shape, e.p))
+  if (FAST) {
+    if (reg < 0 || s.fast[reg].np < 0) return Q_SLOW;
+  } else if (reg < 0 || !shape_contains<R, D>(s, s.regions[reg].shape, e.p))
     reg = containing_subregion<R, D>(s, chamber_of(v, pixel_src ? *pixel_src : e.pixel), e.p);
   if (reg < 0) return -1;
-  const Msm& m = s.msms[s.regions[reg].msm];
+  const Msm& m = s.msms[FAST ? s.fast[reg].msm : s.regions[reg].msm];
   bool complete = false;
   double fp = 2.0 * kChamberRadiusNm;
   R total = 0;
@@ -299,6 +312,8 @@ CM_D int flight_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc,
       // geometry, so that the rates need not stay live (nothing else draws from this stream)
       idx = mech_pick(cum, m.nmech, g.next() * total);
       kind = s.mechs[m.mech0 + idx].kind;
+    } else if (FAST) {
+      return Q_SLOW;
     } else if (e.step > 1000000u) {  // MONSEL_MaterialScatterModel::randomMeanPathLength (:86-90)
       complete = true;
       ++sc.limit;
@@ -316,7 +331,8 @@ CM_D int flight_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc,
   double p1[3] = {e.p[0] + fp * (double)e.d[0], e.p[1] + fp * (double)e.d[1], e.p[2] + fp * (double)e.d[2]};
   double hn[3];
   bool clipped = false;
-  const int next = find_end_of_step<R, D>(s, reg, e.p, p1, hn, &clipped);
+  if (FAST && !step_inside(s, s.fast[reg], e.p, p1)) return Q_SLOW;
+  const int next = FAST ? reg : find_end_of_step<R, D>(s, reg, e.p, p1, hn, &clipped);
   const double dd = sqrt((p1[0] - e.p[0]) * (p1[0] - e.p[0]) + (p1[1] - e.p[1]) * (p1[1] - e.p[1]) +
                          (p1[2] - e.p[2]) * (p1[2] - e.p[2]));
   const R dE = m.csd ? jln_compute(m.jln, (R)dd, e.E) : R(0);
@@ -368,9 +384,16 @@ CM_D int flight_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc,
   return queue;
 }
 
+// append an electron to segment k of the next wave
+template <typename R, typename Sink> CM_D void keep(const RunView<R>& v, int nxt, const El<R>& e, int k, Sink& sink) {
+  const int slot = sink.append_q(v.c->nc[nxt], k);
+  store_live(v.w[nxt], k * v.W + slot, e);
+}
+
 // The flight of wave slot i: reads what the step uses and writes back only what it changes
 // (direction, pixel and key stay in place for the event kernels), then queues the event.
-template <typename R, int D, typename Sink>
+// FAST: an electron whose step needs the full form goes to the next wave's slow segment as it is.
+template <typename R, int D, bool FAST, typename Sink>
 CM_D void flight_one(const RunView<R>& v, int cur, int i, Sink& sink, StepCounts& sc) {
   const Wave<R>& W = v.w[cur];
   El<R> e;
@@ -380,37 +403,31 @@ CM_D void flight_one(const RunView<R>& v, int cur, int i, Sink& sink, StepCounts
   e.step = W.step[i];
   e.region = W.region[i];
   e.key = W.key[i];
-  const int queue = flight_apply<R, D>(v, e, sink, sc, W.pixel + i);  // the pixel is read only on escape
+  const int queue = flight_apply<R, D, FAST>(v, e, sink, sc, W.pixel + i);  // the pixel is read only on escape
   if (queue < 0) {
     if (v.io->job_alive) job_end(v, W.pixel[i], e.step, sink);
     return;
   }
+  if (FAST && queue == Q_SLOW) {
+    e.pixel = W.pixel[i];
+    keep(v, cur ^ 1, e, kSlowSegment, sink);
+    sink.append(&v.c->deferred);
+    return;
+  }
   W.px[i] = e.p[0]; W.py[i] = e.p[1]; W.pz[i] = e.p[2];
   W.E[i] = e.E; W.Ep[i] = e.Ep;
-  W.region[i] = e.region; W.aux[i] = e.aux;
+  W.aux[i] = e.aux;
   W.step[i] = e.step;
-  if (aux_kind(e.aux) == AUX_BARRIER) { W.hx[i] = e.h[0]; W.hy[i] = e.h[1]; W.hz[i] = e.h[2]; }
+  if (!FAST) W.region[i] = e.region;  // a FAST step stays in its region
+  if (!FAST && aux_kind(e.aux) == AUX_BARRIER) { W.hx[i] = e.h[0]; W.hy[i] = e.h[1]; W.hz[i] = e.h[2]; }
   const int slot = sink.append_q(v.c->q, queue);
   v.q[queue][slot] = i;
-}
-
-// wave segment of an electron in `region` at energy E: its material's class, split at kSegmentSplitEv
-template <typename R> CM_D int wave_segment(const SceneView<R>& s, int region, R E) {
-  const int cls = region >= 0 ? s.regions[region].cls : 0;
-  return 2 * cls + (E < (R)kSegmentSplitEv ? 1 : 0);
-}
-
-// append a surviving electron to its segment of the next wave
-template <typename R, typename Sink> CM_D void keep(const RunView<R>& v, int nxt, const El<R>& e, Sink& sink) {
-  const int k = wave_segment(v.s, e.region, e.E);
-  const int slot = sink.append_q(v.c->nc[nxt], k);
-  store_live(v.w[nxt], k * v.W + slot, e);
 }
 
 // wave index of the i-th electron of a wave counted over its class segments in order
 CM_D int wave_index(const Counters* c, int cur, int W, int i) {
   int k = 0;
-  while (k < kSegments - 1 && i >= c->nc[cur][k]) {
+  while (k < kWaveSegments - 1 && i >= c->nc[cur][k]) {
     i -= c->nc[cur][k];
     ++k;
   }
@@ -419,7 +436,7 @@ CM_D int wave_index(const Counters* c, int cur, int W, int i) {
 
 CM_D int survivors(const Counters* c, int nxt) {
   int n = 0;
-  for (int k = 0; k < kSegments; ++k) n += c->nc[nxt][k];
+  for (int k = 0; k < kWaveSegments; ++k) n += c->nc[nxt][k];
   return n;
 }
 
@@ -511,23 +528,28 @@ template <typename R, int D, typename Sink> CM_D bool misc_apply(const RunView<R
   return !(e.E < (R)m.minE);
 }
 
+// the segment after a misc event: an electron at a boundary is within the fast flight's margin of it
+template <typename R> CM_D int segment_after_misc(const RunView<R>& v, const El<R>& e) {
+  return aux_kind(e.aux) == AUX_BARRIER ? kSlowSegment : wave_segment(v.s, e.region, e.E);
+}
+
 // the queue kernels' events: the record of queue entry j, its event, and the survivor kept
 template <typename R, typename Sink> CM_D void elastic_one(const RunView<R>& v, int cur, int j, Sink& sink) {
   El<R> e = load_event(v.w[cur], v.q[Q_EL][j]);
-  if (elastic_apply(v, e)) keep(v, cur ^ 1, e, sink);
+  if (elastic_apply(v, e)) keep(v, cur ^ 1, e, wave_segment(v.s, e.region, e.E), sink);
   else job_end(v, e.pixel, e.step, sink);
 }
 
 template <typename R, typename Sink> CM_D void inelastic_one(const RunView<R>& v, int cur, int j, Sink& sink, StepCounts& sc) {
   El<R> e = load_event(v.w[cur], v.q[Q_TAB][j]);
-  if (inelastic_apply(v, e, sink, sc)) keep(v, cur ^ 1, e, sink);
+  if (inelastic_apply(v, e, sink, sc)) keep(v, cur ^ 1, e, wave_segment(v.s, e.region, e.E), sink);
   else job_end(v, e.pixel, e.step, sink);
 }
 
 template <typename R, int D, typename Sink>
 CM_D void misc_one(const RunView<R>& v, int cur, int j, Sink& sink, StepCounts& sc) {
   El<R> e = load(v.w[cur], v.q[Q_MISC][j]);
-  if (misc_apply<R, D>(v, e, sink, sc)) keep(v, cur ^ 1, e, sink);
+  if (misc_apply<R, D>(v, e, sink, sc)) keep(v, cur ^ 1, e, segment_after_misc(v, e), sink);
   else job_end(v, e.pixel, e.step, sink);
 }
 
@@ -600,7 +622,7 @@ CM_D void tail_update(Counters* c, int cur, int W, int poolCap, bool steps) {
   if (c->pool > poolCap) c->pool = poolCap;
   if (!c->done) {
     if (steps) c->step_units += (unsigned long long)c->n[cur];
-    else c->units[0] += (unsigned long long)c->n[cur];
+    else c->units[0] += (unsigned long long)(c->n[cur] - c->deferred);
     c->units[1] += (unsigned long long)c->q[0];
     c->units[2] += (unsigned long long)c->q[1];
     c->units[3] += (unsigned long long)c->q[2];
@@ -608,7 +630,7 @@ CM_D void tail_update(Counters* c, int cur, int W, int poolCap, bool steps) {
   }
   (void)nn;
   int appended = 0;  // survivors and refills as appended (a stopped job's primaries are not)
-  for (int k = 0; k < kSegments; ++k) {
+  for (int k = 0; k < kWaveSegments; ++k) {
     c->nc[nxt][k] += c->ns[k];
     c->ns[k] = 0;
     c->nc[cur][k] = 0;
@@ -618,7 +640,7 @@ CM_D void tail_update(Counters* c, int cur, int W, int poolCap, bool steps) {
   c->pool -= take_se;
   c->next_primary += (unsigned long long)take_p;
   c->n[cur] = 0;
-  c->q[0] = c->q[1] = c->q[2] = 0;
+  c->q[0] = c->q[1] = c->q[2] = c->deferred = 0;
   c->claim = 0;
   c->done = (c->n[nxt] == 0 && c->pool == 0 && c->next_primary == c->total_primaries) ? 1 : 0;
 }
