@@ -211,7 +211,7 @@ __device__ __forceinline__ void block_stage(const RunView<R>& v, const BlockMem<
 // Electrons of wave `cur` through about `iters` iterations (a flight with its elastic event, or a queued
 // event, per electron and iteration), survivors kept in the next wave.  cap: slots a block may use.
 template <typename R, int D>
-__global__ void __launch_bounds__(kBlockThreads, kBlockPerSm) k_block(RunView<R> v, int cur, int iters, int cap) {
+__global__ void __launch_bounds__(kBlockThreads, kBlockPerSm) k_block(const __grid_constant__ RunView<R> v, int cur, int iters, int cap) {
   const BlockMem<R> b(cm_stage_smem);
   BlockCtl* c = b.ctl;
   const int n = v.c->n[cur];

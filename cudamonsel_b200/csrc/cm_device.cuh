@@ -7,6 +7,7 @@
 #pragma once
 #include <math.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "cm_scene.h"
 
@@ -296,10 +297,55 @@ CM_D void nu_window(double x, const double* xsd, int n, int order, int& first, i
   nu_locate<double>(x, xsd, n, order, first, nearest);
 }
 
+// nodes of an ascending axis below x (0..n), and through `entry` the bucket's order-3 windows
+CM_D int guide_below(const AxisGuide& g, const GuideEntry* guides, double x, const double* xsd, int n, GuideEntry& entry) {
+  int b;
+  if (g.kind == 1) {
+    const double t = (x - g.x0) * g.scale;
+    b = t > 0.0 ? (t < (double)(g.n - 1) ? (int)t : g.n - 1) : 0;
+  } else {
+#ifdef __CUDA_ARCH__
+    const int hi = __double2hiint(x);
+#else
+    long long bits;
+    memcpy(&bits, &x, 8);
+    const int hi = (int)(bits >> 32);
+#endif
+    b = (hi >> g.shift) - g.base;
+    b = b < 0 ? 0 : b > g.n - 1 ? g.n - 1 : b;
+  }
+  entry = guides[g.off + b];
+  const int k = entry.below;
+  return k + (k < n && xsd[k] < x ? 1 : 0);
+}
+
+// first index of the order-3 window (nu_locate's `first`)
+CM_D int nu_first3(const AxisGuide& g, const GuideEntry* guides, double x, const double* xsd, int n) {
+  if (g.kind == 0) {
+    int first, nearest;
+    nu_locate<double>(x, xsd, n, 3, first, nearest);
+    return first;
+  }
+  GuideEntry e;
+  return guide_below(g, guides, x, xsd, n, e) == e.below ? e.first0 : e.first1;
+}
+
 // NULagrangeInterpolation.cu:131-147 for a 1-D table, order 1 (TabulatedInelasticSM::scatterRate)
-template <typename R> CM_D R nu_d1_order1(const R* f, const R* xs, const double* xsd, int n, R x) {
+template <typename R>
+CM_D R nu_d1_order1(const AxisGuide& g, const GuideEntry* guides, const R* f, const R* xs, const double* xsd, int n, R x) {
   int first, nearest;
-  nu_window((double)x, xsd, n, 1, first, nearest);
+  if (g.kind == 0) {
+    nu_window((double)x, xsd, n, 1, first, nearest);
+  } else {  // nu_locate with order 1, its interval found through the guide
+    GuideEntry e;
+    const int up = guide_below(g, guides, (double)x, xsd, n, e);
+    if (up == 0) first = nearest = 0;
+    else if (up == n) { first = n - 2; nearest = n - 1; }
+    else {
+      first = up - 1;
+      nearest = ((double)x - xsd[up - 1]) <= (xsd[up] - (double)x) ? up - 1 : up;
+    }
+  }
   return nu_neville1(f[first], f[first + 1], xs[first], xs[first + 1], nearest - first, x);
 }
 
@@ -318,11 +364,10 @@ template <typename R> CM_D R dot4(const R w[4], const R* f) { return w[0] * f[0]
 
 // NULagrangeInterpolation.cu:169-192 on a 2-D table (order 3)
 template <typename R>
-CM_D R nu_d2(const R* f, const R* xs0, const double* xs0d, int n0, const R* xs1, const double* xs1d, int n1, R xa, R xb) {
-  int i0, near0;
-  nu_window((double)xa, xs0d, n0, 3, i0, near0);
-  int j0, near1;
-  nu_window((double)xb, xs1d, n1, 3, j0, near1);
+CM_D R nu_d2(const Table& tb, const GuideEntry* guides, const R* f, const R* xs0, const double* xs0d, int n0, const R* xs1,
+             const double* xs1d, int n1, R xa, R xb) {
+  const int i0 = nu_first3(tb.guide[0], guides, (double)xa, xs0d, n0);
+  const int j0 = nu_first3(tb.guide[1], guides, (double)xb, xs1d, n1);
   R xv1[4] = {xs1[j0], xs1[j0 + 1], xs1[j0 + 2], xs1[j0 + 3]};
   R w1[4];
   lag4(xv1, xb, w1);
@@ -338,13 +383,12 @@ CM_D R nu_d2(const R* f, const R* xs0, const double* xs0d, int n0, const R* xs1,
 // NULagrangeInterpolation.cu:215-240 on a 3-D table (order 3).  The reference's
 // final 1-D step uses xsamp[0][0..3] (line 236) whatever the window; `fixes`
 // uses the window's own abscissae.  Evaluated in double in both precisions (see Table).
-CM_D double nu_d3(const double* f, const double* xs0, int n0, const double* xs1, int n1, const double* xs2, int n2,
-                  double xa, double xb, double xc, bool fixes) {
+CM_D double nu_d3(const Table& tb, const GuideEntry* guides, const double* f, const double* xs0, int n0, const double* xs1,
+                  int n1, const double* xs2, int n2, double xa, double xb, double xc, bool fixes) {
   using R = double;
-  int i0, near0, j0, near1, k0, near2;
-  nu_window((double)xa, xs0, n0, 3, i0, near0);
-  nu_window((double)xb, xs1, n1, 3, j0, near1);
-  nu_window((double)xc, xs2, n2, 3, k0, near2);
+  const int i0 = nu_first3(tb.guide[0], guides, xa, xs0, n0);
+  const int j0 = nu_first3(tb.guide[1], guides, xb, xs1, n1);
+  const int k0 = nu_first3(tb.guide[2], guides, xc, xs2, n2);
   R xv1[4] = {xs1[j0], xs1[j0 + 1], xs1[j0 + 2], xs1[j0 + 3]};
   R xv2[4] = {xs2[k0], xs2[k0 + 1], xs2[k0 + 2], xs2[k0 + 3]};
   R w1[4], w2[4];
@@ -377,12 +421,11 @@ template <typename R> CM_D const R* blob_at(const SceneView<R>& s, int off) {
 }
 
 // NUTableInterpolation::interpolate (JMONSEL/NUTableInterpolation.cu:98-115)
-template <typename R> CM_D R table_interp(const SceneView<R>& s, int t, R x0, R x1, R x2, int order) {
-  const Table& tb = s.tables[t];
+template <typename R> CM_D R table_interp(const SceneView<R>& s, const Table& tb, R x0, R x1, R x2, int order) {
   const R* v = blob_at(s, tb.off_v);
   if (tb.dim == 1) {
     const double* xsd = s.dbl + tb.off_x64[0];
-    if (order == 1) return nu_d1_order1(v, blob_at(s, tb.off_x[0]), xsd, tb.n[0], x0);
+    if (order == 1) return nu_d1_order1(tb.guide[0], s.guides, v, blob_at(s, tb.off_x[0]), xsd, tb.n[0], x0);
     int first, nearest;
     const R* xs = blob_at(s, tb.off_x[0]);
     nu_window((double)x0, xsd, tb.n[0], 3, first, nearest);
@@ -391,9 +434,9 @@ template <typename R> CM_D R table_interp(const SceneView<R>& s, int t, R x0, R 
     return nu_neville3(fv, xv, nearest - first, x0);
   }
   if (tb.dim == 2)
-    return nu_d2(v, blob_at(s, tb.off_x[0]), s.dbl + tb.off_x64[0], tb.n[0], blob_at(s, tb.off_x[1]),
+    return nu_d2(tb, s.guides, v, blob_at(s, tb.off_x[0]), s.dbl + tb.off_x64[0], tb.n[0], blob_at(s, tb.off_x[1]),
                  s.dbl + tb.off_x64[1], tb.n[1], x0, x1);
-  return (R)nu_d3(s.dbl + tb.off_v64, s.dbl + tb.off_x64[0], tb.n[0], s.dbl + tb.off_x64[1], tb.n[1],
+  return (R)nu_d3(tb, s.guides, s.dbl + tb.off_v64, s.dbl + tb.off_x64[0], tb.n[0], s.dbl + tb.off_x64[1], tb.n[1],
                           s.dbl + tb.off_x64[2], tb.n[2], (double)x0, (double)x1, (double)x2, (s.options & 1) != 0);
 }
 
@@ -410,12 +453,22 @@ template <typename R> CM_D void table_windows(const SceneView<R>& s, int t, R x0
 }
 
 // ------------------------------------------------------------ elastic scattering
-// EPQLibrary/BrowningEmpiricalCrossSection.cu:24-29, sigma in m^2, E in eV
-template <typename R> CM_D R browning_sigma(const Mott& m, R E) {
-  const R e = E / R(1000);
-  const R re = msqrt(e);
-  const R z17 = (R)m.zp17;
-  return R(3.0e-22) * z17 / (e + R(0.005) * z17 * re + R(0.0007) * (R)m.zp2 / re);
+// EPQLibrary/BrowningEmpiricalCrossSection.cu:24-29, sigma in m^2, e = E / (1 keV), re = sqrt(e)
+template <typename R> CM_D R browning_sigma(const ElemRate<R>& q, R e, R re) { return q.b0 / (e + q.b1 * re + q.b2 / re); }
+
+// what a mechanism's NISTMott cross sections share at one energy: Browning's e and sqrt(e) (below any
+// element's extrapolation energy) and log(E) (above)
+template <typename R> struct MottArgs {
+  R e, re, logE;
+};
+template <typename R> CM_D MottArgs<R> mott_args(R belowMin, R belowMax, R E) {
+  MottArgs<R> a{0, 0, 0};
+  if (E < belowMax) {
+    a.e = E / R(1000);
+    a.re = msqrt(a.e);
+  }
+  if (!(E < belowMin)) a.logE = mlog(E);
+  return a;
 }
 
 // BrowningEmpiricalCrossSection.cu:31-45.  The reference reads z through a
@@ -438,16 +491,34 @@ template <typename R, typename G> CM_D R browning_angle(const Mott& m, R E, G& g
 
 // JMONSEL/NISTMottRS.cu:103-119 times the SelectableElasticSM rate factor (1/nm); below the
 // extrapolation energy method 3 is linear in E, methods 1 and 2 scale Browning's cross section
-template <typename R> CM_D R nistmott_rate(const SceneView<R>& s, const Mott& m, int method, R kel, R kbrown, R E, R logE) {
-  if (E < (R)m.extrapolateBelowEnergy[method]) {
-    if (method == 3) return kel * (R)m.mottXSatMin[3] * E / (R)m.extrapolateBelowEnergy[3];
-    return (R)m.sfBrowning[method] * browning_sigma(m, E) * kbrown;
+template <typename R> CM_D R nistmott_rate(const SceneView<R>& s, const ElemRate<R>& q, int method, R E, const MottArgs<R>& a) {
+  if (E < q.below) {
+    if (method == 3) return q.lin * E / q.below;
+    return q.sf * browning_sigma(q, a.e, a.re) * q.kbrown;
   }
   if (E < (R)s.maxMott) {
-    return kel * ulagrange_d1(blob_at(s, m.off_spwem), 61, s.dl50, s.param, (double)logE);
+    return q.kel * ulagrange_d1(blob_at(s, q.off_spwem), 61, s.dl50, s.param, (double)a.logE);
   }
   // ScreenedRutherfordScatteringAngle.cu:24-30
-  return (R)m.rutherfordA / (E + (R)m.rutherfordB) * kbrown;
+  return q.ra / (E + q.rb) * q.kbrown;
+}
+
+// the rate constants of an element under a method, rounded to R as the arithmetic above takes them
+template <typename R> CM_HD ElemRate<R> elem_rate(const Mott& m, int mott, int method, double kel, double kbrown) {
+  ElemRate<R> q;
+  q.below = (R)m.extrapolateBelowEnergy[method];
+  q.sf = (R)m.sfBrowning[method];
+  q.kbrown = (R)kbrown;
+  q.b0 = R(3.0e-22) * (R)m.zp17;
+  q.b1 = R(0.005) * (R)m.zp17;
+  q.b2 = R(0.0007) * (R)m.zp2;
+  q.kel = (R)kel;
+  q.lin = (R)kel * (R)m.mottXSatMin[3];
+  q.ra = (R)m.rutherfordA;
+  q.rb = (R)m.rutherfordB;
+  q.off_spwem = m.off_spwem;
+  q.mott = mott;
+  return q;
 }
 
 // NISTMottRS.cu:121-154 (Browning's angles below the extrapolation energy for every method)
@@ -510,9 +581,9 @@ template <> CM_D float nieminen_loss(float kE, float x) { return kE * expm1f(-(2
 // JMONSEL/JoyLuoNieminenCSD.cu:91-121; the recursive halving is run with an
 // explicit stack in the same order (first half, then second half at the
 // energy reached after the first).
-template <typename R> CM_D R jln_compute(const Jln& c, R len, R kE) {
-  if ((c.nce == 0) || (kE < (R)c.minE) || (kE <= R(0))) return 0;
-  if (kE <= (R)c.breakE) return nieminen_loss(kE, R(1.5) * (R)c.gamma * len * kE * msqrt(kE));
+template <typename R> CM_D R jln_compute(const Jln<R>& c, R len, R kE) {
+  if ((c.nce == 0) || (kE < c.minE) || (kE <= R(0))) return 0;
+  if (kE <= c.breakE) return nieminen_loss(kE, c.gamma15 * len * kE * msqrt(kE));
   // The reference halves the step recursively while the loss exceeds 10 % of
   // the energy (JoyLuoNieminenCSD.cu:101-121).  The segments form a binary tree
   // visited depth first, left half first; node (depth, idx) covers
@@ -527,12 +598,12 @@ template <typename R> CM_D R jln_compute(const Jln& c, R len, R kE) {
     for (int k = 0; k < depth; ++k) l = l / 2;
     const R e = kE + total;
     bool leaf = true;
-    if ((e < (R)c.minE) || (e <= R(0))) {
-    } else if (e <= (R)c.breakE) {
-      total += nieminen_loss(e, R(1.5) * (R)c.gamma * l * e * msqrt(e));
+    if ((e < c.minE) || (e <= R(0))) {
+    } else if (e <= c.breakE) {
+      total += nieminen_loss(e, c.gamma15 * l * e * msqrt(e));
     } else {
       R loss = 0;
-      for (int i = 0; i < c.nce; i++) loss += (R)c.coef[i] * mlog(((R)c.recipJ[i] * e) + (R)c.beta[i]);
+      for (int i = 0; i < c.nce; i++) loss += c.coef[i] * mlog((c.recipJ[i] * e) + c.beta[i]);
       loss *= l / e;
       const int pending = depth - popcount64(idx);
       if (loss <= (R(0.1) * e) || pending >= 46 || depth >= 62) total += -loss;
@@ -555,14 +626,14 @@ template <typename R> CM_D R jln_compute(const Jln& c, R len, R kE) {
 
 // ------------------------------------------------------------ mechanism rates
 // TabulatedInelasticSM.cu:436-459
-template <typename R> CM_D R tabulated_rate(const SceneView<R>& s, const Mech& k, R E) {
-  const R kEa = E + (R)k.energyOffset;
-  if (kEa < (R)k.iimfpDomain0) return 0;
-  return (R)k.rateMult * table_interp(s, k.tIIMFP, kEa, R(0), R(0), 1);
+template <typename R> CM_D R tabulated_rate(const SceneView<R>& s, const Mech<R>& k, R E) {
+  const R kEa = E + k.energyOffset;
+  if (kEa < k.iimfpDomain0) return 0;
+  return k.rateMult * table_interp(s, k.iimfp, kEa, R(0), R(0), 1);
 }
 
 // GanachaudMokraniPhononInelasticSM.cu:46-72
-template <typename R> CM_D R phonon_rate(const Mech& k, R kE) {
+template <typename R> CM_D R phonon_rate(const Mech<R>& k, R kE) {
   // GanachaudMokraniPhononInelasticSM::scatterRate (GanachaudMokraniPhononInelasticSM.cu:46-72).  The energy
   // ratio and the branch decisions are taken in double in both precisions (kE is exact in either), so a
   // float phonon energy never moves an energy near threshold to the other branch; the common small-x
@@ -571,11 +642,11 @@ template <typename R> CM_D R phonon_rate(const Mech& k, R kE) {
   const double xd = k.phononE / (double)kE;
   if (xd < 0.1) {
     const R x = (R)xd;
-    return (R)k.prefactor * x * mlog(R(4) / x);
+    return k.prefactor * x * mlog(R(4) / x);
   }
   if (xd >= 1.0) return 0;
   const double t = sqrt(1.0 - xd);
-  return (R)(k.prefactor * xd * log((1.0 + t) / (1.0 - t)));
+  return (R)(k.prefactor64 * xd * log((1.0 + t) / (1.0 - t)));
 }
 
 // ------------------------------------------------------------ geometry (double)

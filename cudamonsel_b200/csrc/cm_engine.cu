@@ -245,12 +245,12 @@ static int dev_copy(std::vector<void*>& allocs, const std::vector<T>& v, const T
 }
 
 // JoyLuoNieminenCSD::init (JMONSEL/JoyLuoNieminenCSD.cu:42-82) in SI, converted to eV/nm
-static Jln make_jln(const HMaterial& mt, double breakE) {
-  Jln c;
+template <typename R> static Jln<R> make_jln(const HMaterial& mt, double breakE) {
+  Jln<R> c;
   memset(&c, 0, sizeof(c));
   c.nce = (int)mt.Z.size();
   double bh = -mt.ecb;
-  c.minE = bh * kFromSIeV;
+  c.minE = (R)(bh * kFromSIeV);
   if (c.nce == 0) return c;
   double bhplus1eV = bh + kEV * 1.;
   if (breakE < bhplus1eV) breakE = bhplus1eV;
@@ -262,13 +262,13 @@ static Jln make_jln(const HMaterial& mt, double breakE) {
     double beta = 1. - (recipJ * bhplus1eV);
     double coef = 2.01507E-28 * mt.density * mt.wf[i] * mt.Z[i] / mt.A[i];
     gamma += coef * log((recipJ * breakE) + beta);
-    c.coef[i] = coef * 1e-9 / (kEV * kEV);
-    c.recipJ[i] = recipJ * kEV;
-    c.beta[i] = beta;
+    c.coef[i] = (R)(coef * 1e-9 / (kEV * kEV));
+    c.recipJ[i] = (R)(recipJ * kEV);
+    c.beta[i] = (R)beta;
   }
   gamma /= pow(breakE, 3.5);
-  c.gamma = gamma * 1e-9 * pow(kEV, 1.5);
-  c.breakE = breakE * kFromSIeV;
+  c.gamma15 = R(1.5) * (R)(gamma * 1e-9 * pow(kEV, 1.5));
+  c.breakE = (R)(breakE * kFromSIeV);
   return c;
 }
 
@@ -493,6 +493,71 @@ static bool inside_of(const std::vector<Shape>& shapes, const std::vector<Plane>
   }
 }
 
+// The search guide of an ascending axis: linear buckets or the leading bits of the argument, whichever
+// leaves at most one node in every bucket of at most 4096; kind 0 (bisection) when neither does.
+static AxisGuide make_guide(const double* x, int n, std::vector<GuideEntry>& out) {
+  AxisGuide g;
+  memset(&g, 0, sizeof(g));
+  if (n < 4 || n > 60000) return g;
+  for (int i = 0; i < n; ++i)
+    if (!std::isfinite(x[i]) || (i > 0 && !(x[i] > x[i - 1]))) return g;
+  auto bucket = [&](double v) -> int {  // as guide_below does
+    if (g.kind == 1) {
+      const double t = (v - g.x0) * g.scale;
+      return t > 0.0 ? (t < (double)(g.n - 1) ? (int)t : g.n - 1) : 0;
+    }
+    long long bits;
+    memcpy(&bits, &v, 8);
+    const int b = ((int)(bits >> 32) >> g.shift) - g.base;
+    return b < 0 ? 0 : b > g.n - 1 ? g.n - 1 : b;
+  };
+  auto fits = [&]() {
+    for (int i = 1; i < n; ++i)
+      if (bucket(x[i]) == bucket(x[i - 1])) return false;
+    return true;
+  };
+  bool ok = false;
+  g.kind = 1;
+  g.x0 = x[0];
+  for (int per = 1; per <= 8 && !ok; per *= 2) {
+    g.n = (n - 1) * per + 1;
+    if (g.n > 4096) break;
+    g.scale = (double)(g.n - 1) / (x[n - 1] - x[0]);
+    ok = std::isfinite(g.scale) && fits();
+  }
+  if (!ok && x[0] > 0) {
+    g.kind = 2;
+    for (g.shift = 20; g.shift >= 10 && !ok; --g.shift) {
+      long long b0, b1;
+      memcpy(&b0, &x[0], 8);
+      memcpy(&b1, &x[n - 1], 8);
+      g.base = (int)(b0 >> 32) >> g.shift;
+      const long long cells = (((long long)(int)(b1 >> 32)) >> g.shift) - g.base + 1;
+      if (cells > 4096) break;
+      g.n = (int)cells;
+      if ((ok = fits())) break;
+    }
+  }
+  if (!ok) {
+    memset(&g, 0, sizeof(g));
+    return g;
+  }
+  // the order-3 window of an argument with k nodes below it, from the reference's own search
+  auto first3 = [&](int k) {
+    const double v = k == 0 ? x[0] : k == n ? x[n - 1] * 2 + 1 : x[k];  // x[k] has exactly k nodes below it
+    int first, nearest;
+    nu_locate<double>(v, x, n, 3, first, nearest);
+    return (unsigned short)first;
+  };
+  g.off = (int)out.size();
+  int k = 0;
+  for (int b = 0; b < g.n; ++b) {
+    while (k < n && bucket(x[k]) < b) ++k;
+    out.push_back(GuideEntry{(unsigned short)k, first3(k), first3(std::min(k + 1, n)), 0});
+  }
+  return g;
+}
+
 template <typename R>
 static int build_scene(cm_context* ctx, DevScene<R>& ds) {
   if (ds.valid) return 0;
@@ -509,6 +574,7 @@ static int build_scene(cm_context* ctx, DevScene<R>& ds) {
     std::vector<int> rel;     // relative offsets of those fields in data
   };
   std::vector<Piece> pieces;
+  std::vector<GuideEntry> guides;
   // tables, converted by role to eV / nm units
   std::vector<Table> tabs(ctx->tables.size());
   for (size_t ti = 0; ti < ctx->tables.size(); ++ti) {
@@ -527,6 +593,7 @@ static int build_scene(cm_context* ctx, DevScene<R>& ds) {
       for (double v : t.x[k]) pc.data.push_back((R)(v * f));
       d.off_x64[k] = (int)dbl.size();
       for (double v : t.x[k]) dbl.push_back(v * f);
+      d.guide[k] = make_guide(dbl.data() + d.off_x64[k], d.n[k], guides);
       d.domain[k][0] = t.domain[k][0] * f;
       d.domain[k][1] = t.domain[k][1] * f;
     }
@@ -587,80 +654,81 @@ static int build_scene(cm_context* ctx, DevScene<R>& ds) {
     }
   }
   // scatter models
-  std::vector<Msm> msms;
-  std::vector<Mech> mechs;
+  std::vector<Msm<R>> msms;
+  std::vector<Mech<R>> mechs;
   for (auto& hm : ctx->msms) {
     const HMaterial& mt = ctx->mats[hm.material];
-    Msm m;
+    Msm<R> m;
     memset(&m, 0, sizeof(m));
     m.material = hm.material;
     m.vacuum = mt.Z.empty();
     double minE = m.vacuum ? -INFINITY : std::max(0.0, -mt.ecb);
     if (hm.minSet) minE = hm.minE;
-    m.minE = minE * kFromSIeV;
-    m.ecb = mt.ecb * kFromSIeV;
-    m.u0 = mt.ecb * kFromSIeV;
+    m.minE = (R)(minE * kFromSIeV);
+    m.ecb = (R)(mt.ecb * kFromSIeV);
+    m.u0 = (R)(mt.ecb * kFromSIeV);
     m.classical = hm.classical;
     m.lambda = hm.lambda * 1e9;
-    m.lambdaFactor = (kPi * hm.lambda * sqrt(kElectronMass / 2.)) / kHbar * sqrt(kEV);
+    m.lambdaFactor = (R)((kPi * hm.lambda * sqrt(kElectronMass / 2.)) / kHbar * sqrt(kEV));
     m.csd = hm.csd;
-    if (hm.csd) m.jln = make_jln(mt, hm.breakE);
+    if (hm.csd) m.jln = make_jln<R>(mt, hm.breakE);
     m.mech0 = (int)mechs.size();
     m.nmech = (int)hm.mechs.size();
     for (auto& hk : hm.mechs) {
-      Mech k;
+      Mech<R> k;
       memset(&k, 0, sizeof(k));
       k.kind = hk.kind;
+      m.kinds |= (unsigned)hk.kind << (4 * (&hk - hm.mechs.data()));
       if (hk.kind == MECH_NISTMOTT) {
         k.nel = (int)mt.Z.size();
         const double densityNa = mt.density * kAvogadro;
         for (int i = 0; i < k.nel; ++i) {
           auto it = mottIndex.find(mt.Z[i]);
           if (it == mottIndex.end()) return fail(CM_ESTATE, "no NIST Mott table for Z=" + std::to_string(mt.Z[i]));
-          k.mott[i] = it->second;
-          k.mottMethod = hk.method;
           const double sf = (1000. * mt.wf[i]) / mt.A[i];
-          k.kbrown[i] = sf * densityNa * 1e-9;
-          k.kel[i] = (kBohr * kBohr) * sf * densityNa * 1e-9;
+          k.el[i] = elem_rate<R>(motts[it->second], it->second, hk.method, (kBohr * kBohr) * sf * densityNa * 1e-9,
+                                 sf * densityNa * 1e-9);
+          k.belowMin = i == 0 ? k.el[i].below : std::min(k.belowMin, k.el[i].below);
+          k.belowMax = i == 0 ? k.el[i].below : std::max(k.belowMax, k.el[i].below);
         }
+        k.mottMethod = hk.method;
       } else if (hk.kind == MECH_TABULATED) {
         k.methodSE = (hk.method != 2) && (hk.method != 3) ? 1 : hk.method;
-        k.tIIMFP = hk.tables[0];
-        k.tRed = hk.tables[1];
-        k.tTheta = hk.tables[2];
-        k.tSEE0 = hk.tables[3];
-        k.energyOffset = hk.energyOffset * kFromSIeV;
-        k.minEgenSE = 0.;
-        k.rateMult = 1.;
-        k.energyCBbottom = mt.ecb * kFromSIeV;
-        k.bandgap = mt.bandgap * kFromSIeV;
+        k.iimfp = tabs[hk.tables[0]];
+        k.red = tabs[hk.tables[1]];
+        k.theta = tabs[hk.tables[2]];
+        if (hk.tables[3] >= 0) k.se0 = tabs[hk.tables[3]];
+        k.energyOffset = (R)(hk.energyOffset * kFromSIeV);
+        k.minEgenSE = 0;
+        k.rateMult = 1;
+        k.energyCBbottom = (R)(mt.ecb * kFromSIeV);
+        k.bandgap = (R)(mt.bandgap * kFromSIeV);
         k.energyGap = k.bandgap;
-        k.offsetFermiEnergy = (efermi(mt) + hk.energyOffset) * kFromSIeV;
-        k.bEref = (mt.bandgap > 0. ? -mt.bandgap : efermi(mt)) * kFromSIeV;
+        k.offsetFermiEnergy = (R)((efermi(mt) + hk.energyOffset) * kFromSIeV);
+        k.bEref = (R)((mt.bandgap > 0. ? -mt.bandgap : efermi(mt)) * kFromSIeV);
         k.ncore = (int)mt.core.size();
-        for (int i = 0; i < k.ncore && i < kMaxCore; ++i) k.core[i] = mt.core[i] * kFromSIeV;
-        const Table& tr = tabs[k.tRed];
-        const Table& tt = tabs[k.tTheta];
-        k.eiDomain0 = std::max(tr.domain[0][0], tt.domain[0][0]);
-        k.eiDomain1 = std::min(tr.domain[0][1], tt.domain[0][1]);
-        k.iimfpDomain0 = tabs[k.tIIMFP].domain[0][0];
+        for (int i = 0; i < k.ncore && i < kMaxCore; ++i) k.core[i] = (R)(mt.core[i] * kFromSIeV);
+        k.eiDomain0 = (R)std::max(k.red.domain[0][0], k.theta.domain[0][0]);
+        k.iimfpDomain0 = (R)k.iimfp.domain[0][0];
         if (k.methodSE >= 2) {
-          k.rangeSE0lo = tabs[k.tSEE0].range[0];
-          k.rangeSE0hi = tabs[k.tSEE0].range[1];
+          k.rangeSE0lo = (R)k.se0.range[0];
+          k.rangeSE0hi = (R)k.se0.range[1];
         }
       } else if (hk.kind == MECH_FITTED) {
-        k.energySEgen = hk.energySEgen * kFromSIeV;
-        k.eFermi = efermi(mt) * kFromSIeV;
-        k.csd = make_jln(mt, hk.breakE);
+        const double gen = hk.energySEgen * kFromSIeV, ef = efermi(mt) * kFromSIeV;
+        k.energySEgen = (R)gen;
+        k.fittedSE = (R)(gen + ef);
+        k.csd = make_jln<R>(mt, hk.breakE);
       } else if (hk.kind == MECH_PHONON) {
         k.phononE = hk.phononE * kFromSIeV;
         double occ = 0.5 * (1. + (1. / (exp(hk.phononE / (kBoltzmann * hk.temperature)) - 1.)));
         double epsRatio = (hk.eps0 - hk.epsInf) / hk.eps0 / hk.epsInf;
-        k.prefactor = (hk.ratemult * occ * epsRatio) / kBohr * 1e-9;
+        k.prefactor64 = (hk.ratemult * occ * epsRatio) / kBohr * 1e-9;
+        k.prefactor = (R)k.prefactor64;
       } else if (hk.kind == MECH_POLARON) {
-        k.prefactor = hk.prefactor * 1e-9;
-        k.extinction = hk.extinction * kEV;
-        k.cutoff = (-log(10. / hk.prefactor) / hk.extinction) * kFromSIeV;
+        k.prefactor = (R)(hk.prefactor * 1e-9);
+        k.extinction = (R)(hk.extinction * kEV);
+        k.cutoff = (R)((-log(10. / hk.prefactor) / hk.extinction) * kFromSIeV);
       }
       mechs.push_back(k);
     }
@@ -845,7 +913,7 @@ static int build_scene(cm_context* ctx, DevScene<R>& ds) {
       (rc = dev_copy(ds.allocs, msms, &v.msms, h)) || (rc = dev_copy(ds.allocs, mechs, &v.mechs, h)) ||
       (rc = dev_copy(ds.allocs, motts, &v.mott, h)) || (rc = dev_copy(ds.allocs, tabs, &v.tables, h)) ||
       (rc = dev_copy(ds.allocs, blob, &v.blob, h)) || (rc = dev_copy(ds.allocs, dbl, &v.dbl, h)) ||
-      (rc = dev_copy(ds.allocs, grids, &v.grids, h)) || (rc = dev_copy(ds.allocs, cell_start, &v.cell_start, h)) ||
+      (rc = dev_copy(ds.allocs, guides, &v.guides, h)) || (rc = dev_copy(ds.allocs, grids, &v.grids, h)) || (rc = dev_copy(ds.allocs, cell_start, &v.cell_start, h)) ||
       (rc = dev_copy(ds.allocs, grid_items, &v.grid_items, h)) || (rc = dev_copy(ds.allocs, fast, &v.fast, h)) ||
       (rc = dev_copy(ds.allocs, fplanes, &v.fast_planes, h)) || (rc = dev_copy(ds.allocs, fcyls, &v.fast_cyls, h)))
     return rc;
@@ -999,12 +1067,12 @@ template <typename R> __device__ __forceinline__ void flight_fast_loop(const Run
 #define CM_MINB_FLIGHT64 2
 #endif
 template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? CM_MINB_FLIGHT32 : CM_MINB_FLIGHT64) k_flight_fast(RunView<R> v, int cur) {
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? CM_MINB_FLIGHT32 : CM_MINB_FLIGHT64) k_flight_fast(const __grid_constant__ RunView<R> v, int cur) {
   flight_fast_loop(v, cur);
 }
 
 // the full form of the flights in the wave's slow segment
-template <typename R, int D> __global__ void __launch_bounds__(256) k_flight(RunView<R> v, int cur) {
+template <typename R, int D> __global__ void __launch_bounds__(256) k_flight(const __grid_constant__ RunView<R> v, int cur) {
   DeviceSink sink;
   StepCounts sc;
   const int n = v.c->nc[cur][kSlowSegment];
@@ -1036,6 +1104,9 @@ template <typename R, int D> __global__ void __launch_bounds__(256) k_flight(Run
 #else
 #define CM_LB_ELASTIC __launch_bounds__(256)
 #endif
+#ifndef CM_MINB_INELASTIC
+#define CM_MINB_INELASTIC 2
+#endif
 #if defined(CM_MINB_INELASTIC)
 #define CM_LB_INELASTIC __launch_bounds__(256, CM_MINB_INELASTIC)
 #else
@@ -1044,7 +1115,7 @@ template <typename R, int D> __global__ void __launch_bounds__(256) k_flight(Run
 
 // k_elastic runs at 4 CTAs per SM (64 registers, a few spills): linescan +2 %.
 template <typename R>
-__global__ void CM_LB_ELASTIC k_elastic(RunView<R> v, int cur) {
+__global__ void CM_LB_ELASTIC k_elastic(const __grid_constant__ RunView<R> v, int cur) {
   DeviceSink sink;
   const int n = v.c->q[Q_EL];
   if ((int)(blockIdx.x * blockDim.x) >= n || !stage_tables(v)) return;
@@ -1052,7 +1123,7 @@ __global__ void CM_LB_ELASTIC k_elastic(RunView<R> v, int cur) {
 }
 
 template <typename R>
-__global__ void CM_LB_INELASTIC k_inelastic(RunView<R> v, int cur) {
+__global__ void CM_LB_INELASTIC k_inelastic(const __grid_constant__ RunView<R> v, int cur) {
   DeviceSink sink;
   StepCounts sc;
   const int n = v.c->q[Q_TAB];
@@ -1062,7 +1133,7 @@ __global__ void CM_LB_INELASTIC k_inelastic(RunView<R> v, int cur) {
 }
 
 template <typename R, int D>
-__global__ void __launch_bounds__(256) k_misc(RunView<R> v, int cur) {
+__global__ void __launch_bounds__(256) k_misc(const __grid_constant__ RunView<R> v, int cur) {
   DeviceSink sink;
   StepCounts sc;
   const int n = v.c->q[Q_MISC];
@@ -1109,7 +1180,7 @@ template <typename R> static void launch_misc(const RunView<R>& v, int cur, int 
 }
 
 template <typename R, int D>
-__global__ void __launch_bounds__(256) k_spawn(RunView<R> v, int cur) {
+__global__ void __launch_bounds__(256) k_spawn(const __grid_constant__ RunView<R> v, int cur) {
   const int nxt = cur ^ 1;
   int nn, take_se, take_p;
   refill_plan(v.c, nxt, v.W, v.poolCap, nn, take_se, take_p);
@@ -1127,7 +1198,7 @@ template <typename R> static void launch_spawn(const RunView<R>& v, int cur, int
 }
 
 template <typename R>
-__global__ void k_tail(RunView<R> v, int cur, int steps) {
+__global__ void k_tail(const __grid_constant__ RunView<R> v, int cur, int steps) {
   if (blockIdx.x == 0 && threadIdx.x == 0) tail_update(v.c, cur, v.W, v.poolCap, steps != 0);
 }
 
@@ -1138,7 +1209,7 @@ __global__ void k_tail(RunView<R> v, int cur, int steps) {
 // (the tail loop of k_block takes over).  Iterations of a loop body after its end do no
 // work: their kernels find no electrons.
 template <typename R>
-__global__ void k_loop(RunView<R> v, int cur, int steps, cudaGraphConditionalHandle h) {
+__global__ void k_loop(const __grid_constant__ RunView<R> v, int cur, int steps, cudaGraphConditionalHandle h) {
   if (blockIdx.x != 0 || threadIdx.x != 0) return;
   Counters* c = v.c;
   tail_update(c, cur, v.W, v.poolCap, steps != 0);
@@ -1645,7 +1716,8 @@ template <typename R> __global__ void k_eval_nistmott(SceneView<R> s, int mi, in
   const Mott& m = s.mott[mi];
   const R e = (R)(E[i] * kFromSIeV);
   // cross section in m^2 (rate factor 1/kbrown folded back): kel = a0^2, kbrown = 1
-  sig[i] = (double)nistmott_rate(s, m, method, (R)(kBohr * kBohr), R(1), e, mlog(e));
+  const ElemRate<R> q = elem_rate<R>(m, mi, method, kBohr * kBohr, 1.0);
+  sig[i] = (double)nistmott_rate(s, q, method, e, mott_args(q.below, q.below, e));
   FixedRng<R> g{u + 2 * i, 2, 0};
   th[i] = (double)nistmott_angle(s, m, method, e, g);
 }
@@ -1654,7 +1726,7 @@ template <typename R> __global__ void k_eval_table(SceneView<R> s, int t, int n,
                                                    double* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  out[i] = (double)table_interp(s, t, (R)(x[3 * i] * f0), (R)x[3 * i + 1], (R)x[3 * i + 2], order) / vf;
+  out[i] = (double)table_interp(s, s.tables[t], (R)(x[3 * i] * f0), (R)x[3 * i + 1], (R)x[3 * i + 2], order) / vf;
 }
 
 template <typename R> __global__ void k_eval_locate(SceneView<R> s, int t, int n, const double* x, double f0, int order,
@@ -1669,18 +1741,17 @@ template <typename R> __global__ void k_eval_locate(SceneView<R> s, int t, int n
 template <typename R> __global__ void k_eval_pick(SceneView<R> s, int msm, int n, const double* in, double* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const Msm& m = s.msms[msm];
+  const Msm<R>& m = s.msms[msm];
   const R E = (R)(in[2 * i] * kFromSIeV);
-  R cum[kMaxMech];
-  const R total = msm_cumulative_rates(s, m, E, cum);
-  out[2 * i] = total != R(0) ? mech_pick(cum, m.nmech, (R)in[2 * i + 1] * total) : -1;
-  out[2 * i + 1] = (double)total * 1e9;
+  const MsmRates<R> q = msm_rates(s, m, E);
+  out[2 * i] = q.total != R(0) ? mech_pick(s, m, E, q, (R)in[2 * i + 1] * q.total) : -1;
+  out[2 * i + 1] = (double)q.total * 1e9;
 }
 
 template <typename R> __global__ void k_eval_tabulated(SceneView<R> s, int mech, int n, const double* in, double* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const Mech& k = s.mechs[mech];
+  const Mech<R>& k = s.mechs[mech];
   const double* q = in + 9 * i;
   double* o = out + 12 * i;
   R E = (R)(q[0] * kFromSIeV);
@@ -1702,32 +1773,32 @@ template <typename R> __global__ void k_eval_tabulated(SceneView<R> s, int mech,
 template <typename R> __global__ void k_eval_elastic(SceneView<R> s, int mech, int n, const double* in, double* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const Mech& k = s.mechs[mech];
+  const Mech<R>& k = s.mechs[mech];
   const double* q = in + 7 * i;
   double* o = out + 6 * i;
   const R E = (R)(q[0] * kFromSIeV);
   R d[3];
   dir_from_angles(d, (R)q[1], (R)q[2]);
-  o[0] = (double)mech_rate(s, k, E, mlog(E)) * 1e9;
+  o[0] = (double)mech_rate(s, k, E) * 1e9;
   FixedRng<R> g{q + 3, 4, 0};
   const int el = elastic_scatter(s, k, d, E, g);
   o[1] = d[0]; o[2] = d[1]; o[3] = d[2];
-  o[4] = s.mott[k.mott[el]].Z;
+  o[4] = s.mott[k.el[el].mott].Z;
   o[5] = g.used;
 }
 
 template <typename R> __global__ void k_eval_csd(SceneView<R> s, int msm, int n, const double* in, double* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const Msm& m = s.msms[msm];
+  const Msm<R>& m = s.msms[msm];
   const R E = (R)(in[2 * i] * kFromSIeV);
   const R len = (R)(in[2 * i + 1] * 1e9);
   out[3 * i] = m.csd ? (double)jln_compute(m.jln, len, E) * kEV : 0.;
   double fr = 0, pr = 0;
   for (int k = 0; k < m.nmech; ++k) {
-    const Mech& mk = s.mechs[m.mech0 + k];
-    if (mk.kind == MECH_FITTED) fr = (double)mech_rate(s, mk, E, mlog(E)) * 1e9;
-    if (mk.kind == MECH_POLARON) pr = (double)mech_rate(s, mk, E, mlog(E)) * 1e9;
+    const Mech<R>& mk = s.mechs[m.mech0 + k];
+    if (mk.kind == MECH_FITTED) fr = (double)mech_rate(s, mk, E) * 1e9;
+    if (mk.kind == MECH_POLARON) pr = (double)mech_rate(s, mk, E) * 1e9;
   }
   out[3 * i + 1] = fr;
   out[3 * i + 2] = pr;
@@ -1736,7 +1807,7 @@ template <typename R> __global__ void k_eval_csd(SceneView<R> s, int msm, int n,
 template <typename R> __global__ void k_eval_phonon(SceneView<R> s, int mech, int n, const double* in, double* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const Mech& k = s.mechs[mech];
+  const Mech<R>& k = s.mechs[mech];
   const double* q = in + 5 * i;
   double* o = out + 6 * i;
   R E = (R)(q[0] * kFromSIeV), Ep = E;
@@ -1785,11 +1856,9 @@ template <typename R> __global__ void k_eval_barrier(SceneView<R> s, int from, i
 template <typename R> __global__ void k_eval_freepath(SceneView<R> s, int msm, int n, const double* in, double* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const Msm& m = s.msms[msm];
+  const Msm<R>& m = s.msms[msm];
   const R E = (R)(in[2 * i] * kFromSIeV);
-  R total = 0;
-  const R logE = mlog(E);
-  for (int k = 0; k < m.nmech; ++k) total += mech_rate(s, s.mechs[m.mech0 + k], E, logE);
+  const R total = msm_rates(s, m, E).total;
   double fp = 2.0 * kChamberRadiusNm;
   if (total != R(0)) {
     const R f = -mlog((R)in[2 * i + 1]) / total;

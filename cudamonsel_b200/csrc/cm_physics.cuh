@@ -6,25 +6,28 @@
 
 namespace cm {
 
-// MONSEL_MaterialScatterModel::setCache term for one mechanism (1/nm).
-// logE is log(E) (only the NIST Mott grid uses it).
-template <typename R> CM_D R mech_rate(const SceneView<R>& s, const Mech& k, R E, R logE) {
+// MONSEL_MaterialScatterModel::setCache term for one mechanism (1/nm)
+template <typename R> CM_D R mech_rate(const SceneView<R>& s, const Mech<R>& k, R E) {
   switch (k.kind) {
     case MECH_NISTMOTT: {  // SelectableElasticSM.cu:25-47
       R total = 0;
-      for (int i = 0; i < k.nel; ++i) total += nistmott_rate(s, s.mott[k.mott[i]], k.mottMethod, (R)k.kel[i], (R)k.kbrown[i], E, logE);
+      const MottArgs<R> a = mott_args(k.belowMin, k.belowMax, E);
+      for (int i = 0; i < k.nel; ++i) {
+        const ElemRate<R> q = k.el[i];
+        total += nistmott_rate(s, q, k.mottMethod, E, a);
+      }
       return total;
     }
     case MECH_TABULATED:
       return tabulated_rate(s, k, E);
     case MECH_FITTED:  // FittedInelSM.cu:20-25 (a 0.1 nm step's loss, per nm, per SE energy)
-      if (E <= (R)(k.energySEgen + k.eFermi)) return 0;
-      return (-jln_compute(k.csd, R(0.1), E) * R(10)) / (R)k.energySEgen;
+      if (E <= k.fittedSE) return 0;
+      return (-jln_compute(k.csd, R(0.1), E) * R(10)) / k.energySEgen;
     case MECH_PHONON:
       return phonon_rate(k, E);
     case MECH_POLARON:  // GanachaudMokraniPolaronTrapSM.cu:21-27
-      if (E > (R)k.cutoff) return 0;
-      return (R)k.prefactor * mexp(-(R)k.extinction * E);
+      if (E > k.cutoff) return 0;
+      return k.prefactor * mexp(-k.extinction * E);
   }
   return 0;
 }
@@ -47,34 +50,34 @@ template <typename R> CM_D void update_angles(R& theta, R& phi, R dTheta, R dPhi
 
 // TabulatedInelasticSM.cu:153-207 with the constructor defaults (energy for
 // ionisation = deltaE, default branching ratios)
-template <typename R> CM_D R pick_be(const Mech& k, R deltaE) {
-  if ((k.ncore > 0) && (deltaE <= (R)k.core[0])) return 0;
+template <typename R> CM_D R pick_be(const Mech<R>& k, R deltaE) {
+  if ((k.ncore > 0) && (deltaE <= k.core[0])) return 0;
   int i = 0;
-  while ((i < k.ncore) && ((R)k.core[i] <= deltaE)) ++i;
+  while ((i < k.ncore) && (k.core[i] <= deltaE)) ++i;
   if (i == 0) return 0;
-  return (R)k.core[i - 1];
+  return k.core[i - 1];
 }
 
 // TabulatedInelasticSM::scatter (TabulatedInelasticSM.cu:209-434).  d/E is
 // the primary (updated in place); returns true with sd/sE set when a
 // secondary is generated.  Deviates come in the reference's order.
 template <typename R, typename G>
-CM_D bool tabulated_scatter(const SceneView<R>& s, const Mech& k, R d[3], R& E, R sd[3], R& sE, G& g, R* theta_out = nullptr) {
+CM_D bool tabulated_scatter(const SceneView<R>& s, const Mech<R>& k, R d[3], R& E, R sd[3], R& sE, G& g, R* theta_out = nullptr) {
   const R kE0 = E;
-  const R kE = kE0 + (R)k.energyOffset;
-  if (kE < (R)k.eiDomain0) return false;
+  const R kE = kE0 + k.energyOffset;
+  if (kE < k.eiDomain0) return false;
   R theta = 0, phi = 0;
   R randoms[4];
   randoms[0] = g.next(); randoms[1] = g.next(); randoms[2] = g.next(); randoms[3] = g.next();
-  R deltaE = kE * table_interp(s, k.tRed, kE, randoms[0], R(0), 3);
-  const R gap = (R)k.energyGap, bandgap = (R)k.bandgap, oFE = (R)k.offsetFermiEnergy;
+  R deltaE = kE * table_interp(s, k.red, kE, randoms[0], R(0), 3);
+  const R gap = k.energyGap, bandgap = k.bandgap, oFE = k.offsetFermiEnergy;
   if ((deltaE < gap) && (deltaE > (R(0.95) * gap))) deltaE = gap;
   const R d0[3] = {d[0], d[1], d[2]};
   if (deltaE >= bandgap) {
     R red = (deltaE - gap) / (kE - oFE - (R(2) * gap));
     if (red > R(1)) red = 1;
     else if (red < R(0)) red = 0;
-    theta = table_interp(s, k.tTheta, kE, red, randoms[1], 3);
+    theta = table_interp(s, k.theta, kE, red, randoms[1], 3);
     if (theta_out) *theta_out = theta;
     phi = R(2) * R(kPi) * randoms[2];
     update_dir(d, theta, phi);
@@ -91,15 +94,15 @@ CM_D bool tabulated_scatter(const SceneView<R>& s, const Mech& k, R d[3], R& E, 
   } else {
     Eq = (R(2) * kE) - deltaE - (R(2) * msqrt(kE * (kE - deltaE)) * ct);
   }
-  const R bEref = (R)k.bEref, ecb = (R)k.energyCBbottom, minGen = (R)k.minEgenSE, off = (R)k.energyOffset;
+  const R bEref = k.bEref, ecb = k.energyCBbottom, minGen = k.minEgenSE, off = k.energyOffset;
   R energySE;
   const R be = pick_be(k, deltaE);
   if (k.methodSE == 1 || k.methodSE == 2) {
     if (k.methodSE == 1 || be > 0) energySE = (deltaE + bEref) - be;
     else {
-      R e0 = table_interp(s, k.tSEE0, deltaE, randoms[3], R(0), 3);
-      if (e0 < (R)k.rangeSE0lo) e0 = (R)k.rangeSE0lo;
-      else if (e0 > (R)k.rangeSE0hi) e0 = (R)k.rangeSE0hi;
+      R e0 = table_interp(s, k.se0, deltaE, randoms[3], R(0), 3);
+      if (e0 < k.rangeSE0lo) e0 = k.rangeSE0lo;
+      else if (e0 > k.rangeSE0hi) e0 = k.rangeSE0hi;
       energySE = (deltaE + e0) - off;
     }
     if ((energySE + ecb) < minGen) return false;
@@ -144,9 +147,9 @@ CM_D bool tabulated_scatter(const SceneView<R>& s, const Mech& k, R d[3], R& E, 
     return true;
   }
   // plasmon: SE E0 table, isotropic
-  R e0 = table_interp(s, k.tSEE0, deltaE, randoms[3], R(0), 3);
-  if (e0 < (R)k.rangeSE0lo) e0 = (R)k.rangeSE0lo;
-  else if (e0 > (R)k.rangeSE0hi) e0 = (R)k.rangeSE0hi;
+  R e0 = table_interp(s, k.se0, deltaE, randoms[3], R(0), 3);
+  if (e0 < k.rangeSE0lo) e0 = k.rangeSE0lo;
+  else if (e0 > k.rangeSE0hi) e0 = k.rangeSE0hi;
   energySE = (deltaE + e0) - off;
   if ((energySE + ecb) < minGen) return false;
   const R thetaSE = iso_angle(g.next());
@@ -156,23 +159,49 @@ CM_D bool tabulated_scatter(const SceneView<R>& s, const Mech& k, R d[3], R& E, 
   return true;
 }
 
+// the first element whose cumulative rate at E reaches r
+template <typename R> __host__ __device__ __noinline__ int element_pick(const SceneView<R>& s, const Mech<R>& k, R E, R r) {
+  const MottArgs<R> a = mott_args(k.belowMin, k.belowMax, E);
+  R c = 0;
+  for (int i = 0; i < k.nel - 1; ++i) {
+    const ElemRate<R> q = k.el[i];
+    c += nistmott_rate(s, q, k.mottMethod, E, a);
+    if (!(c < r)) return i;
+  }
+  return k.nel - 1;
+}
+
 // SelectableElasticSM::scatter (SelectableElasticSM.cu:49-67) at the step's
 // starting energy Ep; returns the element picked.
-template <typename R, typename G> CM_D int elastic_scatter(const SceneView<R>& s, const Mech& k, R d[3], R Ep, G& g) {
+template <typename R, typename G> CM_D int elastic_scatter(const SceneView<R>& s, const Mech<R>& k, R d[3], R Ep, G& g) {
   const R u = g.next();
   int el = 0;
   if (k.nel > 1) {
-    const R logE = mlog(Ep);
-    R cum[kMaxElem];
-    R tot = 0;
+    // the first element whose cumulative rate reaches u * total: the cumulative rates of the first three
+    // elements stay in registers, those of a longer composition are summed again
+    const MottArgs<R> a = mott_args(k.belowMin, k.belowMax, Ep);
+    R c[3] = {0, 0, 0}, tot = 0;
     for (int i = 0; i < k.nel; ++i) {
-      tot += nistmott_rate(s, s.mott[k.mott[i]], k.mottMethod, (R)k.kel[i], (R)k.kbrown[i], Ep, logE);
-      cum[i] = tot;
+      const ElemRate<R> q = k.el[i];
+      tot += nistmott_rate(s, q, k.mottMethod, Ep, a);
+      c[0] = i == 0 ? tot : c[0];
+      c[1] = i == 1 ? tot : c[1];
+      c[2] = i == 2 ? tot : c[2];
     }
     const R r = u * tot;
-    while (el < k.nel - 1 && cum[el] < r) ++el;
+    if (k.nel <= 4) {
+      if (c[0] < r) {
+        el = 1;
+        if (k.nel > 2 && c[1] < r) {
+          el = 2;
+          if (k.nel > 3 && c[2] < r) el = 3;
+        }
+      }
+    } else {
+      el = element_pick(s, k, Ep, r);
+    }
   }
-  const R alpha = nistmott_angle(s, s.mott[k.mott[el]], k.mottMethod, Ep, g);
+  const R alpha = nistmott_angle(s, s.mott[k.el[el].mott], k.mottMethod, Ep, g);
   const R beta = R(2 * kPi) * g.next();
   update_dir(d, alpha, beta);
   return el;
@@ -200,7 +229,7 @@ template <> CM_D float phonon_theta(double xd, double omxd, float r0) {
 }
 
 // GanachaudMokraniPhononInelasticSM::scatter (GanachaudMokraniPhononInelasticSM.cu:19-44)
-template <typename R, typename G> CM_D void phonon_scatter(const Mech& k, R d[3], R& E, R& Ep, G& g) {
+template <typename R, typename G> CM_D void phonon_scatter(const Mech<R>& k, R d[3], R& E, R& Ep, G& g) {
   const R kE0 = E;
   // the threshold and the energy ratio in double, as in phonon_rate
   if ((double)kE0 < k.phononE) return;
@@ -218,14 +247,14 @@ template <typename R, typename G> CM_D void phonon_scatter(const Mech& k, R d[3]
 // normal (refraction).  hn is the struck boundary's outward normal from
 // find_end_of_step.  Returns the region after the event.
 template <typename R, typename G>
-CM_D int barrier_scatter(const SceneView<R>& s, const Msm& m, double p[3], R d[3], R& E, int cur, int next, const double hn[3],
+CM_D int barrier_scatter(const SceneView<R>& s, const Msm<R>& m, double p[3], R d[3], R& E, int cur, int next, const double hn[3],
                          G& g) {
   if (cur == next) return cur;
-  const Msm& curm = s.msms[s.regions[cur].msm];
-  const Msm& nextm = s.msms[s.regions[next].msm];
-  R deltaU = -(R)curm.ecb;
-  if (!(deltaU == -(R)m.u0)) return cur;
-  deltaU += (R)nextm.ecb;
+  const Msm<R>& curm = s.msms[s.regions[cur].msm];
+  const Msm<R>& nextm = s.msms[s.regions[next].msm];
+  R deltaU = -curm.ecb;
+  if (!(deltaU == -m.u0)) return cur;
+  deltaU += nextm.ecb;
   R nb[3];
   if (s.options & 1) {
     const R sign = is_containing_region(s, cur, next) ? R(-1) : R(1);
@@ -262,10 +291,10 @@ CM_D int barrier_scatter(const SceneView<R>& s, const Msm& m, double p[3], R d[3
         const R ksum = rootPerpE + rootDiff;
         tp = (R(4) * rootPerpE * rootDiff) / (ksum * ksum);
       } else {
-        const R k1 = (R)m.lambdaFactor * rootPerpE;
+        const R k1 = m.lambdaFactor * rootPerpE;
         if (k1 > R(50)) tp = 1;
         else {
-          const R k2 = (R)m.lambdaFactor * rootDiff;
+          const R k2 = m.lambdaFactor * rootDiff;
           const R ratio = msinh(k1 - k2) / msinh(k1 + k2);
           tp = R(1) - (ratio * ratio);
         }

@@ -90,48 +90,102 @@ constexpr double kSegmentSplitEv = 50.0;
 constexpr int kSlowSegment = kSegments, kWaveSegments = kSegments + 1;
 constexpr int kMaxWave = 1 << 27;  // electrons per wave segment: kWaveSegments x and 8 x (the pool) stay within int
 
+// The structs the transport kernels read are in the compute precision R, rounded once when the scene is
+// built: a value the physics casts to float would otherwise cost a double load and a conversion at a
+// sixteenth of the arithmetic rate in every step.
+
 // JoyLuoNieminenCSD (JMONSEL/JoyLuoNieminenCSD.cu:42-121) in eV/nm units
+template <typename R>
 struct Jln {
   int nce;
-  double coef[kMaxElem];     // eV^2 / nm
-  double recipJ[kMaxElem];   // 1/eV
-  double beta[kMaxElem];
-  double breakE, gamma, minE;  // eV, eV^-1.5 nm^-1, eV
+  R minE, breakE;            // eV
+  R gamma15;                 // R(1.5) * R(gamma), gamma in eV^-1.5 nm^-1
+  R coef[kMaxElem];          // eV^2 / nm
+  R recipJ[kMaxElem];        // 1/eV
+  R beta[kMaxElem];
 };
 
+// One element of a NISTMott mechanism: what its cross section (times the rate factor, 1/nm) takes.  kel is
+// a0^2 * scalefactor * density * N_A per table unit, kbrown the same factor for a cross section in nm^2.
+template <typename R>
+struct alignas(16) ElemRate {
+  R below;                   // extrapolation energy of the mechanism's method, eV
+  R sf, kbrown;              // Browning's scale factor and rate factor
+  R b0, b1, b2;              // Browning: b0 / (e + b1 sqrt(e) + b2 / sqrt(e)), e in keV
+  R kel, lin;                // table rate factor; method 3: kel * table value at `below`
+  R ra, rb;                  // screened Rutherford: ra / (E + rb)
+  int off_spwem;             // the element's cross sections in the blob
+  int mott;                  // index into Scene::mott
+};
+
+// A search guide of one axis of an NU table: the argument's bucket, found by arithmetic, holds at most one
+// node, so one comparison with that node finds the interval the reference's bisection finds.  The bucket
+// is (x - x0) * scale rounded down, or for kind 2 the leading bits of x (an axis spaced by a factor).
+struct AxisGuide {
+  int kind;                  // 0: none (bisection), 1: linear, 2: leading bits
+  int off, n;                // entries guides[off, off + n)
+  int shift, base;           // kind 2
+  double x0, scale;          // kind 1
+};
+// bucket entry: nodes below the bucket, and the first index of the order-3 window of an argument that is
+// not above (first0) or above (first1) the bucket's node
+struct alignas(8) GuideEntry {
+  unsigned short below, first0, first1, pad;
+};
+
+// NUTableInterpolation (dims 1..3) in the precision blob, with double copies in SceneView::dbl of every
+// axis (window selection compares the argument with the reference's abscissae in double in both
+// precisions) and of a 3-D table's values (its reference d3 step extrapolates from the first energy
+// window, which amplifies rounding by orders of magnitude, so FP32 evaluates it in double too)
+struct Table {
+  int dim;
+  int n[3];
+  int off_x[3];
+  int off_v;
+  int off_x64[3];            // axes in dbl
+  int off_v64;               // values in dbl (3-D tables), else -1
+  AxisGuide guide[3];
+  double domain[3][2];
+  double range[2];
+};
+
+template <typename R>
 struct Mech {
   int kind;
-  // NISTMott via SelectableElasticSM: per element mott index and rate factor
+  // NISTMott via SelectableElasticSM
   int nel;
-  int mott[kMaxElem];        // index into Scene::mott
   int mottMethod;            // NISTMottRS method 1..3
-  double kel[kMaxElem];      // a0^2 * scalefactor * density * N_A in nm^-1 per (table unit)
-  double kbrown[kMaxElem];   // the same factor for a Browning/Rutherford cross section in nm^2
+  R belowMin, belowMax;      // smallest and largest extrapolation energy of its elements
   // TabulatedInelasticSM (JMONSEL/TabulatedInelasticSM.cu:461-498), energies in eV
   int methodSE;
-  int tIIMFP, tRed, tTheta, tSEE0;
-  double energyOffset, minEgenSE, rateMult, energyCBbottom, bandgap, energyGap, offsetFermiEnergy, bEref;
-  double eiDomain0, eiDomain1, iimfpDomain0, rangeSE0lo, rangeSE0hi;
-  int ncore;
-  double core[kMaxCore];
-  // FittedInelSM
-  double energySEgen, eFermi;
-  Jln csd;
+  R energyOffset, minEgenSE, rateMult, energyCBbottom, bandgap, energyGap, offsetFermiEnergy, bEref;
+  R eiDomain0, iimfpDomain0, rangeSE0lo, rangeSE0hi;
+  // FittedInelSM: SE energy (and lowest energy with a rate), energy per SE
+  R fittedSE, energySEgen;
   // phonon / polaron
-  double phononE, prefactor, extinction, cutoff;
+  R prefactor, extinction, cutoff;
+  double phononE, prefactor64;
+  ElemRate<R> el[kMaxElem];
+  int ncore;
+  R core[kMaxCore];
+  Jln<R> csd;
+  Table iimfp, red, theta, se0;  // copies of the tables it uses
 };
 
+template <typename R>
 struct Msm {
   int material;
   int vacuum;
   int nmech, mech0;          // mechanisms [mech0, mech0+nmech)
+  unsigned kinds;            // their kinds, 4 bits each, the first lowest
   int csd;                   // 0 = ZeroCSD, 1 = JoyLuoNieminenCSD
-  Jln jln;
-  double minE;               // eV (may be -inf)
-  double ecb;                // E_CB bottom of this material, eV
-  double u0;                 // barrier's u0 (= E_CB of the material it was built for), eV
+  R minE;                    // eV (may be -inf)
+  R ecb;                     // E_CB bottom of this material, eV
+  R u0;                      // barrier's u0 (= E_CB of the material it was built for), eV
   int classical;
-  double lambda, lambdaFactor;  // lambdaFactor in 1/sqrt(eV)
+  double lambda;
+  R lambdaFactor;            // 1/sqrt(eV)
+  Jln<R> jln;
 };
 
 // NISTMottRS per element; the tables live in the precision blob, the extrapolation constants are
@@ -148,21 +202,6 @@ struct Mott {
   double rutherfordAlpha;           // alpha = rutherfordAlpha / E
 };
 
-// NUTableInterpolation (dims 1..3) in the precision blob, with double copies in SceneView::dbl of every
-// axis (window selection compares the argument with the reference's abscissae in double in both
-// precisions) and of a 3-D table's values (its reference d3 step extrapolates from the first energy
-// window, which amplifies rounding by orders of magnitude, so FP32 evaluates it in double too)
-struct Table {
-  int dim;
-  int n[3];
-  int off_x[3];
-  int off_v;
-  int off_x64[3];            // axes in dbl
-  int off_v64;               // values in dbl (3-D tables), else -1
-  double domain[3][2];
-  double range[2];
-};
-
 // The whole scene as device pointers (one struct passed by value to kernels)
 template <typename R>
 struct SceneView {
@@ -170,10 +209,11 @@ struct SceneView {
   const Plane* planes;
   const Region* regions;
   const int* children;
-  const Msm* msms;
-  const Mech* mechs;
+  const Msm<R>* msms;
+  const Mech<R>* mechs;
   const Mott* mott;
   const Table* tables;
+  const GuideEntry* guides;
   const ChildGrid* grids;
   const int* cell_start;
   const int* grid_items;

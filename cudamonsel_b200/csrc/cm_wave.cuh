@@ -255,22 +255,46 @@ template <typename R> CM_D int chamber_of(const RunView<R>& v, int px) {
   return io.pchamber ? io.pchamber[px] : v.s.chamber;
 }
 
-// MONSEL_MaterialScatterModel::setCache (MONSEL_MaterialScatterModel.cu:44-62): the cumulative scatter rates
-// of the model's mechanisms at E (1/nm) into cum[0..nmech); returns the total
-template <typename R> CM_D R msm_cumulative_rates(const SceneView<R>& s, const Msm& m, R E, R* cum) {
-  R total = 0;
-  const R logE = mlog(E);
-  for (int k = 0; k < m.nmech; ++k) {
-    total += mech_rate(s, s.mechs[m.mech0 + k], E, logE);
-    cum[k] = total;
+// MONSEL_MaterialScatterModel::scatter (:93-134) of a model with more than four mechanisms: the first one
+// whose cumulative rate at E reaches r
+template <typename R> __host__ __device__ __noinline__ int mech_pick_long(const SceneView<R>& s, const Msm<R>& m, R E, R r) {
+  R c = 0;
+  for (int k = 0; k < m.nmech - 1; ++k) {
+    c += mech_rate(s, s.mechs[m.mech0 + k], E);
+    if (!(c < r)) return k;
   }
-  return total;
+  return m.nmech - 1;
+}
+
+// MONSEL_MaterialScatterModel::setCache (MONSEL_MaterialScatterModel.cu:44-62): the total scatter rate of
+// the model's mechanisms at E (1/nm), and the first three cumulative rates (a local array indexed by
+// mechanism would live in local memory)
+template <typename R> struct MsmRates {
+  R total, c0, c1, c2;
+};
+template <typename R> CM_D MsmRates<R> msm_rates(const SceneView<R>& s, const Msm<R>& m, R E) {
+  MsmRates<R> q{0, 0, 0, 0};
+  for (int k = 0; k < m.nmech; ++k) {
+    q.total += mech_rate(s, s.mechs[m.mech0 + k], E);
+    q.c0 = k == 0 ? q.total : q.c0;
+    q.c1 = k == 1 ? q.total : q.c1;
+    q.c2 = k == 2 ? q.total : q.c2;
+  }
+  return q;
 }
 
 // MONSEL_MaterialScatterModel::scatter (:93-134): the first mechanism whose cumulative rate reaches r
-template <typename R> CM_D int mech_pick(const R* cum, int n, R r) {
+template <typename R> CM_D int mech_pick(const SceneView<R>& s, const Msm<R>& m, R E, const MsmRates<R>& q, R r) {
+  const int n = m.nmech;
+  if (n > 4) return mech_pick_long(s, m, E, r);
   int idx = 0;
-  while (idx < n - 1 && cum[idx] < r) ++idx;
+  if (n > 1 && q.c0 < r) {
+    idx = 1;
+    if (n > 2 && q.c1 < r) {
+      idx = 2;
+      if (n > 3 && q.c2 < r) idx = 3;
+    }
+  }
   return idx;
 }
 
@@ -295,23 +319,23 @@ CM_D int flight_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc,
   } else if (reg < 0 || !shape_contains<R, D>(s, s.regions[reg].shape, e.p))
     reg = containing_subregion<R, D>(s, chamber_of(v, pixel_src ? *pixel_src : e.pixel), e.p);
   if (reg < 0) return -1;
-  const Msm& m = s.msms[FAST ? s.fast[reg].msm : s.regions[reg].msm];
+  const Msm<R>& m = s.msms[FAST ? s.fast[reg].msm : s.regions[reg].msm];
   bool complete = false;
   double fp = 2.0 * kChamberRadiusNm;
   R total = 0;
   int idx = 0, kind = 0;
   {
     Rng<R> g(e.key, e.step, 0);
-    R cum[kMaxMech];
-    total = msm_cumulative_rates(s, m, e.E, cum);
+    const MsmRates<R> rates = msm_rates(s, m, e.E);
+    total = rates.total;
     if (total != R(0)) {
       const R f = -mlog(g.next()) / total;
       if ((double)f < fp) fp = (double)f;
       // MONSEL_MaterialScatterModel::scatter (:93-134) picks the mechanism from the rates at the
       // step's starting energy with the stream's next deviate; it is drawn here, before the
       // geometry, so that the rates need not stay live (nothing else draws from this stream)
-      idx = mech_pick(cum, m.nmech, g.next() * total);
-      kind = s.mechs[m.mech0 + idx].kind;
+      idx = mech_pick(s, m, e.E, rates, g.next() * total);
+      kind = (m.kinds >> (4 * idx)) & 15;
     } else if (FAST) {
       return Q_SLOW;
     } else if (e.step > 1000000u) {  // MONSEL_MaterialScatterModel::randomMeanPathLength (:86-90)
@@ -342,7 +366,7 @@ CM_D int flight_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc,
   e.step += 1;
   e.region = reg;
   ++sc.steps;
-  if ((e.E < (R)m.minE) || complete) return -1;
+  if ((e.E < m.minE) || complete) return -1;
   int queue;
   if (next == reg) {
     ++sc.scat;
@@ -454,8 +478,8 @@ template <typename R, typename Sink> CM_D bool pool_push(const RunView<R>& v, co
 // hand a secondary to the sink (the pool) when MonteCarloSS::trackSecondaryElectron (:165-174) would track it
 template <typename R, typename Sink>
 CM_D void push_secondary(const RunView<R>& v, const El<R>& pe, const R sd[3], R sE, Sink& sink, StepCounts& sc) {
-  const Msm& m = v.s.msms[v.s.regions[pe.region].msm];
-  if (!(sE > (R)m.minE)) return;
+  const Msm<R>& m = v.s.msms[v.s.regions[pe.region].msm];
+  if (!(sE > m.minE)) return;
   El<R> se;
   se.p[0] = pe.p[0]; se.p[1] = pe.p[1]; se.p[2] = pe.p[2];
   se.d[0] = sd[0]; se.d[1] = sd[1]; se.d[2] = sd[2];
@@ -477,29 +501,29 @@ CM_D void push_secondary(const RunView<R>& v, const El<R>& pe, const R sd[3], R 
 // SelectableElasticSM events
 template <typename R> CM_D bool elastic_apply(const RunView<R>& v, El<R>& e) {
   const SceneView<R>& s = v.s;
-  const Msm& m = s.msms[s.regions[e.region].msm];
-  const Mech& k = s.mechs[m.mech0 + aux_val(e.aux)];
+  const Msm<R>& m = s.msms[s.regions[e.region].msm];
+  const Mech<R>& k = s.mechs[m.mech0 + aux_val(e.aux)];
   Rng<R> g(e.key, e.step - 1, 1);
   elastic_scatter(s, k, e.d, e.Ep, g);
-  return !(e.E < (R)m.minE);
+  return !(e.E < m.minE);
 }
 
 // TabulatedInelasticSM events
 template <typename R, typename Sink> CM_D bool inelastic_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc) {
   const SceneView<R>& s = v.s;
-  const Msm& m = s.msms[s.regions[e.region].msm];
-  const Mech& k = s.mechs[m.mech0 + aux_val(e.aux)];
+  const Msm<R>& m = s.msms[s.regions[e.region].msm];
+  const Mech<R>& k = s.mechs[m.mech0 + aux_val(e.aux)];
   Rng<R> g(e.key, e.step - 1, 1);
   R sd[3], sE;
   const bool made = tabulated_scatter(s, k, e.d, e.E, sd, sE, g);
   if (made) push_secondary(v, e, sd, sE, sink, sc);
-  return !(e.E < (R)m.minE);
+  return !(e.E < m.minE);
 }
 
 // barrier crossings, FittedInelSM, phonon, and steps that end without a mechanism
 template <typename R, int D, typename Sink> CM_D bool misc_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc) {
   const SceneView<R>& s = v.s;
-  const Msm& m = s.msms[s.regions[e.region].msm];
+  const Msm<R>& m = s.msms[s.regions[e.region].msm];
   const int kind = aux_kind(e.aux);
   Rng<R> g(e.key, e.step - 1, 1);
   if (kind == AUX_BARRIER) {
@@ -514,18 +538,18 @@ template <typename R, int D, typename Sink> CM_D bool misc_apply(const RunView<R
     return true;
   }
   if (kind == AUX_MECH) {
-    const Mech& k = s.mechs[m.mech0 + aux_val(e.aux)];
+    const Mech<R>& k = s.mechs[m.mech0 + aux_val(e.aux)];
     if (k.kind == MECH_FITTED) {  // FittedInelSM::scatter (FittedInelSM.cu:13-18)
       const R phi = R(2) * R(kPi) * g.next();
       const R theta = iso_angle(g.next());
       R sd[3];
       dir_from_angles(sd, theta, phi);
-      push_secondary(v, e, sd, (R)(k.energySEgen + k.eFermi), sink, sc);
+      push_secondary(v, e, sd, k.fittedSE, sink, sc);
     } else if (k.kind == MECH_PHONON) {
       phonon_scatter(k, e.d, e.E, e.Ep, g);
     }
   }
-  return !(e.E < (R)m.minE);
+  return !(e.E < m.minE);
 }
 
 // the segment after a misc event: an electron at a boundary is within the fast flight's margin of it
