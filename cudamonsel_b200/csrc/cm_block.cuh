@@ -49,69 +49,66 @@ struct BlockCtl {
   int exhausted;       // the wave has no electron left to take
 };
 
-// The block's electrons: structure of arrays over its slots, in shared memory.
+// The block's electrons: structure of arrays over its slots, in shared memory at fixed offsets (so that
+// every access is a shared-memory instruction with an immediate offset).
 template <typename R>
 struct BlockMem {
-  double *px, *py, *pz;
-  unsigned long long* key;
-  R *dx, *dy, *dz, *E, *Ep, *hx, *hy, *hz;
-  int *region, *pixel, *aux;
-  uint32_t* step;
-  unsigned short* list[2];  // [kLists][kBlockSlots] each
-  unsigned short* free_slot;
-  unsigned char* born;      // the slot holds a secondary started in this launch
-  BlockCtl* ctl;
+  static constexpr int n = kBlockSlots;
+  static constexpr int oKey = 24 * n, oR = 32 * n, oW = oR + 8 * n * (int)sizeof(R), oCtl = oW + 16 * n;
+  static constexpr int oList = oCtl + ((int)sizeof(BlockCtl) + 15) / 16 * 16;
+  static constexpr int oFree = oList + 2 * kLists * n * 2, oBorn = oFree + 2 * n, kBytes = oBorn + n;
+  __device__ __forceinline__ static double& p(int a, int i) { return ((double*)cm_stage_smem)[a * n + i]; }
+  __device__ __forceinline__ static unsigned long long& key(int i) { return ((unsigned long long*)(cm_stage_smem + oKey))[i]; }
+  // direction 0..2, E 3, Ep 4, hit normal 5..7
+  __device__ __forceinline__ static R& r(int a, int i) { return ((R*)(cm_stage_smem + oR))[a * n + i]; }
+  // region 0, pixel 1, aux 2, step 3
+  __device__ __forceinline__ static int& w(int a, int i) { return ((int*)(cm_stage_smem + oW))[a * n + i]; }
+  __device__ __forceinline__ static BlockCtl& ctl() { return *(BlockCtl*)(cm_stage_smem + oCtl); }
+  __device__ __forceinline__ static unsigned short& list(int par, int l, int i) {
+    return ((unsigned short*)(cm_stage_smem + oList))[(par * kLists + l) * n + i];
+  }
+  __device__ __forceinline__ static unsigned short& free_slot(int i) { return ((unsigned short*)(cm_stage_smem + oFree))[i]; }
+  // the slot holds a secondary started in this launch
+  __device__ __forceinline__ static unsigned char& born(int i) { return (cm_stage_smem + oBorn)[i]; }
 
-  static constexpr size_t bytes() {
-    return (size_t)kBlockSlots * (4 * 8 + 8 * sizeof(R) + 4 * 4 + 2 * kLists * 2 + 2 + 1) + sizeof(BlockCtl) + 64;
-  }
-  __device__ __forceinline__ explicit BlockMem(unsigned char* p) {
-    constexpr size_t n = kBlockSlots;
-    px = (double*)p; py = px + n; pz = py + n;
-    key = (unsigned long long*)(pz + n);
-    dx = (R*)(key + n); dy = dx + n; dz = dy + n; E = dz + n; Ep = E + n; hx = Ep + n; hy = hx + n; hz = hy + n;
-    region = (int*)(hz + n); pixel = region + n; aux = pixel + n;
-    step = (uint32_t*)(aux + n);
-    ctl = (BlockCtl*)(step + n);
-    list[0] = (unsigned short*)(ctl + 1);
-    list[1] = list[0] + kLists * n;
-    free_slot = list[1] + kLists * n;
-    born = (unsigned char*)(free_slot + n);
-  }
-  __device__ __forceinline__ El<R> load(int i) const {
+  __device__ __forceinline__ static El<R> load(int i) {
     El<R> e;
-    e.p[0] = px[i]; e.p[1] = py[i]; e.p[2] = pz[i];
-    e.d[0] = dx[i]; e.d[1] = dy[i]; e.d[2] = dz[i];
-    e.E = E[i];
-    e.region = region[i]; e.pixel = pixel[i];
-    e.step = step[i]; e.key = key[i];
+    for (int a = 0; a < 3; ++a) {
+      e.p[a] = p(a, i);
+      e.d[a] = r(a, i);
+    }
+    e.E = r(3, i);
+    e.region = w(0, i); e.pixel = w(1, i);
+    e.step = (uint32_t)w(3, i); e.key = key(i);
     return e;
   }
-  __device__ __forceinline__ void store(int i, const El<R>& e) const {
-    px[i] = e.p[0]; py[i] = e.p[1]; pz[i] = e.p[2];
-    dx[i] = e.d[0]; dy[i] = e.d[1]; dz[i] = e.d[2];
-    E[i] = e.E;
-    region[i] = e.region; pixel[i] = e.pixel;
-    step[i] = e.step; key[i] = e.key;
+  __device__ __forceinline__ static void store(int i, const El<R>& e) {
+    for (int a = 0; a < 3; ++a) {
+      p(a, i) = e.p[a];
+      r(a, i) = e.d[a];
+    }
+    r(3, i) = e.E;
+    w(0, i) = e.region; w(1, i) = e.pixel;
+    w(3, i) = (int)e.step; key(i) = e.key;
   }
-  __device__ __forceinline__ void put(int par, int l, int slot) const {
-    list[par][l * kBlockSlots + atomicAdd(&ctl->cnt[par][l], 1)] = (unsigned short)slot;
+  __device__ __forceinline__ static void put(int par, int l, int slot) {
+    list(par, l, atomicAdd(&ctl().cnt[par][l], 1)) = (unsigned short)slot;
   }
 };
 
 // secondaries take a free slot of the block, or go to the run's pool when there is none
 template <typename R>
 struct BlockSink : DeviceSink {
-  const BlockMem<R>& b;
   int par;  // parity of the lists being filled
-  __device__ __forceinline__ BlockSink(const BlockMem<R>& m, int p) : b(m), par(p) {}
+  __device__ __forceinline__ explicit BlockSink(int p) : par(p) {}
   __device__ __forceinline__ bool put_secondary(const RunView<R>& v, const El<R>& se) {
-    const int k = atomicAdd(&b.ctl->taken, 1), avail = b.ctl->nfree;
+    using B = BlockMem<R>;
+    const int k = atomicAdd(&B::ctl().taken, 1), avail = B::ctl().nfree;
     if (k >= avail) return pool_push(v, se, *this);
-    const int slot = b.free_slot[avail - 1 - k];
-    b.store(slot, se);
-    b.born[slot] = 1;
-    b.put(par, wave_segment(v.s, se.region, se.E), slot);
+    const int slot = B::free_slot(avail - 1 - k);
+    B::store(slot, se);
+    B::born(slot) = 1;
+    B::put(par, wave_segment(v.s, se), slot);
     return true;
   }
 };
@@ -119,11 +116,11 @@ struct BlockSink : DeviceSink {
 // One task: up to 32 electrons of one list through their flight (with the elastic event it ends in) or
 // their queued event.  Every lane of the warp calls it; lanes without an electron have slot < 0.
 template <typename R, int D>
-__device__ __forceinline__ void block_task(const RunView<R>& v, const BlockMem<R>& b, int l, int slot, BlockSink<R>& sink,
-                                           StepCounts& sc) {
+__device__ __forceinline__ void block_task(const RunView<R>& v, int l, int slot, BlockSink<R>& sink, StepCounts& sc) {
+  using B = BlockMem<R>;
   int dest = kListNone;
   if (slot >= 0) {
-    El<R> e = b.load(slot);
+    El<R> e = B::load(slot);
     bool alive;
     dest = kListDead;
     if (l <= kListSlow) {
@@ -133,36 +130,37 @@ __device__ __forceinline__ void block_task(const RunView<R>& v, const BlockMem<R
       if (q == Q_SLOW) {
         dest = kListSlow;
       } else if (alive) {
-        b.px[slot] = e.p[0]; b.py[slot] = e.p[1]; b.pz[slot] = e.p[2];
-        b.E[slot] = e.E;
-        b.region[slot] = e.region;
-        b.step[slot] = e.step;
+        for (int a = 0; a < 3; ++a) B::p(a, slot) = e.p[a];
+        B::r(3, slot) = e.E;
+        B::w(0, slot) = e.region;
+        B::w(3, slot) = (int)e.step;
         if (q == Q_EL) {
-          b.dx[slot] = e.d[0]; b.dy[slot] = e.d[1]; b.dz[slot] = e.d[2];
+          for (int a = 0; a < 3; ++a) B::r(a, slot) = e.d[a];
         } else {
-          b.Ep[slot] = e.Ep;
-          b.aux[slot] = e.aux;
-          if (aux_kind(e.aux) == AUX_BARRIER) { b.hx[slot] = e.h[0]; b.hy[slot] = e.h[1]; b.hz[slot] = e.h[2]; }
+          B::r(4, slot) = e.Ep;
+          B::w(2, slot) = e.aux;
+          if (aux_kind(e.aux) == AUX_BARRIER)
+            for (int a = 0; a < 3; ++a) B::r(5 + a, slot) = e.h[a];
         }
-        dest = q == Q_EL ? wave_segment(v.s, e.region, e.E) : q == Q_TAB ? kListTab : kListMisc;
+        dest = q == Q_EL ? segment_after(v.s, e) : q == Q_TAB ? kListTab : kListMisc;
       }
     } else {
-      e.Ep = b.Ep[slot];
-      e.aux = b.aux[slot];
+      e.Ep = B::r(4, slot);
+      e.aux = B::w(2, slot);
       if (l == kListTab) {
         alive = inelastic_apply(v, e, sink, sc);
       } else {
-        e.h[0] = b.hx[slot]; e.h[1] = b.hy[slot]; e.h[2] = b.hz[slot];
+        for (int a = 0; a < 3; ++a) e.h[a] = B::r(5 + a, slot);
         alive = misc_apply<R, D>(v, e, sink, sc);
         if (alive) {
-          b.px[slot] = e.p[0]; b.py[slot] = e.p[1]; b.pz[slot] = e.p[2];
-          b.region[slot] = e.region;
+          for (int a = 0; a < 3; ++a) B::p(a, slot) = e.p[a];
+          B::w(0, slot) = e.region;
         }
       }
       if (alive) {
-        b.dx[slot] = e.d[0]; b.dy[slot] = e.d[1]; b.dz[slot] = e.d[2];
-        b.E[slot] = e.E;
-        dest = l == kListTab ? wave_segment(v.s, e.region, e.E) : segment_after_misc(v, e);
+        for (int a = 0; a < 3; ++a) B::r(a, slot) = e.d[a];
+        B::r(3, slot) = e.E;
+        dest = segment_after(v.s, e);
       }
     }
     if (!alive) job_end(v, e.pixel, e.step, sink);
@@ -172,25 +170,26 @@ __device__ __forceinline__ void block_task(const RunView<R>& v, const BlockMem<R
   const unsigned same = __match_any_sync(0xffffffffu, dest);
   const int lane = threadIdx.x & 31, leader = __ffs(same) - 1;
   int base = 0;
-  if (dest != kListNone && lane == leader) base = atomicAdd(&b.ctl->cnt[sink.par][dest], __popc(same));
+  if (dest != kListNone && lane == leader) base = atomicAdd(&B::ctl().cnt[sink.par][dest], __popc(same));
   base = __shfl_sync(0xffffffffu, base, leader);
   if (dest != kListNone)
-    b.list[sink.par][dest * kBlockSlots + base + __popc(same & ((1u << lane) - 1))] = (unsigned short)slot;
+    B::list(sink.par, dest, base + __popc(same & ((1u << lane) - 1))) = (unsigned short)slot;
 }
 
 // The tasks of an iteration: 32 entries of one list each, events first (they take longest).  events_only:
 // the flights stay in their lists.
 template <typename R, int D>
-__device__ __forceinline__ void block_stage(const RunView<R>& v, const BlockMem<R>& b, int par, bool events_only,
-                                            BlockSink<R>& sink, StepCounts& sc) {
+__device__ __forceinline__ void block_stage(const RunView<R>& v, int par, bool events_only, BlockSink<R>& sink,
+                                            StepCounts& sc) {
+  using B = BlockMem<R>;
   const int lane = threadIdx.x & 31;
   for (;;) {
     int t = 0;
-    if (lane == 0) t = atomicAdd(&b.ctl->task, 1);
+    if (lane == 0) t = atomicAdd(&B::ctl().task, 1);
     t = __shfl_sync(0xffffffffu, t, 0);
     int l = kListTab, n;
     for (;;) {  // the list this task falls in: inelastic, misc, full flights, then the segments
-      n = b.ctl->cnt[par][l];
+      n = B::ctl().cnt[par][l];
       const int k = (n + 31) >> 5;
       if (t < k) break;
       t -= k;
@@ -203,8 +202,8 @@ __device__ __forceinline__ void block_stage(const RunView<R>& v, const BlockMem<
       } else if (++l == kSegments) return;
     }
     const int i = 32 * t + lane;
-    const int slot = i < n ? (int)b.list[par][l * kBlockSlots + i] : -1;
-    block_task<R, D>(v, b, l, slot, sink, sc);
+    const int slot = i < n ? (int)B::list(par, l, i) : -1;
+    block_task<R, D>(v, l, slot, sink, sc);
   }
 }
 
@@ -212,8 +211,8 @@ __device__ __forceinline__ void block_stage(const RunView<R>& v, const BlockMem<
 // event, per electron and iteration), survivors kept in the next wave.  cap: slots a block may use.
 template <typename R, int D>
 __global__ void __launch_bounds__(kBlockThreads, kBlockPerSm) k_block(const __grid_constant__ RunView<R> v, int cur, int iters, int cap) {
-  const BlockMem<R> b(cm_stage_smem);
-  BlockCtl* c = b.ctl;
+  using B = BlockMem<R>;
+  BlockCtl& c = B::ctl();
   const int n = v.c->n[cur];
   const int grid = gridDim.x, tid = threadIdx.x, T = kBlockThreads;
   if (n == 0) return;
@@ -227,8 +226,8 @@ __global__ void __launch_bounds__(kBlockThreads, kBlockPerSm) k_block(const __gr
   quota = (quota + run - 1) / run * run;
   if (quota > cap - reserve) quota = (cap - reserve) / run * run;
   const long long dealt = (long long)quota * grid;
-  for (int i = tid; i < cap; i += T) b.free_slot[i] = (unsigned short)(cap - 1 - i);
-  for (int i = tid; i < 2 * kLists; i += T) (&c->cnt[0][0])[i] = 0;
+  for (int i = tid; i < cap; i += T) B::free_slot(i) = (unsigned short)(cap - 1 - i);
+  for (int i = tid; i < 2 * kLists; i += T) (&c.cnt[0][0])[i] = 0;
   __syncthreads();
   int mine = 0;  // electrons of the share that exist
   {
@@ -240,54 +239,54 @@ __global__ void __launch_bounds__(kBlockThreads, kBlockPerSm) k_block(const __gr
   }
   auto take = [&](int i, int slot, int par) {
     const int k = segment_of(first, i);
-    const El<R> e = load_live(v.w[cur], k * v.W + (i - first[k]));
-    b.store(slot, e);
-    b.born[slot] = 0;
-    b.put(par, k, slot);
+    const El<R> e = load_live(v.now, k * v.W + (i - first[k]));
+    B::store(slot, e);
+    B::born(slot) = 0;
+    B::put(par, k, slot);
   };
   for (int j = tid; j < mine; j += T) take((j / run * grid + (int)blockIdx.x) * run + j % run, j, 0);
   if (tid == 0) {
-    c->nfree = cap - mine;
-    c->taken = 0;
-    c->task = 0;
-    c->claim_n = 0;
-    c->exhausted = dealt >= n;
+    c.nfree = cap - mine;
+    c.taken = 0;
+    c.task = 0;
+    c.claim_n = 0;
+    c.exhausted = dealt >= n;
   }
   __syncthreads();
   StepCounts sc;
   int par = 0, it = 0;
   for (;; ++it) {
     // the last iteration runs the queued events only, so that every electron ends between two steps
-    const bool out = c->exhausted != 0;
-    const bool last = (c->nfree == cap && out) || (it >= iters && out) || it >= kBlockHardLimit;
-    BlockSink<R> sink(b, par ^ 1);
-    block_stage<R, D>(v, b, par, last, sink, sc);
+    const bool out = c.exhausted != 0;
+    const bool last = (c.nfree == cap && out) || (it >= iters && out) || it >= kBlockHardLimit;
+    BlockSink<R> sink(par ^ 1);
+    block_stage<R, D>(v, par, last, sink, sc);
     __syncthreads();
     if (last) break;
     // free slots: those the secondaries took are gone, those of the electrons that ended come back
-    const int avail = c->nfree, tk = c->taken < avail ? c->taken : avail, nd = c->cnt[par ^ 1][kListDead];
-    for (int i = tid; i < nd; i += T) b.free_slot[avail - tk + i] = b.list[par ^ 1][kListDead * kBlockSlots + i];
+    const int avail = c.nfree, tk = c.taken < avail ? c.taken : avail, nd = c.cnt[par ^ 1][kListDead];
+    for (int i = tid; i < nd; i += T) B::free_slot(avail - tk + i) = B::list(par ^ 1, kListDead, i);
     __syncthreads();
-    if (tid < kLists) c->cnt[par][tid] = 0;
+    if (tid < kLists) c.cnt[par][tid] = 0;
     if (tid == 0) {
       const int nf = avail - tk + nd, want = nf - reserve;
       int m = 0;
       if (!out && (want >= 32 || nf == cap)) {
         const long long base = dealt + atomicAdd(&v.c->claim, want);
         m = base >= n ? 0 : (n - base < want ? (int)(n - base) : want);
-        c->claim_base = (int)base;
-        if (base + want >= n) c->exhausted = 1;
+        c.claim_base = (int)base;
+        if (base + want >= n) c.exhausted = 1;
       }
-      c->claim_n = m;
-      c->nfree = nf - m;
-      c->taken = 0;
-      c->task = 0;
-      c->cnt[par ^ 1][kListDead] = 0;
+      c.claim_n = m;
+      c.nfree = nf - m;
+      c.taken = 0;
+      c.task = 0;
+      c.cnt[par ^ 1][kListDead] = 0;
     }
     __syncthreads();
-    const int m = c->claim_n;
+    const int m = c.claim_n;
     if (m > 0) {
-      for (int i = tid; i < m; i += T) take(c->claim_base + i, b.free_slot[c->nfree + i], par ^ 1);
+      for (int i = tid; i < m; i += T) take(c.claim_base + i, B::free_slot(c.nfree + i), par ^ 1);
       __syncthreads();
     }
     par ^= 1;
@@ -298,27 +297,27 @@ __global__ void __launch_bounds__(kBlockThreads, kBlockPerSm) k_block(const __gr
     DeviceSink sink;
     for (int h = 0; h < 2; ++h)
       for (int l = 0; l < kWaveSegments; ++l) {
-        const int p = par ^ h, k = c->cnt[p][l];
+        const int p = par ^ h, k = c.cnt[p][l];
         for (int i = tid; i < k; i += T) {
-          const int slot = b.list[p][l * kBlockSlots + i];
-          const El<R> e = b.load(slot);
-          if (b.born[slot]) pool_push(v, e, sink);
+          const int slot = B::list(p, l, i);
+          const El<R> e = B::load(slot);
+          if (B::born(slot)) pool_push(v, e, sink);
           else keep(v, cur ^ 1, e, l, sink);
         }
       }
     // a wave this launch did not get through is passed on as it is
-    while (!c->exhausted) {
+    while (!c.exhausted) {
       __syncthreads();
       if (tid == 0) {
         const long long base = dealt + atomicAdd(&v.c->claim, 4096);
-        c->claim_n = base >= n ? 0 : (n - base < 4096 ? (int)(n - base) : 4096);
-        c->claim_base = (int)base;
-        if (base + 4096 >= n) c->exhausted = 1;
+        c.claim_n = base >= n ? 0 : (n - base < 4096 ? (int)(n - base) : 4096);
+        c.claim_base = (int)base;
+        if (base + 4096 >= n) c.exhausted = 1;
       }
       __syncthreads();
-      for (int i = tid; i < c->claim_n; i += T) {
-        const int w = c->claim_base + i, k = segment_of(first, w);
-        keep(v, cur ^ 1, load_live(v.w[cur], k * v.W + (w - first[k])), k, sink);
+      for (int i = tid; i < c.claim_n; i += T) {
+        const int w = c.claim_base + i, k = segment_of(first, w);
+        keep(v, cur ^ 1, load_live(v.now, k * v.W + (w - first[k])), k, sink);
       }
       __syncthreads();
     }
@@ -335,8 +334,8 @@ static int block_cap(int W, int grid) {
 
 template <typename R, int D> static void launch_block_d(const RunView<R>& v, int cur, int nsm, int iters, cudaStream_t s) {
   const int grid = nsm * kBlockPerSm;
-  cudaFuncSetAttribute(k_block<R, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BlockMem<R>::bytes());
-  k_block<R, D><<<grid, kBlockThreads, BlockMem<R>::bytes(), s>>>(v, cur, iters, block_cap(v.W, grid));
+  cudaFuncSetAttribute(k_block<R, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, BlockMem<R>::kBytes);
+  k_block<R, D><<<grid, kBlockThreads, BlockMem<R>::kBytes, s>>>(v, cur, iters, block_cap(v.W, grid));
 }
 
 template <typename R> static void launch_block(const RunView<R>& v, int cur, int nsm, int iters, cudaStream_t s) {

@@ -496,7 +496,7 @@ template <typename R> CM_D R nistmott_rate(const SceneView<R>& s, const ElemRate
     if (method == 3) return q.lin * E / q.below;
     return q.sf * browning_sigma(q, a.e, a.re) * q.kbrown;
   }
-  if (E < (R)s.maxMott) {
+  if (E < s.maxMott) {
     return q.kel * ulagrange_d1(blob_at(s, q.off_spwem), 61, s.dl50, s.param, (double)a.logE);
   }
   // ScreenedRutherfordScatteringAngle.cu:24-30
@@ -522,9 +522,9 @@ template <typename R> CM_HD ElemRate<R> elem_rate(const Mott& m, int mott, int m
 }
 
 // NISTMottRS.cu:121-154 (Browning's angles below the extrapolation energy for every method)
-template <typename R, typename G> CM_D R nistmott_angle(const SceneView<R>& s, const Mott& m, int method, R E, G& g) {
-  if (E < (R)m.extrapolateBelowEnergy[method]) return browning_angle(m, E, g, (s.options & 1) != 0);
-  if (E < (R)s.maxMott) {
+template <typename R, typename G> CM_D R nistmott_angle(const SceneView<R>& s, const Mott& m, R below, R E, G& g) {
+  if (E < below) return browning_angle(m, E, g, (s.options & 1) != 0);
+  if (E < s.maxMott) {
     const double lg = log((double)E);  // double in both precisions: see ulagrange_d1
     const R u = g.next();
     const double q = ulagrange_d2(s.dbl + m.off_x1d, 61, 201, s.dl50, 0.0, s.param, 0.005, lg, (double)u);
@@ -1217,24 +1217,19 @@ template <typename R> CM_D bool is_containing_region(const SceneView<R>& s, int 
   return false;
 }
 
-// both ends of a step lie strictly inside a region described by f (see FastRegion)
-template <typename R> CM_D bool step_inside(const SceneView<R>& s, const FastRegion& f, const double* p0, const double* p1) {
+// p lies strictly inside a region described by f (see FastRegion)
+template <typename R> CM_D bool point_inside(const SceneView<R>& s, const FastRegion& f, const double* p) {
+  bool in = true;
   for (int i = 0; i < f.np; ++i) {
-    const FastPlane& P = s.fast_planes[f.plane0 + i];
-    const double a = P.n[0] * p0[0] + P.n[1] * p0[1] + P.n[2] * p0[2];
-    const double b = P.n[0] * p1[0] + P.n[1] * p1[1] + P.n[2] * p1[2];
-    if (!(a < P.d && b < P.d)) return false;
+    const FastPlane P = s.fast_planes[f.plane0 + i];
+    in = in && P.n[0] * p[0] + P.n[1] * p[1] + P.n[2] * p[2] < P.d;
   }
-  if (f.cyl < 0) return true;
+  if (f.cyl < 0 || !in) return in;
   const FastCyl& c = s.fast_cyls[f.cyl];
-  const double* const ends[2] = {p0, p1};
-  for (int k = 0; k < 2; ++k) {
-    const double q[3] = {ends[k][0] - c.e0[0], ends[k][1] - c.e0[1], ends[k][2] - c.e0[2]};
-    const double a = q[0] * c.ax[0] + q[1] * c.ax[1] + q[2] * c.ax[2];
-    const double r[3] = {q[0] - a * c.ax[0], q[1] - a * c.ax[1], q[2] - a * c.ax[2]};
-    if (!(r[0] * r[0] + r[1] * r[1] + r[2] * r[2] < c.rad2)) return false;
-  }
-  return true;
+  const double q[3] = {p[0] - c.e0[0], p[1] - c.e0[1], p[2] - c.e0[2]};
+  const double a = q[0] * c.ax[0] + q[1] * c.ax[1] + q[2] * c.ax[2];
+  const double r[3] = {q[0] - a * c.ax[0], q[1] - a * c.ax[1], q[2] - a * c.ax[2]};
+  return r[0] * r[0] + r[1] * r[1] + r[2] * r[2] < c.rad2;
 }
 
 // RegionBase.cu:74-119.  p1 is clipped to the boundary; returns the region just

@@ -892,7 +892,7 @@ static int build_scene(cm_context* ctx, DevScene<R>& ds) {
   std::vector<FastPlane> fplanes;
   std::vector<FastCyl> fcyls;
   for (const Region& r : regions) {
-    FastRegion f{r.msm, r.cls, (int)fplanes.size(), -1, -1};
+    FastRegion f{r.msm, r.cls, (int)fplanes.size(), -1, -1, {0, 0, 0}};
     if (r.nchild == 0) {
       const size_t c0 = fcyls.size();
       if (inside_of(shapes, planes, r.shape, fplanes, fcyls) && fcyls.size() - c0 <= 1) {
@@ -922,7 +922,7 @@ static int build_scene(cm_context* ctx, DevScene<R>& ds) {
   v.depth = depth;
   v.dl50 = log(0.050 * kToSIkeV * kFromSIeV);
   v.param = (log(20.0 * kToSIkeV) - log(0.050 * kToSIkeV)) / 60.0;
-  v.maxMott = 20.0 * kToSIkeV * kFromSIeV;
+  v.maxMott = (R)(20.0 * kToSIkeV * kFromSIeV);
   v.nstaged = 0;
   v.nstage = nstage;
   ++ds.gen;
@@ -941,21 +941,22 @@ template <> RunBuffers<float>& buffers_of<float>(cm_context* c) { return c->rb32
 // warp-aggregated append: one atomic per group of converged lanes
 struct DeviceSink {
   __device__ __forceinline__ int append(int* counter) {
-    cg::coalesced_group g = cg::coalesced_threads();
+    const unsigned same = __activemask();
+    const int lane = threadIdx.x & 31, leader = __ffs(same) - 1;
     int base = 0;
-    if (g.thread_rank() == 0) base = atomicAdd(counter, (int)g.size());
-    base = g.shfl(base, 0);
-    return base + (int)g.thread_rank();
+    if (lane == leader) base = atomicAdd(counter, __popc(same));
+    base = __shfl_sync(same, base, leader);
+    return base + __popc(same & ((1u << lane) - 1));
   }
   // lanes may target different counters (one per event queue): group them by
   // queue first, then one atomic per group
   __device__ __forceinline__ int append_q(int* counters, int q) {
-    cg::coalesced_group g = cg::coalesced_threads();
-    cg::coalesced_group part = cg::labeled_partition(g, q);
+    const unsigned same = __match_any_sync(__activemask(), q);
+    const int lane = threadIdx.x & 31, leader = __ffs(same) - 1;
     int base = 0;
-    if (part.thread_rank() == 0) base = atomicAdd(counters + q, (int)part.size());
-    base = part.shfl(base, 0);
-    return base + (int)part.thread_rank();
+    if (lane == leader) base = atomicAdd(counters + q, __popc(same));
+    base = __shfl_sync(same, base, leader);
+    return base + __popc(same & ((1u << lane) - 1));
   }
   __device__ __forceinline__ void count(uint32_t* h) { atomicAdd(h, 1u); }
   // counters[idx] += value, one atomic per group of converged lanes with the same idx
@@ -1255,19 +1256,8 @@ static int run_alloc(std::vector<void*>& allocs, void** p, size_t bytes) {
 }
 
 template <typename R>
-static int alloc_wave(std::vector<void*>& allocs, Wave<R>& w, int cap) {
-  auto A = [&](void** p, size_t bytes) -> int { return run_alloc(allocs, p, bytes); };
-  int rc = 0;
-  size_t n = (size_t)cap;
-  if ((rc = A((void**)&w.px, n * 8)) || (rc = A((void**)&w.py, n * 8)) || (rc = A((void**)&w.pz, n * 8)) ||
-      (rc = A((void**)&w.dx, n * sizeof(R))) || (rc = A((void**)&w.dy, n * sizeof(R))) ||
-      (rc = A((void**)&w.dz, n * sizeof(R))) || (rc = A((void**)&w.E, n * sizeof(R))) ||
-      (rc = A((void**)&w.Ep, n * sizeof(R))) || (rc = A((void**)&w.region, n * 4)) ||
-      (rc = A((void**)&w.pixel, n * 4)) || (rc = A((void**)&w.aux, n * 4)) || (rc = A((void**)&w.step, n * 4)) ||
-      (rc = A((void**)&w.key, n * 8)) || (rc = A((void**)&w.hx, n * sizeof(R))) ||
-      (rc = A((void**)&w.hy, n * sizeof(R))) || (rc = A((void**)&w.hz, n * sizeof(R))))
-    return rc;
-  return 0;
+static int alloc_wave(std::vector<void*>& allocs, Wave<R>& w, size_t cap) {
+  return run_alloc(allocs, (void**)&w.base, Wave<R>::bytes(cap));
 }
 
 // bytes of one electron record (Wave<R>): position 3 x f64, 8 fields of R, 4 int32, the u64 key
@@ -1291,8 +1281,8 @@ static int ensure_buffers(cm_context* ctx, int W, int poolCap) {
     return fail(CM_ENOMEM, msg);
   }
   int rc;
-  if ((rc = alloc_wave(rb.allocs, rb.w[0], kWaveSegments * W)) ||
-      (rc = alloc_wave(rb.allocs, rb.w[1], kWaveSegments * W)) ||
+  if ((rc = alloc_wave(rb.allocs, rb.w[0], (size_t)kWaveSegments * W)) ||
+      (rc = alloc_wave(rb.allocs, rb.w[1], (size_t)kWaveSegments * W)) ||
       (rc = alloc_wave(rb.allocs, rb.pool, poolCap))) {
     rb.release();  // nothing half-built stays behind: the next run allocates afresh
     return rc;
@@ -1326,10 +1316,18 @@ static int pool_records(int W, double emax_eV, int factor) {
 // iterations of a loop body (an even number: the waves alternate)
 constexpr int kLoopBody = 16;
 
+// the view of an iteration: the waves swap at each one (cur: which of the counters' sets is the present)
+template <typename R> static RunView<R> view_at(const RunView<R>& v, int cur) {
+  RunView<R> u = v;
+  if (cur) std::swap(u.now, u.next);
+  return u;
+}
+
 // the kernels of one transport iteration of the queue loop and of the tail loop, launched on s
 template <typename R>
-static void launch_queue_iteration(const cm_context* ctx, const RunView<R>& v, const RunView<R>& vs, int cur, int grid,
+static void launch_queue_iteration(const cm_context* ctx, const RunView<R>& v0, const RunView<R>& vs0, int cur, int grid,
                                    size_t smem, cudaStream_t s, cudaGraphConditionalHandle* h, cudaEvent_t* ev) {
+  const RunView<R> v = view_at(v0, cur), vs = view_at(vs0, cur);
   // The full flights run beside the fast ones, and the inelastic and misc events beside the elastic ones:
   // each is a few electrons whose serial latency (~50 us) would otherwise be added to every iteration.  A
   // profiled run launches them one after another, with events between them.
@@ -1370,8 +1368,9 @@ static void launch_queue_iteration(const cm_context* ctx, const RunView<R>& v, c
 }
 
 template <typename R>
-static void launch_tail_iteration(const cm_context* ctx, const RunView<R>& v, int cur, int grid, int tail_steps,
+static void launch_tail_iteration(const cm_context* ctx, const RunView<R>& v0, int cur, int grid, int tail_steps,
                                   cudaStream_t s, cudaGraphConditionalHandle* h, cudaEvent_t* ev) {
+  const RunView<R> v = view_at(v0, cur);
   launch_block(v, cur, ctx->nsm, tail_steps, s);
   if (ev) cudaEventRecordWithFlags(ev[0], s, cudaEventRecordExternal);
   launch_spawn<R>(v, cur, grid, s);
@@ -1460,21 +1459,20 @@ static int run_error(int err, const Counters& hc) {
 template <typename R> static void dump_live(const RunBuffers<R>& rb, const Counters& hc) {
   if (!getenv("CM_DEBUG_DUMP")) return;
   const int cur = hc.n[0] ? 0 : 1;
-  const int k = std::min(8, hc.n[cur]);
-  std::vector<double> px(k), py(k), pz(k);
-  std::vector<R> E(k), dz(k);
-  std::vector<int> reg(k);
-  std::vector<uint32_t> stp(k);
-  cudaMemcpy(px.data(), rb.w[cur].px, k * 8, cudaMemcpyDeviceToHost);
-  cudaMemcpy(py.data(), rb.w[cur].py, k * 8, cudaMemcpyDeviceToHost);
-  cudaMemcpy(pz.data(), rb.w[cur].pz, k * 8, cudaMemcpyDeviceToHost);
-  cudaMemcpy(E.data(), rb.w[cur].E, k * sizeof(R), cudaMemcpyDeviceToHost);
-  cudaMemcpy(dz.data(), rb.w[cur].dz, k * sizeof(R), cudaMemcpyDeviceToHost);
-  cudaMemcpy(reg.data(), rb.w[cur].region, k * 4, cudaMemcpyDeviceToHost);
-  cudaMemcpy(stp.data(), rb.w[cur].step, k * 4, cudaMemcpyDeviceToHost);
-  for (int i = 0; i < k; ++i)
-    fprintf(stderr, "live[%d] pos %g %g %g nm E %g eV dz %g region %d step %u\n", i, px[i], py[i], pz[i], (double)E[i],
-            (double)dz[i], reg[i], stp[i]);
+  for (int seg = 0; seg < kWaveSegments; ++seg) {
+    const int k = std::min(8, hc.nc[cur][seg]);
+    if (k == 0) continue;
+    // the tiles that hold the segment's first records
+    const size_t first = (size_t)seg * rb.cap, t0 = first / 32, t1 = (first + k - 1) / 32;
+    std::vector<unsigned char> host((t1 - t0 + 1) * Wave<R>::kTile);
+    cudaMemcpy(host.data(), rb.w[cur].base + t0 * Wave<R>::kTile, host.size(), cudaMemcpyDeviceToHost);
+    const Wave<R> w{host.data()};
+    for (int i = 0; i < k; ++i) {
+      const El<R> e = load_live(w, (int)(first - t0 * 32) + i);
+      fprintf(stderr, "live[%d:%d] pos %g %g %g nm E %g eV dz %g region %d step %u\n", seg, i, e.p[0], e.p[1], e.p[2],
+              (double)e.E, (double)e.d[2], e.region, e.step);
+    }
+  }
 }
 
 // Transport loop.  Inputs are device arrays.  A run launches the cached device-driven loop graph once; a
@@ -1503,8 +1501,8 @@ static int run_device_once(cm_context* ctx, const cm_run_desc* d, uint32_t* back
 #endif
   v.s = ds.view;
   v.s.chamber = d->chamber;
-  v.w[0] = rb.w[0];
-  v.w[1] = rb.w[1];
+  v.now = rb.w[0];
+  v.next = rb.w[1];
   v.pool = rb.pool;
   for (int k = 0; k < 3; ++k) v.q[k] = rb.q[k];
   v.c = ctx->counters;
@@ -1719,7 +1717,7 @@ template <typename R> __global__ void k_eval_nistmott(SceneView<R> s, int mi, in
   const ElemRate<R> q = elem_rate<R>(m, mi, method, kBohr * kBohr, 1.0);
   sig[i] = (double)nistmott_rate(s, q, method, e, mott_args(q.below, q.below, e));
   FixedRng<R> g{u + 2 * i, 2, 0};
-  th[i] = (double)nistmott_angle(s, m, method, e, g);
+  th[i] = (double)nistmott_angle(s, m, q.below, e, g);
 }
 
 template <typename R> __global__ void k_eval_table(SceneView<R> s, int t, int n, const double* x, double f0, double vf, int order,
@@ -1779,9 +1777,9 @@ template <typename R> __global__ void k_eval_elastic(SceneView<R> s, int mech, i
   const R E = (R)(q[0] * kFromSIeV);
   R d[3];
   dir_from_angles(d, (R)q[1], (R)q[2]);
-  o[0] = (double)mech_rate(s, k, E) * 1e9;
+  o[0] = (double)mech_rate(s, k, k.kind, E) * 1e9;
   FixedRng<R> g{q + 3, 4, 0};
-  const int el = elastic_scatter(s, k, d, E, g);
+  const int el = elastic_scatter<R, true>(s, k, d, E, g);
   o[1] = d[0]; o[2] = d[1]; o[3] = d[2];
   o[4] = s.mott[k.el[el].mott].Z;
   o[5] = g.used;
@@ -1797,8 +1795,8 @@ template <typename R> __global__ void k_eval_csd(SceneView<R> s, int msm, int n,
   double fr = 0, pr = 0;
   for (int k = 0; k < m.nmech; ++k) {
     const Mech<R>& mk = s.mechs[m.mech0 + k];
-    if (mk.kind == MECH_FITTED) fr = (double)mech_rate(s, mk, E) * 1e9;
-    if (mk.kind == MECH_POLARON) pr = (double)mech_rate(s, mk, E) * 1e9;
+    if (mk.kind == MECH_FITTED) fr = (double)mech_rate(s, mk, mk.kind, E) * 1e9;
+    if (mk.kind == MECH_POLARON) pr = (double)mech_rate(s, mk, mk.kind, E) * 1e9;
   }
   out[3 * i + 1] = fr;
   out[3 * i + 2] = pr;
@@ -2994,23 +2992,8 @@ struct Carve {
   }
 };
 
-template <typename R> static void carve_wave(Carve& a, Wave<R>& w, int cap) {
-  w.px = a.take<double>(cap);
-  w.py = a.take<double>(cap);
-  w.pz = a.take<double>(cap);
-  w.dx = a.take<R>(cap);
-  w.dy = a.take<R>(cap);
-  w.dz = a.take<R>(cap);
-  w.E = a.take<R>(cap);
-  w.Ep = a.take<R>(cap);
-  w.region = a.take<int>(cap);
-  w.pixel = a.take<int>(cap);
-  w.aux = a.take<int>(cap);
-  w.step = a.take<uint32_t>(cap);
-  w.key = a.take<unsigned long long>(cap);
-  w.hx = a.take<R>(cap);
-  w.hy = a.take<R>(cap);
-  w.hz = a.take<R>(cap);
+template <typename R> static void carve_wave(Carve& a, Wave<R>& w, size_t cap) {
+  w.base = a.take<unsigned char>(Wave<R>::bytes(cap));
 }
 
 template <typename R>
@@ -3035,7 +3018,7 @@ static int run_noalloc(cm_context* ctx, const cm_run_desc* d, uint32_t* back, ui
   // bytes per electron record: position (3 double), direction, pre-step
   // direction (3 R each), E and Ep (R), region, pixel, aux, step (4 B each), key (8 B)
   const size_t rec = 3 * 8 + 8 * sizeof(R) + 4 * 4 + 8;
-  const size_t pad = (3 * 16 + 3) * 256;  // worst-case rounding of the 51 pieces below
+  const size_t pad = 3 * Wave<R>::kTile + 6 * 256;  // worst-case rounding of the 6 pieces below
   const size_t left = kNoAllocScratchBytes - a.off;
   long long W = (long long)((left > pad ? left - pad : 0) / ((2 * kWaveSegments + 8) * rec + 3 * 4));
   if (d->wave > 0 && d->wave < W) W = d->wave;
@@ -3049,8 +3032,8 @@ static int run_noalloc(cm_context* ctx, const cm_run_desc* d, uint32_t* back, ui
 #endif
   v.s = ds.view;
   v.s.chamber = d->chamber;
-  carve_wave(a, v.w[0], kWaveSegments * (int)W);
-  carve_wave(a, v.w[1], kWaveSegments * (int)W);
+  carve_wave(a, v.now, (size_t)kWaveSegments * W);
+  carve_wave(a, v.next, (size_t)kWaveSegments * W);
   for (int k = 0; k < 3; ++k) v.q[k] = a.take<int>(W);
   carve_wave(a, v.pool, poolCap);
   if (a.off > kNoAllocScratchBytes) return fail(CM_EINVAL, "cm_run_noalloc: scratch layout does not fit");
@@ -3076,6 +3059,7 @@ static int run_noalloc(cm_context* ctx, const cm_run_desc* d, uint32_t* back, ui
   if (hbad)
     return fail(CM_EINVAL, "cm_run_noalloc: a pixel has a non-positive energy, a negative primary count or "
                            "pixel_nbins out of range");
+  const RunView<R> v0 = v;
   const int grid = ctx->nsm * 8;
   const int maxIt = d->max_iterations > 0 ? d->max_iterations : 500000;
   Counters hc;
@@ -3085,6 +3069,7 @@ static int run_noalloc(cm_context* ctx, const cm_run_desc* d, uint32_t* back, ui
   for (;;) {
     for (int k = 0; k < 16; ++k, ++it) {
       const int cur = it & 1;
+      const RunView<R> v = view_at(v0, cur);
       launch_flight(v, cur, grid, s);
       k_flight_fast<R><<<grid, 256, 0, s>>>(v, cur);
       k_elastic<R><<<grid, 256, 0, s>>>(v, cur);

@@ -7,8 +7,8 @@
 namespace cm {
 
 // MONSEL_MaterialScatterModel::setCache term for one mechanism (1/nm)
-template <typename R> CM_D R mech_rate(const SceneView<R>& s, const Mech<R>& k, R E) {
-  switch (k.kind) {
+template <typename R> CM_D R mech_rate(const SceneView<R>& s, const Mech<R>& k, int kind, R E) {
+  switch (kind) {
     case MECH_NISTMOTT: {  // SelectableElasticSM.cu:25-47
       R total = 0;
       const MottArgs<R> a = mott_args(k.belowMin, k.belowMax, E);
@@ -172,11 +172,14 @@ template <typename R> __host__ __device__ __noinline__ int element_pick(const Sc
 }
 
 // SelectableElasticSM::scatter (SelectableElasticSM.cu:49-67) at the step's
-// starting energy Ep; returns the element picked.
-template <typename R, typename G> CM_D int elastic_scatter(const SceneView<R>& s, const Mech<R>& k, R d[3], R Ep, G& g) {
+// starting energy Ep; returns the element picked.  Below every element's extrapolation energy the angle is
+// Browning's, which (as the reference compiles it) is isotropic whatever the element: the element is then
+// picked only when the caller asks for it (PICK).
+template <typename R, bool PICK = false, typename G>
+CM_D int elastic_scatter(const SceneView<R>& s, const Mech<R>& k, R d[3], R Ep, G& g) {
   const R u = g.next();
   int el = 0;
-  if (k.nel > 1) {
+  if (k.nel > 1 && (PICK || !(Ep < k.belowMin) || (s.options & 1))) {
     // the first element whose cumulative rate reaches u * total: the cumulative rates of the first three
     // elements stay in registers, those of a longer composition are summed again
     const MottArgs<R> a = mott_args(k.belowMin, k.belowMax, Ep);
@@ -201,7 +204,7 @@ template <typename R, typename G> CM_D int elastic_scatter(const SceneView<R>& s
       el = element_pick(s, k, Ep, r);
     }
   }
-  const R alpha = nistmott_angle(s, s.mott[k.el[el].mott], k.mottMethod, Ep, g);
+  const R alpha = nistmott_angle(s, s.mott[k.el[el].mott], k.el[el].below, Ep, g);
   const R beta = R(2 * kPi) * g.next();
   update_dir(d, alpha, beta);
   return el;

@@ -62,12 +62,13 @@ struct ChildGrid {
 // most one cylinder wall.  A step whose two ends are both in there meets no boundary, and the region test
 // and the boundary search need not run: kFastMarginNm is far above the rounding of either evaluation (at
 // most ~1e-6 nm for coordinates below 1e9 nm), so both decide alike.
-struct FastRegion {
+struct alignas(16) FastRegion {
   int msm, cls;          // as the Region's
   int plane0, np;        // half-spaces fast_planes[plane0, plane0 + np); np < 0: no such description
   int cyl;               // fast_cyls index, -1: none
+  int pad[3];
 };
-struct FastPlane {
+struct alignas(16) FastPlane {
   double n[3], d;        // inside: n . p < d
 };
 struct FastCyl {
@@ -173,9 +174,7 @@ struct Mech {
 };
 
 template <typename R>
-struct Msm {
-  int material;
-  int vacuum;
+struct alignas(16) Msm {
   int nmech, mech0;          // mechanisms [mech0, mech0+nmech)
   unsigned kinds;            // their kinds, 4 bits each, the first lowest
   int csd;                   // 0 = ZeroCSD, 1 = JoyLuoNieminenCSD
@@ -185,6 +184,8 @@ struct Msm {
   int classical;
   double lambda;
   R lambdaFactor;            // 1/sqrt(eV)
+  int material;
+  int vacuum;
   Jln<R> jln;
 };
 
@@ -227,7 +228,7 @@ struct SceneView {
   int options;               // bit 0: JMONSEL fixes, bit 1: exact CSG in FP32
   int depth;                 // deepest intersection nesting; 0 = every shape is a leaf (plane set or sphere)
   double dl50, param;        // NISTMott log-energy grid (eV)
-  double maxMott;            // NISTMottRS MAX_NISTMOTT in eV
+  R maxMott;                 // NISTMottRS MAX_NISTMOTT in eV
   int nstaged;               // elements of blob's prefix this kernel holds in shared memory (0: none)
   int nstage;                // elements of the prefix the scene places for staging (a multiple of 16 bytes)
 };

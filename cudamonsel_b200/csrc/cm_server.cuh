@@ -392,8 +392,8 @@ static int batch_round(Batcher& b) {
 #endif
   v.s = ds.view;
   v.s.chamber = 0;  // each pixel names its own chamber
-  v.w[0] = rb.w[0];
-  v.w[1] = rb.w[1];
+  v.now = rb.w[0];
+  v.next = rb.w[1];
   v.pool = rb.pool;
   for (int k = 0; k < 3; ++k) v.q[k] = rb.q[k];
   v.c = ctx->counters;
@@ -442,7 +442,7 @@ static int batch_round(Batcher& b) {
   if (!(ctx->options & CM_OPT_GLOBAL_TABLES)) vs.s.nstaged = v.s.nstage;
   const size_t smem = (size_t)vs.s.nstaged * sizeof(R);
   const LoopKey key{ds.gen, 0, grid, ctx->nsm * CM_INEL_BLOCKS_PER_SM, tu.tail_steps, (int)vs.s.nstaged};
-  if (!b.round_exec[0] || !(b.round_key == key) || b.round_buffers != (const void*)rb.w[0].px ||
+  if (!b.round_exec[0] || !(b.round_key == key) || b.round_buffers != (const void*)rb.w[0].base ||
       b.round_pool != rb.poolCap) {
     b.drop_rounds();
     for (int loop = 0; loop < 2; ++loop) {
@@ -455,7 +455,7 @@ static int batch_round(Batcher& b) {
       CM_CUDA(cudaGraphInstantiate(&b.round_exec[loop], b.round_graph[loop], 0));
     }
     b.round_key = key;
-    b.round_buffers = (const void*)rb.w[0].px;
+    b.round_buffers = (const void*)rb.w[0].base;
     b.round_pool = rb.poolCap;
   }
   // While the wave is full and no job waits for admission, kRoundRepeats rounds run back to back before

@@ -10,16 +10,44 @@
 
 namespace cm {
 
-// structure-of-arrays electron records (one per wave slot)
+// Electron records, one per wave slot, in tiles of 32: within a tile every field is an array of 32, so a
+// warp's neighbouring slots read whole lines, and one address serves every field of a record.
 template <typename R>
 struct Wave {
-  double *px, *py, *pz;
-  R *dx, *dy, *dz;
-  R *E, *Ep;
-  int *region, *pixel, *aux;
-  uint32_t* step;
-  unsigned long long* key;
-  R *hx, *hy, *hz;
+  unsigned char* base;
+  static constexpr size_t kTile = 32 * (4 * 8 + 8 * sizeof(R) + 4 * 4);
+  CM_D static size_t bytes(size_t cap) { return (cap + 31) / 32 * kTile; }
+};
+
+// the fields of one record (base pointers of its lane in the tile)
+template <typename R>
+struct Rec {
+  double* f;  // position, key
+  R* r;       // direction, E, Ep, hit normal
+  int* w;     // region, pixel, aux, step
+  CM_D Rec(const Wave<R>& v, int i) {
+    unsigned char* t = v.base + (size_t)((unsigned)i >> 5) * Wave<R>::kTile;
+    const int lane = i & 31;
+    f = (double*)t + lane;
+    r = (R*)(t + 32 * 4 * 8) + lane;
+    w = (int*)(t + 32 * (4 * 8 + 8 * sizeof(R))) + lane;
+  }
+  CM_D double& px() const { return f[0]; }
+  CM_D double& py() const { return f[32]; }
+  CM_D double& pz() const { return f[64]; }
+  CM_D unsigned long long& key() const { return ((unsigned long long*)f)[96]; }
+  CM_D R& dx() const { return r[0]; }
+  CM_D R& dy() const { return r[32]; }
+  CM_D R& dz() const { return r[64]; }
+  CM_D R& E() const { return r[96]; }
+  CM_D R& Ep() const { return r[128]; }
+  CM_D R& hx() const { return r[160]; }
+  CM_D R& hy() const { return r[192]; }
+  CM_D R& hz() const { return r[224]; }
+  CM_D int& region() const { return w[0]; }
+  CM_D int& pixel() const { return w[32]; }
+  CM_D int& aux() const { return w[64]; }
+  CM_D uint32_t& step() const { return ((uint32_t*)w)[96]; }
 };
 
 struct Counters {
@@ -54,57 +82,66 @@ struct El {
   R h[3];
 };
 
-template <typename R> CM_D El<R> load(const Wave<R>& w, int i) {
-  El<R> e;
-  e.p[0] = w.px[i]; e.p[1] = w.py[i]; e.p[2] = w.pz[i];
-  e.d[0] = w.dx[i]; e.d[1] = w.dy[i]; e.d[2] = w.dz[i];
-  e.E = w.E[i]; e.Ep = w.Ep[i];
-  e.region = w.region[i]; e.pixel = w.pixel[i]; e.aux = w.aux[i];
-  e.step = w.step[i]; e.key = w.key[i];
-  e.h[0] = w.hx[i]; e.h[1] = w.hy[i]; e.h[2] = w.hz[i];
-  return e;
-}
-
 // The fields a step starts from (position, direction, energy, region, pixel, step count, key).  Ep, aux
 // and the hit normal are written by the flight for its event and read only by that event, so records
 // moved between waves and the pool carry the live fields alone (60 of 80 bytes in FP32).
-template <typename R> CM_D El<R> load_live(const Wave<R>& w, int i) {
+template <typename R> CM_D El<R> load_live(const Wave<R>& v, int i) {
+  const Rec<R> w(v, i);
   El<R> e;
-  e.p[0] = w.px[i]; e.p[1] = w.py[i]; e.p[2] = w.pz[i];
-  e.d[0] = w.dx[i]; e.d[1] = w.dy[i]; e.d[2] = w.dz[i];
-  e.E = w.E[i];
-  e.region = w.region[i]; e.pixel = w.pixel[i];
-  e.step = w.step[i]; e.key = w.key[i];
+  e.p[0] = w.px(); e.p[1] = w.py(); e.p[2] = w.pz();
+  e.d[0] = w.dx(); e.d[1] = w.dy(); e.d[2] = w.dz();
+  e.E = w.E();
+  e.region = w.region(); e.pixel = w.pixel();
+  e.step = w.step(); e.key = w.key();
   return e;
 }
 
-template <typename R> CM_D void store_live(const Wave<R>& w, int i, const El<R>& e) {
-  w.px[i] = e.p[0]; w.py[i] = e.p[1]; w.pz[i] = e.p[2];
-  w.dx[i] = e.d[0]; w.dy[i] = e.d[1]; w.dz[i] = e.d[2];
-  w.E[i] = e.E;
-  w.region[i] = e.region; w.pixel[i] = e.pixel;
-  w.step[i] = e.step; w.key[i] = e.key;
+template <typename R> CM_D void store_live(const Wave<R>& v, int i, const El<R>& e) {
+  const Rec<R> w(v, i);
+  w.px() = e.p[0]; w.py() = e.p[1]; w.pz() = e.p[2];
+  w.dx() = e.d[0]; w.dy() = e.d[1]; w.dz() = e.d[2];
+  w.E() = e.E;
+  w.region() = e.region; w.pixel() = e.pixel;
+  w.step() = e.step; w.key() = e.key;
 }
 
 // what an elastic or inelastic event reads: the live fields, the step's starting energy and the mechanism
-template <typename R> CM_D El<R> load_event(const Wave<R>& w, int i) {
-  El<R> e = load_live(w, i);
-  e.Ep = w.Ep[i];
-  e.aux = w.aux[i];
+template <typename R> CM_D El<R> load_event(const Wave<R>& v, int i) {
+  El<R> e = load_live(v, i);
+  const Rec<R> w(v, i);
+  e.Ep = w.Ep();
+  e.aux = w.aux();
   return e;
 }
 
-// wave segment of an electron in `region` at energy E: its material's class, split at kSegmentSplitEv
-template <typename R> CM_D int wave_segment(const SceneView<R>& s, int region, R E) {
-  if (region < 0 || s.fast[region].np < 0) return kSlowSegment;
-  return 2 * s.fast[region].cls + (E < (R)kSegmentSplitEv ? 1 : 0);
+// ... and a misc event, which may be a boundary crossing
+template <typename R> CM_D El<R> load(const Wave<R>& v, int i) {
+  El<R> e = load_event(v, i);
+  const Rec<R> w(v, i);
+  e.h[0] = w.hx(); e.h[1] = w.hy(); e.h[2] = w.hz();
+  return e;
 }
 
 enum { Q_EL = 0, Q_TAB = 1, Q_MISC = 2, Q_SLOW = 3 };
 enum { AUX_MECH = 1, AUX_BARRIER = 2, AUX_PASS = 3 };
 CM_HD int aux_pack(int kind, int v) { return (kind << 24) | (v & 0xffffff); }
-CM_HD int aux_kind(int a) { return a >> 24; }
+constexpr int AUX_INSIDE = 1 << 28;  // the electron is strictly inside its region (FastRegion)
+CM_HD int aux_kind(int a) { return (a >> 24) & 15; }
 CM_HD int aux_val(int a) { return a & 0xffffff; }
+
+// Wave segment of an electron: its material's class, split at kSegmentSplitEv, when it is strictly inside
+// its region (which the fast flight takes as given), else the slow segment.  inside: known to be.
+template <typename R> CM_D int wave_segment(const SceneView<R>& s, const El<R>& e, bool inside = false) {
+  if (e.region < 0) return kSlowSegment;
+  const FastRegion f = s.fast[e.region];
+  if (!inside && (f.np < 0 || !point_inside(s, f, e.p))) return kSlowSegment;
+  return 2 * f.cls + (e.E < (R)kSegmentSplitEv ? 1 : 0);
+}
+
+// the segment after an event: an electron at a boundary just met is within the margin of it
+template <typename R> CM_D int segment_after(const SceneView<R>& s, const El<R>& e) {
+  return aux_kind(e.aux) == AUX_BARRIER ? kSlowSegment : wave_segment(s, e, (e.aux & AUX_INSIDE) != 0);
+}
 
 #ifdef CM_TRACE
 // step records of a debugging build (never compiled into the library)
@@ -161,7 +198,7 @@ struct RunView {
   int tracecap;
 #endif
   SceneView<R> s;
-  Wave<R> w[2];
+  Wave<R> now, next;  // the iteration's wave and the one it fills
   Wave<R> pool;
   int* q[3];
   Counters* c;
@@ -260,7 +297,7 @@ template <typename R> CM_D int chamber_of(const RunView<R>& v, int px) {
 template <typename R> __host__ __device__ __noinline__ int mech_pick_long(const SceneView<R>& s, const Msm<R>& m, R E, R r) {
   R c = 0;
   for (int k = 0; k < m.nmech - 1; ++k) {
-    c += mech_rate(s, s.mechs[m.mech0 + k], E);
+    c += mech_rate(s, s.mechs[m.mech0 + k], (m.kinds >> (4 * k)) & 15, E);
     if (!(c < r)) return k;
   }
   return m.nmech - 1;
@@ -275,7 +312,7 @@ template <typename R> struct MsmRates {
 template <typename R> CM_D MsmRates<R> msm_rates(const SceneView<R>& s, const Msm<R>& m, R E) {
   MsmRates<R> q{0, 0, 0, 0};
   for (int k = 0; k < m.nmech; ++k) {
-    q.total += mech_rate(s, s.mechs[m.mech0 + k], E);
+    q.total += mech_rate(s, s.mechs[m.mech0 + k], (m.kinds >> (4 * k)) & 15, E);
     q.c0 = k == 0 ? q.total : q.c0;
     q.c1 = k == 1 ? q.total : q.c1;
     q.c2 = k == 2 ? q.total : q.c2;
@@ -307,34 +344,35 @@ template <typename R> CM_D int mech_pick(const SceneView<R>& s, const Msm<R>& m,
 // or, when pixel_src is given, read from there if the electron escapes): the event queue of its end, or
 // -1 when the electron ended here (escaped and tallied, stopped, trapped).
 //
-// FAST: the step of an electron that stays strictly inside a childless region, without the region test,
+// FAST: the step of an electron strictly inside a childless region that stays so, without the region test,
 // the boundary search, crossings and escapes; Q_SLOW, with nothing changed or counted, when this step may
 // need them (the full form then takes it from the start: the random stream is keyed by the step).
 template <typename R, int D, bool FAST = false, typename Sink>
 CM_D int flight_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc, const int* pixel_src = nullptr) {
   const SceneView<R>& s = v.s;
   int reg = e.region;
+  const FastRegion f = FAST ? s.fast[reg] : FastRegion();
   if (FAST) {
-    if (reg < 0 || s.fast[reg].np < 0) return Q_SLOW;
   } else if (reg < 0 || !shape_contains<R, D>(s, s.regions[reg].shape, e.p))
     reg = containing_subregion<R, D>(s, chamber_of(v, pixel_src ? *pixel_src : e.pixel), e.p);
   if (reg < 0) return -1;
-  const Msm<R>& m = s.msms[FAST ? s.fast[reg].msm : s.regions[reg].msm];
+  const Msm<R>& m = s.msms[FAST ? f.msm : s.regions[reg].msm];
   bool complete = false;
   double fp = 2.0 * kChamberRadiusNm;
   R total = 0;
   int idx = 0, kind = 0;
   {
     Rng<R> g(e.key, e.step, 0);
+    const R u0 = g.next(), u1 = g.next();
     const MsmRates<R> rates = msm_rates(s, m, e.E);
     total = rates.total;
     if (total != R(0)) {
-      const R f = -mlog(g.next()) / total;
-      if ((double)f < fp) fp = (double)f;
+      const R path = -mlog(u0) / total;
+      if ((double)path < fp) fp = (double)path;
       // MONSEL_MaterialScatterModel::scatter (:93-134) picks the mechanism from the rates at the
       // step's starting energy with the stream's next deviate; it is drawn here, before the
       // geometry, so that the rates need not stay live (nothing else draws from this stream)
-      idx = mech_pick(s, m, e.E, rates, g.next() * total);
+      idx = mech_pick(s, m, e.E, rates, u1 * total);
       kind = (m.kinds >> (4 * idx)) & 15;
     } else if (FAST) {
       return Q_SLOW;
@@ -355,7 +393,7 @@ CM_D int flight_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc,
   double p1[3] = {e.p[0] + fp * (double)e.d[0], e.p[1] + fp * (double)e.d[1], e.p[2] + fp * (double)e.d[2]};
   double hn[3];
   bool clipped = false;
-  if (FAST && !step_inside(s, s.fast[reg], e.p, p1)) return Q_SLOW;
+  if (FAST && !point_inside(s, f, p1)) return Q_SLOW;
   const int next = FAST ? reg : find_end_of_step<R, D>(s, reg, e.p, p1, hn, &clipped);
   const double dd = sqrt((p1[0] - e.p[0]) * (p1[0] - e.p[0]) + (p1[1] - e.p[1]) * (p1[1] - e.p[1]) +
                          (p1[2] - e.p[2]) * (p1[2] - e.p[2]));
@@ -386,7 +424,7 @@ CM_D int flight_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc,
     } else {
       if (kind == MECH_POLARON) return -1;  // GanachaudMokraniPolaronTrapSM::scatter: trapped, E = 0
       queue = kind == MECH_NISTMOTT ? Q_EL : kind == MECH_TABULATED ? Q_TAB : Q_MISC;
-      e.aux = aux_pack(AUX_MECH, idx);
+      e.aux = aux_pack(AUX_MECH, idx) | (FAST ? AUX_INSIDE : 0);
     }
   } else if (next >= 0) {
     ++sc.bar;
@@ -411,7 +449,7 @@ CM_D int flight_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc,
 // append an electron to segment k of the next wave
 template <typename R, typename Sink> CM_D void keep(const RunView<R>& v, int nxt, const El<R>& e, int k, Sink& sink) {
   const int slot = sink.append_q(v.c->nc[nxt], k);
-  store_live(v.w[nxt], k * v.W + slot, e);
+  store_live(v.next, k * v.W + slot, e);
 }
 
 // The flight of wave slot i: reads what the step uses and writes back only what it changes
@@ -419,43 +457,33 @@ template <typename R, typename Sink> CM_D void keep(const RunView<R>& v, int nxt
 // FAST: an electron whose step needs the full form goes to the next wave's slow segment as it is.
 template <typename R, int D, bool FAST, typename Sink>
 CM_D void flight_one(const RunView<R>& v, int cur, int i, Sink& sink, StepCounts& sc) {
-  const Wave<R>& W = v.w[cur];
+  const Rec<R> w(v.now, i);
   El<R> e;
-  e.p[0] = W.px[i]; e.p[1] = W.py[i]; e.p[2] = W.pz[i];
-  e.d[0] = W.dx[i]; e.d[1] = W.dy[i]; e.d[2] = W.dz[i];
-  e.E = W.E[i];
-  e.step = W.step[i];
-  e.region = W.region[i];
-  e.key = W.key[i];
-  const int queue = flight_apply<R, D, FAST>(v, e, sink, sc, W.pixel + i);  // the pixel is read only on escape
+  e.p[0] = w.px(); e.p[1] = w.py(); e.p[2] = w.pz();
+  e.d[0] = w.dx(); e.d[1] = w.dy(); e.d[2] = w.dz();
+  e.E = w.E();
+  e.step = w.step();
+  e.region = w.region();
+  e.key = w.key();
+  const int queue = flight_apply<R, D, FAST>(v, e, sink, sc, &w.pixel());  // the pixel is read only on escape
   if (queue < 0) {
-    if (v.io->job_alive) job_end(v, W.pixel[i], e.step, sink);
+    if (v.io->job_alive) job_end(v, w.pixel(), e.step, sink);
     return;
   }
   if (FAST && queue == Q_SLOW) {
-    e.pixel = W.pixel[i];
+    e.pixel = w.pixel();
     keep(v, cur ^ 1, e, kSlowSegment, sink);
     sink.append(&v.c->deferred);
     return;
   }
-  W.px[i] = e.p[0]; W.py[i] = e.p[1]; W.pz[i] = e.p[2];
-  W.E[i] = e.E; W.Ep[i] = e.Ep;
-  W.aux[i] = e.aux;
-  W.step[i] = e.step;
-  if (!FAST) W.region[i] = e.region;  // a FAST step stays in its region
-  if (!FAST && aux_kind(e.aux) == AUX_BARRIER) { W.hx[i] = e.h[0]; W.hy[i] = e.h[1]; W.hz[i] = e.h[2]; }
+  w.px() = e.p[0]; w.py() = e.p[1]; w.pz() = e.p[2];
+  w.E() = e.E; w.Ep() = e.Ep;
+  w.aux() = e.aux;
+  w.step() = e.step;
+  if (!FAST) w.region() = e.region;  // a FAST step stays in its region
+  if (!FAST && aux_kind(e.aux) == AUX_BARRIER) { w.hx() = e.h[0]; w.hy() = e.h[1]; w.hz() = e.h[2]; }
   const int slot = sink.append_q(v.c->q, queue);
   v.q[queue][slot] = i;
-}
-
-// wave index of the i-th electron of a wave counted over its class segments in order
-CM_D int wave_index(const Counters* c, int cur, int W, int i) {
-  int k = 0;
-  while (k < kWaveSegments - 1 && i >= c->nc[cur][k]) {
-    i -= c->nc[cur][k];
-    ++k;
-  }
-  return k * W + i;
 }
 
 CM_D int survivors(const Counters* c, int nxt) {
@@ -552,28 +580,23 @@ template <typename R, int D, typename Sink> CM_D bool misc_apply(const RunView<R
   return !(e.E < m.minE);
 }
 
-// the segment after a misc event: an electron at a boundary is within the fast flight's margin of it
-template <typename R> CM_D int segment_after_misc(const RunView<R>& v, const El<R>& e) {
-  return aux_kind(e.aux) == AUX_BARRIER ? kSlowSegment : wave_segment(v.s, e.region, e.E);
-}
-
 // the queue kernels' events: the record of queue entry j, its event, and the survivor kept
 template <typename R, typename Sink> CM_D void elastic_one(const RunView<R>& v, int cur, int j, Sink& sink) {
-  El<R> e = load_event(v.w[cur], v.q[Q_EL][j]);
-  if (elastic_apply(v, e)) keep(v, cur ^ 1, e, wave_segment(v.s, e.region, e.E), sink);
+  El<R> e = load_event(v.now, v.q[Q_EL][j]);
+  if (elastic_apply(v, e)) keep(v, cur ^ 1, e, segment_after(v.s, e), sink);
   else job_end(v, e.pixel, e.step, sink);
 }
 
 template <typename R, typename Sink> CM_D void inelastic_one(const RunView<R>& v, int cur, int j, Sink& sink, StepCounts& sc) {
-  El<R> e = load_event(v.w[cur], v.q[Q_TAB][j]);
-  if (inelastic_apply(v, e, sink, sc)) keep(v, cur ^ 1, e, wave_segment(v.s, e.region, e.E), sink);
+  El<R> e = load_event(v.now, v.q[Q_TAB][j]);
+  if (inelastic_apply(v, e, sink, sc)) keep(v, cur ^ 1, e, segment_after(v.s, e), sink);
   else job_end(v, e.pixel, e.step, sink);
 }
 
 template <typename R, int D, typename Sink>
 CM_D void misc_one(const RunView<R>& v, int cur, int j, Sink& sink, StepCounts& sc) {
-  El<R> e = load(v.w[cur], v.q[Q_MISC][j]);
-  if (misc_apply<R, D>(v, e, sink, sc)) keep(v, cur ^ 1, e, segment_after_misc(v, e), sink);
+  El<R> e = load(v.now, v.q[Q_MISC][j]);
+  if (misc_apply<R, D>(v, e, sink, sc)) keep(v, cur ^ 1, e, segment_after(v.s, e), sink);
   else job_end(v, e.pixel, e.step, sink);
 }
 
@@ -600,8 +623,8 @@ CM_D void spawn_one(const RunView<R>& v, int nxt, int j, int take_se, int poolTo
                     Sink& sink) {
   if (j < take_se) {
     const El<R> se = load_live(v.pool, poolTop - 1 - j);
-    const int seg = wave_segment(v.s, se.region, se.E);
-    store_live(v.w[nxt], seg * v.W + v.c->nc[nxt][seg] + sink.append_q(v.c->ns, seg), se);
+    const int seg = wave_segment(v.s, se);
+    store_live(v.next, seg * v.W + v.c->nc[nxt][seg] + sink.append_q(v.c->ns, seg), se);
     return;
   }
   // GaussianBeam::createElectron (NISTMonte/GaussianBeam.cu:52-65) + initializeTrajectory (MonteCarloSS.cu:99-105)
@@ -633,8 +656,8 @@ CM_D void spawn_one(const RunView<R>& v, int nxt, int j, int take_se, int poolTo
   e.aux = 0;
   e.step = 0;
   e.h[0] = e.h[1] = e.h[2] = 0;
-  const int seg = wave_segment(v.s, e.region, e.E);
-  store_live(v.w[nxt], seg * v.W + v.c->nc[nxt][seg] + sink.append_q(v.c->ns, seg), e);
+  const int seg = wave_segment(v.s, e);
+  store_live(v.next, seg * v.W + v.c->nc[nxt][seg] + sink.append_q(v.c->ns, seg), e);
   job_start(v, px, sink);
 }
 
