@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(kBlockThreads, kBlockPerSm) k_block(const __gr
       const int nf = avail - tk + nd, want = nf - reserve;
       int m = 0;
       if (!out && (want >= 32 || nf == cap)) {
-        const long long base = dealt + atomicAdd(&v.c->claim, want);
+        const long long base = dealt + atomicAdd(&v.c->claim.v, want);
         m = base >= n ? 0 : (n - base < want ? (int)(n - base) : want);
         c.claim_base = (int)base;
         if (base + want >= n) c.exhausted = 1;
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kBlockThreads, kBlockPerSm) k_block(const __gr
     while (!c.exhausted) {
       __syncthreads();
       if (tid == 0) {
-        const long long base = dealt + atomicAdd(&v.c->claim, 4096);
+        const long long base = dealt + atomicAdd(&v.c->claim.v, 4096);
         c.claim_n = base >= n ? 0 : (n - base < 4096 ? (int)(n - base) : 4096);
         c.claim_base = (int)base;
         if (base + 4096 >= n) c.exhausted = 1;

@@ -950,11 +950,11 @@ struct DeviceSink {
   }
   // lanes may target different counters (one per event queue): group them by
   // queue first, then one atomic per group
-  __device__ __forceinline__ int append_q(int* counters, int q) {
+  __device__ __forceinline__ int append_q(Line* counters, int q) {
     const unsigned same = __match_any_sync(__activemask(), q);
     const int lane = threadIdx.x & 31, leader = __ffs(same) - 1;
     int base = 0;
-    if (lane == leader) base = atomicAdd(counters + q, __popc(same));
+    if (lane == leader) base = atomicAdd(&counters[q].v, __popc(same));
     base = __shfl_sync(same, base, leader);
     return base + __popc(same & ((1u << lane) - 1));
   }
@@ -1012,17 +1012,60 @@ template <typename R> __device__ __forceinline__ bool stage_tables(const RunView
   return __syncthreads_and(done) != 0;
 }
 
-__device__ __forceinline__ void flush_counts(Counters* c, StepCounts& sc) {
-  // a thread counts one launch's steps in 32 bits; the warp's sums and the run's totals are 64-bit
+// the block's step counts added to the run's totals: one atomic per total and block (one per warp would
+// have tens of thousands of them queue for one cache line in every launch).  Every thread calls it.
+__device__ __forceinline__ void flush_counts(Counters* c, const StepCounts& sc) {
+  __shared__ unsigned long long sums[7];
+  if (threadIdx.x < 7) sums[threadIdx.x] = 0;
+  __syncthreads();
+  // a thread counts one launch's steps in 32 bits; the sums are 64-bit
   const unsigned int mine[7] = {sc.steps, sc.scat, sc.bar, sc.esc, sc.sec, sc.zero, sc.limit};
-  unsigned long long* const total[7] = {&c->steps,       &c->scatters,   &c->barriers,   &c->escapes,
-                                        &c->secondaries, &c->ended_zero, &c->ended_limit};
 #pragma unroll
   for (int k = 0; k < 7; ++k) {
     unsigned long long sum = mine[k];
     for (int off = 16; off > 0; off >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, off);
-    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(total[k], sum);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(&sums[k], sum);
   }
+  __syncthreads();
+  if (threadIdx.x < 7 && sums[threadIdx.x]) {
+    unsigned long long* const total[7] = {&c->steps,       &c->scatters,   &c->barriers,   &c->escapes,
+                                          &c->secondaries, &c->ended_zero, &c->ended_limit};
+    unsigned long long* t = total[0];
+#pragma unroll
+    for (int k = 1; k < 7; ++k) t = threadIdx.x == k ? total[k] : t;
+    atomicAdd(t, sums[threadIdx.x]);
+  }
+}
+
+// Appends by whole blocks: every thread calls slot() with the list its item joins (0..K-1, or -1) and gets
+// the item's place in it.  Warps count in shared memory and one thread per list reserves the block's places
+// with one global atomic.  One atomic per warp and list instead, ~70 k per launch of a full wave on a few
+// addresses, took most of the flight's time: it ran as fast at 16 resident warps per SM as at 32.
+template <int K> struct BlockAppend {
+  int cnt[2][K];
+  int base[K];
+};
+template <int K> __device__ __forceinline__ void append_init(BlockAppend<K>& a) {
+  if (threadIdx.x < 2 * K) (&a.cnt[0][0])[threadIdx.x] = 0;
+  __syncthreads();
+}
+// counter(k): the global counter of list k; par alternates between calls
+template <int K, typename F>
+__device__ __forceinline__ int append_slot(BlockAppend<K>& a, int par, int list, F counter) {
+  __syncwarp();
+  const unsigned same = __match_any_sync(0xffffffffu, list);
+  const int lane = threadIdx.x & 31, leader = __ffs(same) - 1;
+  int w = 0;
+  if (list >= 0 && lane == leader) w = atomicAdd(&a.cnt[par][list], __popc(same));
+  w = __shfl_sync(0xffffffffu, w, leader);
+  __syncthreads();
+  if (threadIdx.x < K) {
+    const int n = a.cnt[par][threadIdx.x];
+    if (n) a.base[threadIdx.x] = atomicAdd(counter(threadIdx.x), n);
+    a.cnt[par ^ 1][threadIdx.x] = 0;
+  }
+  __syncthreads();
+  return list < 0 ? -1 : a.base[list] + w + __popc(same & ((1u << lane) - 1));
 }
 
 // Where each class segment of wave `cur` starts in the order the threads take its electrons, in the block's
@@ -1054,9 +1097,24 @@ template <typename R> __device__ __forceinline__ void flight_fast_loop(const Run
   if ((int)(blockIdx.x * blockDim.x) >= n) return;
   __shared__ int first[kWaveSegments + 1];
   segment_starts(v.c, cur, first);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int k = segment_of(first, i);  // the i-th electron over the class segments in order
-    flight_one<R, 0, true>(v, cur, k * v.W + (i - first[k]), sink, sc);
+  __shared__ BlockAppend<4> app;
+  append_init(app);
+  int par = 0;
+  for (int i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x, par ^= 1) {
+    const int i = i0 + threadIdx.x;
+    int dest = -1, w = 0;
+    if (i < n) {
+      const int k = segment_of(first, i);  // the i-th electron over the class segments in order
+      w = k * v.W + (i - first[k]);
+      dest = flight_one<R, 0, true>(v, w, sink, sc);
+    }
+    const int slot = append_slot(app, par, dest, [&](int k) {
+      if (k < Q_SLOW) return &v.c->q[k].v;
+      atomicAdd(&v.c->deferred.v, app.cnt[par][Q_SLOW]);
+      return &v.c->nc[cur ^ 1][kSlowSegment].v;
+    });
+    if (dest == Q_SLOW) store_live(v.next, kSlowSegment * v.W + slot, load_live(v.now, w));
+    else if (dest >= 0) v.q[dest][slot] = w;
   }
   flush_counts(v.c, sc);
 }
@@ -1078,8 +1136,16 @@ template <typename R, int D> __global__ void __launch_bounds__(256) k_flight(con
   StepCounts sc;
   const int n = v.c->nc[cur][kSlowSegment];
   if ((int)(blockIdx.x * blockDim.x) >= n) return;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
-    flight_one<R, D, false>(v, cur, kSlowSegment * v.W + j, sink, sc);
+  __shared__ BlockAppend<3> app;
+  append_init(app);
+  int par = 0;
+  for (int j0 = blockIdx.x * blockDim.x; j0 < n; j0 += gridDim.x * blockDim.x, par ^= 1) {
+    const int w = kSlowSegment * v.W + j0 + threadIdx.x;
+    int dest = -1;
+    if (j0 + (int)threadIdx.x < n) dest = flight_one<R, D, false>(v, w, sink, sc);
+    const int slot = append_slot(app, par, dest, [&](int k) { return &v.c->q[k].v; });
+    if (dest >= 0) v.q[dest][slot] = w;
+  }
   flush_counts(v.c, sc);
 }
 
@@ -1114,13 +1180,28 @@ template <typename R, int D> __global__ void __launch_bounds__(256) k_flight(con
 #define CM_LB_INELASTIC __launch_bounds__(256)
 #endif
 
+// the events of a queue's n entries, survivors appended to their segments of the next wave
+template <typename R, typename F>
+__device__ __forceinline__ void event_loop(const RunView<R>& v, int cur, int n, F event) {
+  __shared__ BlockAppend<kWaveSegments> app;
+  append_init(app);
+  int par = 0;
+  for (int j0 = blockIdx.x * blockDim.x; j0 < n; j0 += gridDim.x * blockDim.x, par ^= 1) {
+    El<R> e;
+    int dest = -1;
+    if (j0 + (int)threadIdx.x < n) dest = event(j0 + (int)threadIdx.x, e);
+    const int slot = append_slot(app, par, dest, [&](int k) { return &v.c->nc[cur ^ 1][k].v; });
+    if (dest >= 0) store_live(v.next, dest * v.W + slot, e);
+  }
+}
+
 // k_elastic runs at 4 CTAs per SM (64 registers, a few spills): linescan +2 %.
 template <typename R>
 __global__ void CM_LB_ELASTIC k_elastic(const __grid_constant__ RunView<R> v, int cur) {
   DeviceSink sink;
   const int n = v.c->q[Q_EL];
   if ((int)(blockIdx.x * blockDim.x) >= n || !stage_tables(v)) return;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) elastic_one(v, cur, j, sink);
+  event_loop(v, cur, n, [&](int j, El<R>& e) { return elastic_one(v, j, e, sink); });
 }
 
 template <typename R>
@@ -1129,7 +1210,7 @@ __global__ void CM_LB_INELASTIC k_inelastic(const __grid_constant__ RunView<R> v
   StepCounts sc;
   const int n = v.c->q[Q_TAB];
   if ((int)(blockIdx.x * blockDim.x) >= n || !stage_tables(v)) return;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) inelastic_one(v, cur, j, sink, sc);
+  event_loop(v, cur, n, [&](int j, El<R>& e) { return inelastic_one(v, j, e, sink, sc); });
   flush_counts(v.c, sc);
 }
 
@@ -1138,8 +1219,8 @@ __global__ void __launch_bounds__(256) k_misc(const __grid_constant__ RunView<R>
   DeviceSink sink;
   StepCounts sc;
   const int n = v.c->q[Q_MISC];
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
-    misc_one<R, D>(v, cur, j, sink, sc);
+  if ((int)(blockIdx.x * blockDim.x) >= n) return;
+  event_loop(v, cur, n, [&](int j, El<R>& e) { return misc_one<R, D>(v, j, e, sink, sc); });
   flush_counts(v.c, sc);
 }
 
@@ -1187,9 +1268,19 @@ __global__ void __launch_bounds__(256) k_spawn(const __grid_constant__ RunView<R
   refill_plan(v.c, nxt, v.W, v.poolCap, nn, take_se, take_p);
   const int poolTop = v.c->pool < v.poolCap ? v.c->pool : v.poolCap;
   const unsigned long long first = v.c->next_primary;
+  const int n = take_se + take_p;
+  if ((int)(blockIdx.x * blockDim.x) >= n) return;
   DeviceSink sink;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < take_se + take_p; j += gridDim.x * blockDim.x)
-    spawn_one<R, D>(v, nxt, j, take_se, poolTop, first, sink);
+  __shared__ BlockAppend<kWaveSegments> app;
+  append_init(app);
+  int par = 0;
+  for (int j0 = blockIdx.x * blockDim.x; j0 < n; j0 += gridDim.x * blockDim.x, par ^= 1) {
+    El<R> e;
+    int dest = -1;
+    if (j0 + (int)threadIdx.x < n) dest = spawn_one<R, D>(v, j0 + (int)threadIdx.x, take_se, poolTop, first, e, sink);
+    const int slot = append_slot(app, par, dest, [&](int k) { return &v.c->ns[k].v; });
+    if (dest >= 0) store_live(v.next, dest * v.W + v.c->nc[nxt][dest] + slot, e);
+  }
 }
 
 template <typename R> static void launch_spawn(const RunView<R>& v, int cur, int grid, cudaStream_t s) {
@@ -1229,9 +1320,11 @@ __global__ void k_loop(const __grid_constant__ RunView<R> v, int cur, int steps,
   cudaGraphSetConditional(h, go ? 1u : 0u);
 }
 
-// opens a loop of the device-driven run unless the run is already done or failed
-__global__ void k_gate(const Counters* c, cudaGraphConditionalHandle h) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(h, (!c->done && !c->error) ? 1u : 0u);
+// opens a loop of the device-driven run unless the run is already done or failed; the queue loop also not
+// when the run starts in the tail loop
+__global__ void k_gate(const Counters* c, const RunIO* io, int queue, cudaGraphConditionalHandle h) {
+  if (blockIdx.x == 0 && threadIdx.x == 0)
+    cudaGraphSetConditional(h, (!c->done && !c->error && !(queue && io->start_tail)) ? 1u : 0u);
 }
 
 #ifdef CM_TRACE
@@ -1313,8 +1406,11 @@ static int pool_records(int W, double emax_eV, int factor) {
   return (int)std::min<double>(f * (double)W, (double)(1 << 30));
 }
 
-// iterations of a loop body (an even number: the waves alternate)
+// iterations of a replayed or served round (an even number: the waves alternate), and of the bodies of the
+// device-driven loops: a body runs to its end, so the iterations after a loop's last are idle launches
+// (~3 us each), and each turn of a loop costs ~8 us
 constexpr int kLoopBody = 16;
+constexpr int kQueueBody = 16, kTailBody = 2;
 
 // the view of an iteration: the waves swap at each one (cur: which of the counters' sets is the present)
 template <typename R> static RunView<R> view_at(const RunView<R>& v, int cur) {
@@ -1380,6 +1476,13 @@ static void launch_tail_iteration(const cm_context* ctx, const RunView<R>& v0, i
   if (ev) cudaEventRecordWithFlags(ev[2], s, cudaEventRecordExternal);
 }
 
+// A run whose electrons never fill the GPU (about one more per 100 eV of a primary's energy is alive at the
+// peak of its cascade) starts in the tail loop; the queue kernels would move its first steps at ~60 us an
+// iteration.  A run with an iteration limit keeps to the queue loop first, whose iterations the limit counts.
+static bool starts_in_tail(unsigned long long total, double emax_eV, int tail_below) {
+  return (double)total * (1.0 + emax_eV / 100.0) < (double)tail_below;
+}
+
 // One graph for a whole run: a gate, a WHILE loop of queue iterations, a gate, a WHILE loop of tail
 // iterations (CUDA conditional nodes; k_loop decides on the device whether a loop goes on).  Its kernels
 // read the run's inputs through v.io, so the instantiated graph is kept in the buffers and serves every
@@ -1405,7 +1508,9 @@ static int build_loop_graph(cm_context* ctx, RunBuffers<R>& rb, const RunView<R>
     // the gate kernel, then the WHILE node whose body holds kLoopBody iterations
     const Counters* cp = v.c;
     cudaGraphConditionalHandle hh = h[loop];
-    void* args[] = {(void*)&cp, (void*)&hh};
+    const RunIO* iop = v.io;
+    int queue = loop == 0;
+    void* args[] = {(void*)&cp, (void*)&iop, (void*)&queue, (void*)&hh};
     cudaKernelNodeParams kp = {};
     kp.func = (void*)k_gate;
     kp.gridDim = dim3(1);
@@ -1424,7 +1529,7 @@ static int build_loop_graph(cm_context* ctx, RunBuffers<R>& rb, const RunView<R>
     if ((e = cudaStreamBeginCaptureToGraph(ctx->cap_stream, body, nullptr, nullptr, 0,
                                            cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
       return bail(e, "cudaStreamBeginCaptureToGraph");
-    for (int it = 0; it < kLoopBody; ++it) {
+    for (int it = 0; it < (loop == 0 ? kQueueBody : kTailBody); ++it) {
       if (loop == 0) launch_queue_iteration<R>(ctx, v, vs, it & 1, grid, smem, ctx->cap_stream, &hh, nullptr);
       else launch_tail_iteration<R>(ctx, v, it & 1, grid, tail_steps, ctx->cap_stream, &hh, nullptr);
     }
@@ -1448,7 +1553,7 @@ static int run_error(int err, const Counters& hc) {
     case CM_ELIMIT: {
       char msg[256];
       snprintf(msg, sizeof(msg), "iteration limit reached (live %d %d, pool %d, primaries %llu of %llu)", hc.n[0],
-               hc.n[1], hc.pool, hc.next_primary, hc.total_primaries);
+               hc.n[1], hc.pool.v, hc.next_primary, hc.total_primaries);
       return fail(err, msg);
     }
     default: return fail(err, "the transport kernels reported error " + std::to_string(err));
@@ -1460,7 +1565,7 @@ template <typename R> static void dump_live(const RunBuffers<R>& rb, const Count
   if (!getenv("CM_DEBUG_DUMP")) return;
   const int cur = hc.n[0] ? 0 : 1;
   for (int seg = 0; seg < kWaveSegments; ++seg) {
-    const int k = std::min(8, hc.nc[cur][seg]);
+    const int k = std::min(8, hc.nc[cur][seg].v);
     if (k == 0) continue;
     // the tiles that hold the segment's first records
     const size_t first = (size_t)seg * rb.cap, t0 = first / 32, t1 = (first + k - 1) / 32;
@@ -1531,6 +1636,7 @@ static int run_device_once(cm_context* ctx, const cm_run_desc* d, uint32_t* back
   io.max_slots = maxIt;
   io.tail_below = tu.tail_below;
   io.queue_only = (ctx->options & CM_OPT_QUEUE_STEPS) ? 1 : 0;
+  io.start_tail = starts_in_tail(total, emax_eV, tu.tail_below) && !io.queue_only && d->max_iterations <= 0;
   io.cancel = ctx->cancel ? ctx->cancel_dev : nullptr;
   CM_CUDA(cudaMemcpyAsync(rb.io, &io, sizeof(RunIO), cudaMemcpyHostToDevice, stream));
 
@@ -1626,7 +1732,7 @@ static int run_device_once(cm_context* ctx, const cm_run_desc* d, uint32_t* back
       }
       // all primaries started and fewer electrons left (waves and pool) than the tail threshold: the tail
       // iterations (unless CM_OPT_QUEUE_STEPS keeps the queue kernels to the end)
-      const long long left = (long long)hc.n[0] + hc.n[1] + std::min(hc.pool, v.poolCap);
+      const long long left = (long long)hc.n[0] + hc.n[1] + std::min(hc.pool.v, v.poolCap);
       tail = !(ctx->options & CM_OPT_QUEUE_STEPS) && hc.next_primary == hc.total_primaries && left < tu.tail_below;
       if (qslots + tslots >= maxIt) {
         status = run_error(CM_ELIMIT, hc);
@@ -3045,6 +3151,11 @@ static int run_noalloc(cm_context* ctx, const cm_run_desc* d, uint32_t* back, ui
   // flag and the caller's tallies start at zero; waves, queues and pool are
   // only read below the counts, so they need no clearing
   const size_t hbytes = (size_t)n * d->hist_stride * sizeof(uint32_t);
+  // Through k_block, whose blocks hold the whole small wave in shared memory, unless the caller limits the
+  // iterations (the queue kernels') or wants the queue kernels; a pool overflow there, where a launch takes
+  // many steps before the refill empties the pool, repeats the run with them.
+  bool blocks = d->max_iterations <= 0 && !(ctx->options & CM_OPT_QUEUE_STEPS);
+again:
   CM_CUDA(cudaMemsetAsync(c, 0, sizeof(Counters), s));
   CM_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), s));
   CM_CUDA(cudaMemsetAsync(back, 0, hbytes, s));
@@ -3067,9 +3178,15 @@ static int run_noalloc(cm_context* ctx, const cm_run_desc* d, uint32_t* back, ui
   const auto t0 = std::chrono::steady_clock::now();
   int it = 0, status = 0;
   for (;;) {
-    for (int k = 0; k < 16; ++k, ++it) {
+    for (int k = 0; k < (blocks ? 2 : 16); ++k, ++it) {
       const int cur = it & 1;
       const RunView<R> v = view_at(v0, cur);
+      if (blocks) {
+        launch_block(v, cur, ctx->nsm, CM_TAIL_STEPS, s);
+        launch_spawn<R>(v, cur, grid, s);
+        k_tail<R><<<1, 32, 0, s>>>(v, cur, 1);
+        continue;
+      }
       launch_flight(v, cur, grid, s);
       k_flight_fast<R><<<grid, 256, 0, s>>>(v, cur);
       k_elastic<R><<<grid, 256, 0, s>>>(v, cur);
@@ -3081,6 +3198,10 @@ static int run_noalloc(cm_context* ctx, const cm_run_desc* d, uint32_t* back, ui
     CM_CUDA(cudaGetLastError());
     CM_CUDA(cudaMemcpyAsync(&hc, c, sizeof(Counters), cudaMemcpyDeviceToHost, s));
     CM_CUDA(cudaStreamSynchronize(s));
+    if (hc.error == CM_EOVERFLOW && blocks) {
+      blocks = false;
+      goto again;
+    }
     if (hc.error) {
       status = hc.error == CM_EOVERFLOW
                    ? fail(CM_EOVERFLOW, "cm_run_noalloc: the secondary pool in the fixed scratch overflowed; pass "
@@ -3111,7 +3232,9 @@ static int run_noalloc(cm_context* ctx, const cm_run_desc* d, uint32_t* back, ui
     st->device_ms = ms;
     st->ended_zero_energy = (int64_t)hc.ended_zero;
     st->ended_step_limit = (int64_t)hc.ended_limit;
-    for (int k = 0; k < 6; ++k) st->kernel_launches[k] = it;
+    for (int k = 0; k < 6; ++k) st->kernel_launches[k] = blocks && k < 4 ? 0 : it;
+    st->step_launches = blocks ? it : 0;
+    st->step_units = (int64_t)hc.step_units;
     for (int k = 0; k < 4; ++k) st->units[k] = (int64_t)hc.units[k];
   }
   return status;

@@ -357,6 +357,8 @@ static int batch_add(Batcher& b, JobRecord& j) {
   return 0;
 }
 
+// iterations of a round in the tail (launches of many steps each; an even number)
+constexpr int kTailRound = 4;
 // rounds a batch runs between two reads of its counters while its wave is full and no job waits
 constexpr int kRoundRepeats = 4;
 
@@ -432,7 +434,7 @@ static int batch_round(Batcher& b) {
   // many steps per launch (the tail kernels) whenever fewer electrons are in the wave and pool than
   // fill the GPU, even with primaries still to start; the refill then fills the wave only up to that many,
   // so a light load runs at the latency of a job alone and a heavy one through the queue kernels
-  const long long left = (long long)hc.n[0] + hc.n[1] + std::min(hc.pool, v.poolCap);
+  const long long left = (long long)hc.n[0] + hc.n[1] + std::min(hc.pool.v, v.poolCap);
   const bool tail = !(ctx->options & CM_OPT_QUEUE_STEPS) && left < tu.tail_below;
   hc.fill = tail ? std::min(W, tu.tail_below) : 0;
   CM_CUDA(cudaMemcpyAsync(ctx->counters, &hc, sizeof(Counters), cudaMemcpyHostToDevice, s));
@@ -442,21 +444,21 @@ static int batch_round(Batcher& b) {
   if (!(ctx->options & CM_OPT_GLOBAL_TABLES)) vs.s.nstaged = v.s.nstage;
   const size_t smem = (size_t)vs.s.nstaged * sizeof(R);
   const LoopKey key{ds.gen, 0, grid, ctx->nsm * CM_INEL_BLOCKS_PER_SM, tu.tail_steps, (int)vs.s.nstaged};
-  if (!b.round_exec[0] || !(b.round_key == key) || b.round_buffers != (const void*)rb.w[0].base ||
-      b.round_pool != rb.poolCap) {
+  if (!(b.round_key == key) || b.round_buffers != (const void*)rb.w[0].base || b.round_pool != rb.poolCap) {
     b.drop_rounds();
-    for (int loop = 0; loop < 2; ++loop) {
-      CM_CUDA(cudaStreamBeginCapture(ctx->cap_stream, cudaStreamCaptureModeThreadLocal));
-      for (int it = 0; it < kLoopBody; ++it) {
-        if (loop == 0) launch_queue_iteration<R>(ctx, v, vs, it & 1, grid, smem, ctx->cap_stream, nullptr, nullptr);
-        else launch_tail_iteration<R>(ctx, v, it & 1, grid, tu.tail_steps, ctx->cap_stream, nullptr, nullptr);
-      }
-      CM_CUDA(cudaStreamEndCapture(ctx->cap_stream, &b.round_graph[loop]));
-      CM_CUDA(cudaGraphInstantiate(&b.round_exec[loop], b.round_graph[loop], 0));
-    }
     b.round_key = key;
     b.round_buffers = (const void*)rb.w[0].base;
     b.round_pool = rb.poolCap;
+  }
+  const int loop = tail ? 1 : 0;
+  if (!b.round_exec[loop]) {  // each kind of round is captured when the batch first needs it
+    CM_CUDA(cudaStreamBeginCapture(ctx->cap_stream, cudaStreamCaptureModeThreadLocal));
+    for (int it = 0; it < (tail ? kTailRound : kLoopBody); ++it) {
+      if (loop == 0) launch_queue_iteration<R>(ctx, v, vs, it & 1, grid, smem, ctx->cap_stream, nullptr, nullptr);
+      else launch_tail_iteration<R>(ctx, v, it & 1, grid, tu.tail_steps, ctx->cap_stream, nullptr, nullptr);
+    }
+    CM_CUDA(cudaStreamEndCapture(ctx->cap_stream, &b.round_graph[loop]));
+    CM_CUDA(cudaGraphInstantiate(&b.round_exec[loop], b.round_graph[loop], 0));
   }
   // While the wave is full and no job waits for admission, kRoundRepeats rounds run back to back before
   // the counters are read: the host's turn between rounds (counter copies, job bookkeeping) leaves the GPU

@@ -50,13 +50,24 @@ struct Rec {
   CM_D uint32_t& step() const { return ((uint32_t*)w)[96]; }
 };
 
+// A counter the kernels append through, alone in its cache line: appends to different queues and segments
+// then go to different slices of L2 instead of queueing behind one another.
+struct alignas(128) Line {
+  int v;
+  CM_HD operator int() const { return v; }
+  CM_HD void operator=(int x) { v = x; }
+  CM_HD void operator+=(int x) { v += x; }
+  CM_HD void operator-=(int x) { v -= x; }
+};
+
 struct Counters {
-  int n[2];              // electrons in each wave
-  int nc[2][kWaveSegments];  // of which in each segment (segment k holds slots [k W, k W + nc))
-  int ns[kWaveSegments];     // electrons the refill appends after the survivors of each segment
-  int pool;
-  int q[3];
-  int deferred;  // fast flights handed on to the next iteration's full flights
+  Line nc[2][kWaveSegments];  // electrons in each segment of each wave (segment k holds slots [k W, k W + nc))
+  Line ns[kWaveSegments];     // electrons the refill appends after the survivors of each segment
+  Line q[3];
+  Line deferred;  // fast flights handed on to the next iteration's full flights
+  Line pool;
+  Line claim;  // wave electrons taken by the blocks of the resident-steps kernel beyond their first share
+  int n[2];       // electrons in each wave
   int error;
   int done;
   unsigned long long next_primary, total_primaries;
@@ -68,7 +79,6 @@ struct Counters {
   unsigned long long slots, tail_slots;  // iteration slots the device-driven loop ran (all, tail)
   unsigned long long ended_zero, ended_limit;  // electrons ended by the zero-energy cut, by the step limit
   int fill;  // the refill fills the wave up to this many electrons (0: W); set by the job server's tail rounds
-  int claim;  // wave electrons taken by the blocks of the resident-steps kernel beyond their first share
 };
 
 template <typename R>
@@ -176,6 +186,7 @@ struct RunIO {
   long long max_slots;
   int tail_below;
   int queue_only;
+  int start_tail;  // the run goes to the tail loop at once
   const volatile int* cancel;
   // A run of several jobs (the job server's shared wave; all null otherwise): per pixel its chamber, the
   // offset of its tally row (u32 elements into back/fwd) and its job; per job the electrons alive (a
@@ -453,10 +464,11 @@ template <typename R, typename Sink> CM_D void keep(const RunView<R>& v, int nxt
 }
 
 // The flight of wave slot i: reads what the step uses and writes back only what it changes
-// (direction, pixel and key stay in place for the event kernels), then queues the event.
-// FAST: an electron whose step needs the full form goes to the next wave's slow segment as it is.
+// (direction, pixel and key stay in place for the event kernels).  Returns the event queue the slot joins,
+// -1 when the electron ended, and for FAST Q_SLOW, nothing written, when the step needs the full form: the
+// electron then goes to the next wave's slow segment as it is.
 template <typename R, int D, bool FAST, typename Sink>
-CM_D void flight_one(const RunView<R>& v, int cur, int i, Sink& sink, StepCounts& sc) {
+CM_D int flight_one(const RunView<R>& v, int i, Sink& sink, StepCounts& sc) {
   const Rec<R> w(v.now, i);
   El<R> e;
   e.p[0] = w.px(); e.p[1] = w.py(); e.p[2] = w.pz();
@@ -468,22 +480,16 @@ CM_D void flight_one(const RunView<R>& v, int cur, int i, Sink& sink, StepCounts
   const int queue = flight_apply<R, D, FAST>(v, e, sink, sc, &w.pixel());  // the pixel is read only on escape
   if (queue < 0) {
     if (v.io->job_alive) job_end(v, w.pixel(), e.step, sink);
-    return;
+    return -1;
   }
-  if (FAST && queue == Q_SLOW) {
-    e.pixel = w.pixel();
-    keep(v, cur ^ 1, e, kSlowSegment, sink);
-    sink.append(&v.c->deferred);
-    return;
-  }
+  if (FAST && queue == Q_SLOW) return Q_SLOW;
   w.px() = e.p[0]; w.py() = e.p[1]; w.pz() = e.p[2];
   w.E() = e.E; w.Ep() = e.Ep;
   w.aux() = e.aux;
   w.step() = e.step;
   if (!FAST) w.region() = e.region;  // a FAST step stays in its region
   if (!FAST && aux_kind(e.aux) == AUX_BARRIER) { w.hx() = e.h[0]; w.hy() = e.h[1]; w.hz() = e.h[2]; }
-  const int slot = sink.append_q(v.c->q, queue);
-  v.q[queue][slot] = i;
+  return queue;
 }
 
 CM_D int survivors(const Counters* c, int nxt) {
@@ -494,7 +500,7 @@ CM_D int survivors(const Counters* c, int nxt) {
 
 // a record appended to the secondary pool; false (and CM_EOVERFLOW) when the pool is full
 template <typename R, typename Sink> CM_D bool pool_push(const RunView<R>& v, const El<R>& se, Sink& sink) {
-  const int slot = sink.append(&v.c->pool);
+  const int slot = sink.append(&v.c->pool.v);
   if (slot >= v.poolCap) {
     sink.error(&v.c->error, -5 /* CM_EOVERFLOW */);
     return false;
@@ -580,24 +586,28 @@ template <typename R, int D, typename Sink> CM_D bool misc_apply(const RunView<R
   return !(e.E < m.minE);
 }
 
-// the queue kernels' events: the record of queue entry j, its event, and the survivor kept
-template <typename R, typename Sink> CM_D void elastic_one(const RunView<R>& v, int cur, int j, Sink& sink) {
-  El<R> e = load_event(v.now, v.q[Q_EL][j]);
-  if (elastic_apply(v, e)) keep(v, cur ^ 1, e, segment_after(v.s, e), sink);
-  else job_end(v, e.pixel, e.step, sink);
+// the queue kernels' events: the record of queue entry j through its event; the segment of the next wave
+// the survivor joins, or -1
+template <typename R, typename Sink> CM_D int elastic_one(const RunView<R>& v, int j, El<R>& e, Sink& sink) {
+  e = load_event(v.now, v.q[Q_EL][j]);
+  if (elastic_apply(v, e)) return segment_after(v.s, e);
+  job_end(v, e.pixel, e.step, sink);
+  return -1;
 }
 
-template <typename R, typename Sink> CM_D void inelastic_one(const RunView<R>& v, int cur, int j, Sink& sink, StepCounts& sc) {
-  El<R> e = load_event(v.now, v.q[Q_TAB][j]);
-  if (inelastic_apply(v, e, sink, sc)) keep(v, cur ^ 1, e, segment_after(v.s, e), sink);
-  else job_end(v, e.pixel, e.step, sink);
+template <typename R, typename Sink> CM_D int inelastic_one(const RunView<R>& v, int j, El<R>& e, Sink& sink, StepCounts& sc) {
+  e = load_event(v.now, v.q[Q_TAB][j]);
+  if (inelastic_apply(v, e, sink, sc)) return segment_after(v.s, e);
+  job_end(v, e.pixel, e.step, sink);
+  return -1;
 }
 
 template <typename R, int D, typename Sink>
-CM_D void misc_one(const RunView<R>& v, int cur, int j, Sink& sink, StepCounts& sc) {
-  El<R> e = load(v.now, v.q[Q_MISC][j]);
-  if (misc_apply<R, D>(v, e, sink, sc)) keep(v, cur ^ 1, e, segment_after(v.s, e), sink);
-  else job_end(v, e.pixel, e.step, sink);
+CM_D int misc_one(const RunView<R>& v, int j, El<R>& e, Sink& sink, StepCounts& sc) {
+  e = load(v.now, v.q[Q_MISC][j]);
+  if (misc_apply<R, D>(v, e, sink, sc)) return segment_after(v.s, e);
+  job_end(v, e.pixel, e.step, sink);
+  return -1;
 }
 
 // refill plan of the next wave: secondaries from the pool first; new primaries
@@ -617,15 +627,12 @@ CM_D void refill_plan(const Counters* c, int nxt, int W, int poolCap, int& nn, i
 }
 
 // the j-th electron the refill adds to the next wave: a secondary from the top
-// of the pool or a new primary, appended after the survivors of its segment
+// of the pool or a new primary; the segment it joins (after its survivors), or -1
 template <typename R, int D, typename Sink>
-CM_D void spawn_one(const RunView<R>& v, int nxt, int j, int take_se, int poolTop, unsigned long long first,
-                    Sink& sink) {
+CM_D int spawn_one(const RunView<R>& v, int j, int take_se, int poolTop, unsigned long long first, El<R>& e, Sink& sink) {
   if (j < take_se) {
-    const El<R> se = load_live(v.pool, poolTop - 1 - j);
-    const int seg = wave_segment(v.s, se);
-    store_live(v.next, seg * v.W + v.c->nc[nxt][seg] + sink.append_q(v.c->ns, seg), se);
-    return;
+    e = load_live(v.pool, poolTop - 1 - j);
+    return wave_segment(v.s, e);
   }
   // GaussianBeam::createElectron (NISTMonte/GaussianBeam.cu:52-65) + initializeTrajectory (MonteCarloSS.cu:99-105)
   const RunIO& io = *v.io;
@@ -637,9 +644,8 @@ CM_D void spawn_one(const RunView<R>& v, int nxt, int j, int take_se, int poolTo
     else hi = mid;
   }
   const int px = lo;
-  if (io.job_stop && io.job_stop[io.pjob[px]]) return;  // a stopped job starts no more primaries
+  if (io.job_stop && io.job_stop[io.pjob[px]]) return -1;  // a stopped job starts no more primaries
   const unsigned long long k = gi - io.prefix[px] + (io.pfirst ? io.pfirst[px] : 0ull);
-  El<R> e;
   e.key = mix64(io.pkey[px] + mix64(k + 1));
   Rng<R> g(e.key, 0xFFFFFFFFu, 0);
   const double u1 = (double)g.next(), u2 = (double)g.next();
@@ -656,9 +662,8 @@ CM_D void spawn_one(const RunView<R>& v, int nxt, int j, int take_se, int poolTo
   e.aux = 0;
   e.step = 0;
   e.h[0] = e.h[1] = e.h[2] = 0;
-  const int seg = wave_segment(v.s, e);
-  store_live(v.next, seg * v.W + v.c->nc[nxt][seg] + sink.append_q(v.c->ns, seg), e);
   job_start(v, px, sink);
+  return wave_segment(v.s, e);
 }
 
 // end of an iteration: counters of the next wave, reset of this one (steps: the iteration ran k_block)
@@ -687,7 +692,8 @@ CM_D void tail_update(Counters* c, int cur, int W, int poolCap, bool steps) {
   c->pool -= take_se;
   c->next_primary += (unsigned long long)take_p;
   c->n[cur] = 0;
-  c->q[0] = c->q[1] = c->q[2] = c->deferred = 0;
+  for (int k = 0; k < 3; ++k) c->q[k] = 0;
+  c->deferred = 0;
   c->claim = 0;
   c->done = (c->n[nxt] == 0 && c->pool == 0 && c->next_primary == c->total_primaries) ? 1 : 0;
 }
