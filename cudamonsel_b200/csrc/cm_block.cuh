@@ -124,7 +124,7 @@ __device__ __forceinline__ void block_task(const RunView<R>& v, int l, int slot,
     bool alive;
     dest = kListDead;
     if (l <= kListSlow) {
-      const int q = l == kListSlow ? flight_apply<R, D>(v, e, sink, sc) : flight_apply<R, 0, true>(v, e, sink, sc);
+      const int q = l == kListSlow ? flight_apply<R, D>(v, e, sink, sc) : flight_fast(v, e, sc, [](El<R>&) {});
       alive = q >= 0;
       if (q == Q_EL) alive = elastic_apply(v, e);
       if (q == Q_SLOW) {

@@ -581,9 +581,7 @@ template <> CM_D float nieminen_loss(float kE, float x) { return kE * expm1f(-(2
 // JMONSEL/JoyLuoNieminenCSD.cu:91-121; the recursive halving is run with an
 // explicit stack in the same order (first half, then second half at the
 // energy reached after the first).
-template <typename R> CM_D R jln_compute(const Jln<R>& c, R len, R kE) {
-  if ((c.nce == 0) || (kE < c.minE) || (kE <= R(0))) return 0;
-  if (kE <= c.breakE) return nieminen_loss(kE, c.gamma15 * len * kE * msqrt(kE));
+template <typename R> CM_D R jln_above_break(const Jln<R>& c, R len, R kE) {
   // The reference halves the step recursively while the loss exceeds 10 % of
   // the energy (JoyLuoNieminenCSD.cu:101-121).  The segments form a binary tree
   // visited depth first, left half first; node (depth, idx) covers
@@ -624,12 +622,24 @@ template <typename R> CM_D R jln_compute(const Jln<R>& c, R len, R kE) {
   return total;
 }
 
+template <typename R> CM_D R jln_compute(const Jln<R>& c, R len, R kE) {
+  if ((c.nce == 0) || (kE < c.minE) || (kE <= R(0))) return 0;
+  if (kE <= c.breakE) return nieminen_loss(kE, c.gamma15 * len * kE * msqrt(kE));
+  return jln_above_break(c, len, kE);
+}
+
 // ------------------------------------------------------------ mechanism rates
 // TabulatedInelasticSM.cu:436-459
 template <typename R> CM_D R tabulated_rate(const SceneView<R>& s, const Mech<R>& k, R E) {
   const R kEa = E + k.energyOffset;
   if (kEa < k.iimfpDomain0) return 0;
   return k.rateMult * table_interp(s, k.iimfp, kEa, R(0), R(0), 1);
+}
+
+// the rate for x = hbar omega / E from 0.1 on (rare: out of line, out of the other rates' registers)
+__host__ __device__ __noinline__ double phonon_rate_slow(double prefactor, double xd) {
+  const double t = sqrt(1.0 - xd);
+  return prefactor * xd * log((1.0 + t) / (1.0 - t));
 }
 
 // GanachaudMokraniPhononInelasticSM.cu:46-72
@@ -645,8 +655,7 @@ template <typename R> CM_D R phonon_rate(const Mech<R>& k, R kE) {
     return k.prefactor * x * mlog(R(4) / x);
   }
   if (xd >= 1.0) return 0;
-  const double t = sqrt(1.0 - xd);
-  return (R)(k.prefactor64 * xd * log((1.0 + t) / (1.0 - t)));
+  return (R)phonon_rate_slow(k.prefactor64, xd);
 }
 
 // ------------------------------------------------------------ geometry (double)

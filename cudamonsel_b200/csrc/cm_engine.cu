@@ -893,7 +893,7 @@ static int build_scene(cm_context* ctx, DevScene<R>& ds) {
   std::vector<FastCyl> fcyls;
   for (const Region& r : regions) {
     FastRegion f{r.msm, r.cls, (int)fplanes.size(), -1, -1, {0, 0, 0}};
-    if (r.nchild == 0) {
+    if (r.nchild == 0 && msms[r.msm].nmech <= 4) {  // the fast flight picks among at most four mechanisms
       const size_t c0 = fcyls.size();
       if (inside_of(shapes, planes, r.shape, fplanes, fcyls) && fcyls.size() - c0 <= 1) {
         f.np = (int)fplanes.size() - f.plane0;

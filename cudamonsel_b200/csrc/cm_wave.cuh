@@ -332,9 +332,9 @@ template <typename R> CM_D MsmRates<R> msm_rates(const SceneView<R>& s, const Ms
 }
 
 // MONSEL_MaterialScatterModel::scatter (:93-134): the first mechanism whose cumulative rate reaches r
-template <typename R> CM_D int mech_pick(const SceneView<R>& s, const Msm<R>& m, R E, const MsmRates<R>& q, R r) {
+// (of up to four)
+template <typename R> CM_D int mech_pick4(const Msm<R>& m, const MsmRates<R>& q, R r) {
   const int n = m.nmech;
-  if (n > 4) return mech_pick_long(s, m, E, r);
   int idx = 0;
   if (n > 1 && q.c0 < r) {
     idx = 1;
@@ -346,6 +346,10 @@ template <typename R> CM_D int mech_pick(const SceneView<R>& s, const Msm<R>& m,
   return idx;
 }
 
+template <typename R> CM_D int mech_pick(const SceneView<R>& s, const Msm<R>& m, R E, const MsmRates<R>& q, R r) {
+  return m.nmech > 4 ? mech_pick_long(s, m, E, r) : mech_pick4(m, q, r);
+}
+
 // ---------------------------------------------------------------- flight
 // MonteCarloSS::takeStep (NISTMonte/MonteCarloSS.cu:107-163) up to the event:
 // region check, MONSEL_MaterialScatterModel::randomMeanPathLength, the
@@ -354,20 +358,14 @@ template <typename R> CM_D int mech_pick(const SceneView<R>& s, const Msm<R>& m,
 // One step's flight on a record held in registers (p, d, E, step, region and key valid; the pixel too,
 // or, when pixel_src is given, read from there if the electron escapes): the event queue of its end, or
 // -1 when the electron ended here (escaped and tallied, stopped, trapped).
-//
-// FAST: the step of an electron strictly inside a childless region that stays so, without the region test,
-// the boundary search, crossings and escapes; Q_SLOW, with nothing changed or counted, when this step may
-// need them (the full form then takes it from the start: the random stream is keyed by the step).
-template <typename R, int D, bool FAST = false, typename Sink>
+template <typename R, int D, typename Sink>
 CM_D int flight_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc, const int* pixel_src = nullptr) {
   const SceneView<R>& s = v.s;
   int reg = e.region;
-  const FastRegion f = FAST ? s.fast[reg] : FastRegion();
-  if (FAST) {
-  } else if (reg < 0 || !shape_contains<R, D>(s, s.regions[reg].shape, e.p))
+  if (reg < 0 || !shape_contains<R, D>(s, s.regions[reg].shape, e.p))
     reg = containing_subregion<R, D>(s, chamber_of(v, pixel_src ? *pixel_src : e.pixel), e.p);
   if (reg < 0) return -1;
-  const Msm<R>& m = s.msms[FAST ? f.msm : s.regions[reg].msm];
+  const Msm<R>& m = s.msms[s.regions[reg].msm];
   bool complete = false;
   double fp = 2.0 * kChamberRadiusNm;
   R total = 0;
@@ -385,8 +383,6 @@ CM_D int flight_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc,
       // geometry, so that the rates need not stay live (nothing else draws from this stream)
       idx = mech_pick(s, m, e.E, rates, u1 * total);
       kind = (m.kinds >> (4 * idx)) & 15;
-    } else if (FAST) {
-      return Q_SLOW;
     } else if (e.step > 1000000u) {  // MONSEL_MaterialScatterModel::randomMeanPathLength (:86-90)
       complete = true;
       ++sc.limit;
@@ -404,8 +400,7 @@ CM_D int flight_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc,
   double p1[3] = {e.p[0] + fp * (double)e.d[0], e.p[1] + fp * (double)e.d[1], e.p[2] + fp * (double)e.d[2]};
   double hn[3];
   bool clipped = false;
-  if (FAST && !point_inside(s, f, p1)) return Q_SLOW;
-  const int next = FAST ? reg : find_end_of_step<R, D>(s, reg, e.p, p1, hn, &clipped);
+  const int next = find_end_of_step<R, D>(s, reg, e.p, p1, hn, &clipped);
   const double dd = sqrt((p1[0] - e.p[0]) * (p1[0] - e.p[0]) + (p1[1] - e.p[1]) * (p1[1] - e.p[1]) +
                          (p1[2] - e.p[2]) * (p1[2] - e.p[2]));
   const R dE = m.csd ? jln_compute(m.jln, (R)dd, e.E) : R(0);
@@ -435,7 +430,7 @@ CM_D int flight_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc,
     } else {
       if (kind == MECH_POLARON) return -1;  // GanachaudMokraniPolaronTrapSM::scatter: trapped, E = 0
       queue = kind == MECH_NISTMOTT ? Q_EL : kind == MECH_TABULATED ? Q_TAB : Q_MISC;
-      e.aux = aux_pack(AUX_MECH, idx) | (FAST ? AUX_INSIDE : 0);
+      e.aux = aux_pack(AUX_MECH, idx);
     }
   } else if (next >= 0) {
     ++sc.bar;
@@ -457,6 +452,46 @@ CM_D int flight_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc,
   return queue;
 }
 
+// The step of an electron strictly inside a childless region that stays so, without the region test, the
+// boundary search, crossings and escapes; Q_SLOW, with nothing changed or counted, when this step may need
+// them (flight_apply then takes it from the start: the random stream is keyed by the step).  e holds the
+// energy, step, key and region; rest(e) reads the position and direction, which the rates do not need
+// (read with the others they would spill).
+template <typename R, typename Rest> CM_D int flight_fast(const RunView<R>& v, El<R>& e, StepCounts& sc, Rest rest) {
+  const SceneView<R>& s = v.s;
+  const FastRegion f = s.fast[e.region];
+  const Msm<R>& m = s.msms[f.msm];
+  double fp = 2.0 * kChamberRadiusNm;
+  int idx;
+  {
+    Rng<R> g(e.key, e.step, 0);
+    const R u0 = g.next(), u1 = g.next();
+    const MsmRates<R> rates = msm_rates(s, m, e.E);
+    if (rates.total == R(0)) return Q_SLOW;
+    const R path = -mlog(u0) / rates.total;
+    if ((double)path < fp) fp = (double)path;
+    idx = mech_pick4(m, rates, u1 * rates.total);
+  }
+  rest(e);
+  const double p1[3] = {e.p[0] + fp * (double)e.d[0], e.p[1] + fp * (double)e.d[1], e.p[2] + fp * (double)e.d[2]};
+  if (!point_inside(s, f, p1)) return Q_SLOW;
+  e.Ep = e.E;
+  if (m.csd) {
+    const double dd = sqrt((p1[0] - e.p[0]) * (p1[0] - e.p[0]) + (p1[1] - e.p[1]) * (p1[1] - e.p[1]) +
+                           (p1[2] - e.p[2]) * (p1[2] - e.p[2]));
+    e.E += jln_compute(m.jln, (R)dd, e.E);
+  }
+  e.p[0] = p1[0]; e.p[1] = p1[1]; e.p[2] = p1[2];
+  e.step += 1;
+  ++sc.steps;
+  if (e.E < m.minE) return -1;
+  ++sc.scat;
+  const int kind = (m.kinds >> (4 * idx)) & 15;
+  if (kind == MECH_POLARON) return -1;  // GanachaudMokraniPolaronTrapSM::scatter: trapped, E = 0
+  e.aux = aux_pack(AUX_MECH, idx) | AUX_INSIDE;
+  return kind == MECH_NISTMOTT ? Q_EL : kind == MECH_TABULATED ? Q_TAB : Q_MISC;
+}
+
 // append an electron to segment k of the next wave
 template <typename R, typename Sink> CM_D void keep(const RunView<R>& v, int nxt, const El<R>& e, int k, Sink& sink) {
   const int slot = sink.append_q(v.c->nc[nxt], k);
@@ -471,13 +506,21 @@ template <typename R, int D, bool FAST, typename Sink>
 CM_D int flight_one(const RunView<R>& v, int i, Sink& sink, StepCounts& sc) {
   const Rec<R> w(v.now, i);
   El<R> e;
-  e.p[0] = w.px(); e.p[1] = w.py(); e.p[2] = w.pz();
-  e.d[0] = w.dx(); e.d[1] = w.dy(); e.d[2] = w.dz();
   e.E = w.E();
   e.step = w.step();
   e.region = w.region();
   e.key = w.key();
-  const int queue = flight_apply<R, D, FAST>(v, e, sink, sc, &w.pixel());  // the pixel is read only on escape
+  auto rest = [&](El<R>& x) {
+    x.p[0] = w.px(); x.p[1] = w.py(); x.p[2] = w.pz();
+    x.d[0] = w.dx(); x.d[1] = w.dy(); x.d[2] = w.dz();
+  };
+  int queue;
+  if (FAST) {
+    queue = flight_fast(v, e, sc, rest);
+  } else {
+    rest(e);
+    queue = flight_apply<R, D>(v, e, sink, sc, &w.pixel());  // the pixel is read only on escape
+  }
   if (queue < 0) {
     if (v.io->job_alive) job_end(v, w.pixel(), e.step, sink);
     return -1;
