@@ -1153,26 +1153,21 @@ CM_D bool point_in_box(const double* bb, const double* p) {
   return p[0] >= bb[0] && p[1] >= bb[1] && p[2] >= bb[2] && p[0] <= bb[3] && p[1] <= bb[4] && p[2] <= bb[5];
 }
 
-// the segment p0 -> p1 meets the box (slab test over u in [0, 1])
-CM_D bool segment_meets_box(const double* bb, const double* p0, const double* p1) {
+// The segment p0 -> p1 meets the box (slab test over u in [0, 1]).  rd holds the reciprocals of the
+// segment's components, formed once per step: the product differs from the quotient by 2 ulp, ~1e-7 nm of
+// the longest step, and the boxes are padded by at least 1e-3 nm, so no struck child is ever left out.  The
+// segment's own box is compared first; most children fail that.
+CM_D bool segment_meets_box(const double* bb, const double* p0, const double* p1, const double* rd) {
   double lo = 0.0, hi = 1.0;
+  for (int a = 0; a < 3; ++a)
+    if (fmin(p0[a], p1[a]) > bb[3 + a] || fmax(p0[a], p1[a]) < bb[a]) return false;
   for (int a = 0; a < 3; ++a) {
-    const double d = p1[a] - p0[a];
-    if (d == 0.0) {
-      if (p0[a] < bb[a] || p0[a] > bb[3 + a]) return false;
-      continue;
-    }
-    double t0 = (bb[a] - p0[a]) / d, t1 = (bb[3 + a] - p0[a]) / d;
-    if (t0 > t1) {
-      const double t = t0;
-      t0 = t1;
-      t1 = t;
-    }
-    lo = t0 > lo ? t0 : lo;
-    hi = t1 < hi ? t1 : hi;
-    if (lo > hi) return false;
+    if (p1[a] == p0[a]) continue;
+    const double u = (bb[a] - p0[a]) * rd[a], w = (bb[3 + a] - p0[a]) * rd[a];
+    lo = fmax(lo, fmin(u, w));
+    hi = fmin(hi, fmax(u, w));
   }
-  return true;
+  return lo <= hi;
 }
 
 // RegionBase.cu:50-60, iterative: the first child whose shape holds p owns it
@@ -1252,10 +1247,11 @@ CM_D int find_end_of_step(const SceneView<R>& s, int reg, const double* p0, doub
   double t = nv.u;
   hitn[0] = nv.n[0]; hitn[1] = nv.n[1]; hitn[2] = nv.n[2];
   if ((t <= 1.0) && r.parent >= 0) base = r.parent;
+  const double rd[3] = {1.0 / (p1[0] - p0[0]), 1.0 / (p1[1] - p0[1]), 1.0 / (p1[2] - p0[2])};
   if (r.grid < 0) {
     for (int i = 0; i < r.nchild; ++i) {
       const int c = s.children[r.child0 + i];
-      if (!segment_meets_box(s.regions[c].bb, p0, p1)) continue;
+      if (!segment_meets_box(s.regions[c].bb, p0, p1, rd)) continue;
       NV cn = shape_first_normal<R, D>(s, s.regions[c].shape, p0, p1);
       if ((cn.u <= 1.0) && (cn.u < t)) {
         t = cn.u;
@@ -1269,7 +1265,7 @@ CM_D int find_end_of_step(const SceneView<R>& s, int reg, const double* p0, doub
     int bpos = 0x7fffffff;
     auto visit = [&](int pos) {
       const int c = s.children[r.child0 + pos];
-      if (!segment_meets_box(s.regions[c].bb, p0, p1)) return;
+      if (!segment_meets_box(s.regions[c].bb, p0, p1, rd)) return;
       NV cn = shape_first_normal<R, D>(s, s.regions[c].shape, p0, p1);
       if ((cn.u <= 1.0) && ((cn.u < t) || (cn.u == t && bpos != 0x7fffffff && pos < bpos))) {
         t = cn.u;
@@ -1284,7 +1280,14 @@ CM_D int find_end_of_step(const SceneView<R>& s, int reg, const double* p0, doub
     const double ex = p1[0] - p0[0], ey = p1[1] - p0[1];
     const double X1 = g.x0 + g.nx * g.dx, Y1 = g.y0 + g.ny * g.dy;
     double tlo = 0.0, thi = 1.0;
-    bool hit = true;
+    // the children lie between z0 and z1: an electron that leaves upwards over the whole chamber crosses
+    // that layer in a few cells
+    bool hit = fmin(p0[2], p1[2]) <= g.z1 && fmax(p0[2], p1[2]) >= g.z0;
+    if (hit && p1[2] != p0[2]) {
+      const double u = (g.z0 - p0[2]) * rd[2], w = (g.z1 - p0[2]) * rd[2];
+      tlo = fmax(tlo, fmin(u, w));
+      thi = fmin(thi, fmax(u, w));
+    }
     if (ex == 0.0) hit = p0[0] >= g.x0 && p0[0] <= X1;
     else {
       double a0 = (g.x0 - p0[0]) / ex, a1 = (X1 - p0[0]) / ex;

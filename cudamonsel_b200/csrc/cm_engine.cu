@@ -842,7 +842,7 @@ static int build_scene(cm_context* ctx, DevScene<R>& ds) {
   for (Region& r : regions) {
     if (r.nchild < kGridMinChildren || (ctx->options & CM_OPT_SCAN_CHILDREN)) continue;
     std::vector<int> bounded, unbounded;
-    double lo[2] = {INFINITY, INFINITY}, hi[2] = {-INFINITY, -INFINITY};
+    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     for (int i = 0; i < r.nchild; ++i) {
       const double* bb = regions[children[r.child0 + i]].bb;
       if (std::isinf(bb[0]) || std::isinf(bb[1]) || std::isinf(bb[3]) || std::isinf(bb[4]) || bb[0] > bb[3] ||
@@ -851,7 +851,7 @@ static int build_scene(cm_context* ctx, DevScene<R>& ds) {
         continue;
       }
       bounded.push_back(i);
-      for (int a = 0; a < 2; ++a) {
+      for (int a = 0; a < 3; ++a) {
         lo[a] = std::min(lo[a], bb[a]);
         hi[a] = std::max(hi[a], bb[3 + a]);
       }
@@ -866,6 +866,8 @@ static int build_scene(cm_context* ctx, DevScene<R>& ds) {
     g.y0 = lo[1];
     g.dx = wx / g.nx;
     g.dy = wy / g.ny;
+    g.z0 = lo[2];
+    g.z1 = hi[2];
     std::vector<std::vector<int>> lists((size_t)g.nx * g.ny);
     for (int i : bounded) {  // ascending positions, so every cell list is ascending
       const double* bb = regions[children[r.child0 + i]].bb;

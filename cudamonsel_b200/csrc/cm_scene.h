@@ -53,6 +53,7 @@ struct Region {
 // resolve ties by position, so they find what the in-order scan finds.
 struct ChildGrid {
   double x0, y0, dx, dy;  // nm
+  double z0, z1;          // the listed children's boxes lie between
   int nx, ny;
   int cell0;              // cell (ix, iy) lists grid_items[cell_start[cell0 + iy * nx + ix] .. next)
   int unb0, nunb;         // the unbounded children: grid_items[unb0 .. unb0 + nunb)
