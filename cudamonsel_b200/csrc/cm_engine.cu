@@ -1247,11 +1247,14 @@ template <typename R> static void launch_flight(const RunView<R>& v, int cur, in
 #include "cm_block.cuh"
 namespace cm {
 
-// the launch settings a run uses: the context's tuning, built-in defaults where it holds 0
-template <typename R> static cm_tuning resolved_tuning(const cm_context* ctx) {
+// the launch settings a run uses: the context's tuning, built-in defaults where it holds 0.  A scene with
+// shape trees enters the tail at half as many electrons: k_block's tree walks spill at its 128 registers
+// (one B200, 131072 against 262144: rounded features 66.5 / 69.4 ms, FP64 line scan 34.8 / 37.0 ms, FP64
+// image 111.5 / 110.7 ms; leaf scenes: FP32 line scan 46.3 / 45.3 ms, deep 131.9 / 126.1 ms).
+template <typename R> static cm_tuning resolved_tuning(const cm_context* ctx, int depth = 0) {
   cm_tuning t = ctx->tune[sizeof(R) == 8 ? CM_PREC_FP64 : CM_PREC_FP32];
   if (t.wave <= 0) t.wave = 1 << 21;
-  if (t.tail_below <= 0) t.tail_below = CM_TAIL_BELOW;
+  if (t.tail_below <= 0) t.tail_below = depth > 0 ? CM_TAIL_BELOW / 2 : CM_TAIL_BELOW;
   if (t.tail_steps <= 0) t.tail_steps = CM_TAIL_STEPS;
   if (t.blocks_per_sm <= 0) t.blocks_per_sm = 8;
   return t;
@@ -1263,63 +1266,117 @@ template <typename R> static void launch_misc(const RunView<R>& v, int cur, int 
   else k_misc<R, kMaxShapeDepth><<<grid, 256, 0, s>>>(v, cur);
 }
 
+// How an iteration ends: kEndSteps: it ran k_block; kEndLoop: it belongs to a loop of the device-driven run,
+// whose condition is set.
+constexpr int kEndSteps = 1, kEndLoop = 2;
+
+// End of an iteration, by one warp once every refill has been appended: the counters of the next wave, the
+// reset of this one's, and in the device-driven run the condition of the loop it is in: another iteration,
+// or not when the run is done or failed (a device error, the iteration limit, a cancel flag set by the
+// host), and for the queue loop also once every primary has started and fewer electrons are left than
+// io.tail_below (the tail loop of k_block takes over).  Iterations of a loop body after its end do no work:
+// their kernels find no electrons.  The lanes read the counters side by side: read one after another, each
+// in its own cache line, they took 8 us of every iteration.
+template <typename R>
+__device__ __forceinline__ void end_iteration(const RunView<R>& v, int cur, int end, cudaGraphConditionalHandle h) {
+  Counters* c = v.c;
+  const RunIO& io = *v.io;
+  const int lane = threadIdx.x & 31, nxt = cur ^ 1;
+  const bool seg = lane < kWaveSegments;
+  // (volatile: other blocks of this launch have changed some of them)
+  const int kept = seg ? *(volatile int*)&c->nc[nxt][lane].v : 0, added = seg ? *(volatile int*)&c->ns[lane].v : 0;
+  const int queued = lane < 3 ? *(volatile int*)&c->q[lane].v : 0;
+  const int nn = __reduce_add_sync(0xffffffffu, kept), appended = __reduce_add_sync(0xffffffffu, kept + added);
+  if (seg) {
+    c->nc[nxt][lane] = kept + added;
+    c->ns[lane] = 0;
+    c->nc[cur][lane] = 0;
+  }
+  if (lane < 3) {
+    if (!c->done) c->units[1 + lane] += (unsigned long long)queued;
+    c->q[lane] = 0;
+  }
+  __syncwarp();
+  if (lane != 0) return;
+  int take_se, take_p;
+  refill_plan(c, nn, v.W, v.poolCap, take_se, take_p);
+  int pool = c->pool < v.poolCap ? (int)c->pool : v.poolCap;
+  const unsigned long long next = c->next_primary + (unsigned long long)take_p, total = c->total_primaries;
+  const int was = c->n[cur], error0 = c->error;
+  const long long slots = (long long)c->slots + 1;
+  pool -= take_se;
+  if (!c->done) {
+    if (end & kEndSteps) c->step_units += (unsigned long long)was;
+    else c->units[0] += (unsigned long long)(was - c->deferred);
+    c->iterations += 1;
+  }
+  const bool done = appended == 0 && pool == 0 && next == total;
+  c->n[nxt] = appended;  // survivors and refills as appended (a stopped job's primaries are not)
+  c->n[cur] = 0;
+  c->pool = pool;
+  c->next_primary = next;
+  c->deferred = 0;
+  c->claim = 0;
+  c->ticket = 0;
+  c->done = done ? 1 : 0;
+  if (!(end & kEndLoop)) return;
+  c->slots = (unsigned long long)slots;
+  if (end & kEndSteps) c->tail_slots += 1;
+  int error = error0;
+  if (!done && !error) {
+    if (slots >= io.max_slots) error = CM_ELIMIT;
+    else if (io.cancel && *io.cancel) error = CM_ECANCELED;
+    if (error) c->error = error;
+  }
+  bool go = !done && !error;
+  if (go && !(end & kEndSteps) && !io.queue_only && next == total && (long long)appended + pool < io.tail_below) go = false;
+  cudaGraphSetConditional(h, go ? 1u : 0u);
+}
+
+// The refill of the next wave, and by the last block that is done with it the end of the iteration.
 template <typename R, int D>
-__global__ void __launch_bounds__(256) k_spawn(const __grid_constant__ RunView<R> v, int cur) {
+__global__ void __launch_bounds__(256) k_spawn(const __grid_constant__ RunView<R> v, int cur, int end, cudaGraphConditionalHandle h) {
   const int nxt = cur ^ 1;
-  int nn, take_se, take_p;
-  refill_plan(v.c, nxt, v.W, v.poolCap, nn, take_se, take_p);
-  const int poolTop = v.c->pool < v.poolCap ? v.c->pool : v.poolCap;
+  int nn = 0, take_se, take_p;
+#pragma unroll
+  for (int k = 0; k < kWaveSegments; ++k) nn += v.c->nc[nxt][k];
+  refill_plan(v.c, nn, v.W, v.poolCap, take_se, take_p);
+  const int poolTop = v.c->pool < v.poolCap ? (int)v.c->pool : v.poolCap;
   const unsigned long long first = v.c->next_primary;
   const int n = take_se + take_p;
-  if ((int)(blockIdx.x * blockDim.x) >= n) return;
-  DeviceSink sink;
-  __shared__ BlockAppend<kWaveSegments> app;
-  append_init(app);
-  int par = 0;
-  for (int j0 = blockIdx.x * blockDim.x; j0 < n; j0 += gridDim.x * blockDim.x, par ^= 1) {
-    El<R> e;
-    int dest = -1;
-    if (j0 + (int)threadIdx.x < n) dest = spawn_one<R, D>(v, j0 + (int)threadIdx.x, take_se, poolTop, first, e, sink);
-    const int slot = append_slot(app, par, dest, [&](int k) { return &v.c->ns[k].v; });
-    if (dest >= 0) store_live(v.next, dest * v.W + v.c->nc[nxt][dest] + slot, e);
+  if ((int)(blockIdx.x * blockDim.x) < n) {
+    DeviceSink sink;
+    __shared__ BlockAppend<kWaveSegments> app;
+    append_init(app);
+    int par = 0;
+    for (int j0 = blockIdx.x * blockDim.x; j0 < n; j0 += gridDim.x * blockDim.x, par ^= 1) {
+      El<R> e;
+      int dest = -1;
+      if (j0 + (int)threadIdx.x < n) dest = spawn_one<R, D>(v, j0 + (int)threadIdx.x, take_se, poolTop, first, e, sink);
+      const int slot = append_slot(app, par, dest, [&](int k) { return &v.c->ns[k].v; });
+      if (dest >= 0) store_live(v.next, dest * v.W + v.c->nc[nxt][dest] + slot, e);
+    }
   }
-}
-
-template <typename R> static void launch_spawn(const RunView<R>& v, int cur, int grid, cudaStream_t s) {
-  if (v.s.depth == 0) k_spawn<R, 0><<<grid, 256, 0, s>>>(v, cur);
-  else if (v.s.depth <= 2) k_spawn<R, 2><<<grid, 256, 0, s>>>(v, cur);
-  else k_spawn<R, kMaxShapeDepth><<<grid, 256, 0, s>>>(v, cur);
+  __shared__ int last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&v.c->ticket.v, 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last || threadIdx.x >= 32) return;
+  __threadfence();
+  end_iteration(v, cur, end, h);
 }
 
 template <typename R>
-__global__ void k_tail(const __grid_constant__ RunView<R> v, int cur, int steps) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) tail_update(v.c, cur, v.W, v.poolCap, steps != 0);
-}
-
-// The device-driven loop: each of its iterations ends with k_loop, which updates the counters as k_tail
-// does and then sets the condition of the conditional node it runs under: another iteration, or not when
-// the run is done or failed (a device error, the iteration limit, a cancel flag set by the host), and for
-// the queue loop also once every primary has started and fewer electrons are left than io.tail_below
-// (the tail loop of k_block takes over).  Iterations of a loop body after its end do no
-// work: their kernels find no electrons.
-template <typename R>
-__global__ void k_loop(const __grid_constant__ RunView<R> v, int cur, int steps, cudaGraphConditionalHandle h) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  Counters* c = v.c;
-  tail_update(c, cur, v.W, v.poolCap, steps != 0);
-  const RunIO& io = *v.io;
-  c->slots += 1;
-  if (steps) c->tail_slots += 1;
-  if (!c->done && !c->error) {
-    if ((long long)c->slots >= io.max_slots) c->error = CM_ELIMIT;
-    else if (io.cancel && *io.cancel) c->error = CM_ECANCELED;
-  }
-  bool go = !c->done && !c->error;
-  if (go && !steps && !io.queue_only) {
-    const long long left = (long long)c->n[cur ^ 1] + (c->pool < v.poolCap ? c->pool : v.poolCap);
-    if (c->next_primary == c->total_primaries && left < io.tail_below) go = false;
-  }
-  cudaGraphSetConditional(h, go ? 1u : 0u);
+static void launch_spawn(const RunView<R>& v, int cur, int nsm, int end, cudaGraphConditionalHandle* h, cudaStream_t s) {
+  const int grid = 4 * nsm;
+  const cudaGraphConditionalHandle hh = h ? *h : 0;
+  if (h) end |= kEndLoop;
+  if (v.s.depth == 0) k_spawn<R, 0><<<grid, 256, 0, s>>>(v, cur, end, hh);
+  else if (v.s.depth <= 2) k_spawn<R, 2><<<grid, 256, 0, s>>>(v, cur, end, hh);
+  else k_spawn<R, kMaxShapeDepth><<<grid, 256, 0, s>>>(v, cur, end, hh);
 }
 
 // opens a loop of the device-driven run unless the run is already done or failed; the queue loop also not
@@ -1458,24 +1515,18 @@ static void launch_queue_iteration(const cm_context* ctx, const RunView<R>& v0, 
   else k_elastic<R><<<grid, 256, 0, s>>>(v, cur);
   join(2);
   if (ev) cudaEventRecordWithFlags(ev[3], s, cudaEventRecordExternal);
-  launch_spawn<R>(v, cur, grid, s);
+  launch_spawn<R>(v, cur, ctx->nsm, 0, h, s);
   if (ev) cudaEventRecordWithFlags(ev[4], s, cudaEventRecordExternal);
-  if (h) k_loop<R><<<1, 32, 0, s>>>(v, cur, 0, *h);
-  else k_tail<R><<<1, 32, 0, s>>>(v, cur, 0);
-  if (ev) cudaEventRecordWithFlags(ev[5], s, cudaEventRecordExternal);
 }
 
 template <typename R>
-static void launch_tail_iteration(const cm_context* ctx, const RunView<R>& v0, int cur, int grid, int tail_steps,
-                                  cudaStream_t s, cudaGraphConditionalHandle* h, cudaEvent_t* ev) {
+static void launch_tail_iteration(const cm_context* ctx, const RunView<R>& v0, int cur, int tail_steps, cudaStream_t s,
+                                  cudaGraphConditionalHandle* h, cudaEvent_t* ev) {
   const RunView<R> v = view_at(v0, cur);
   launch_block(v, cur, ctx->nsm, tail_steps, s);
   if (ev) cudaEventRecordWithFlags(ev[0], s, cudaEventRecordExternal);
-  launch_spawn<R>(v, cur, grid, s);
+  launch_spawn<R>(v, cur, ctx->nsm, kEndSteps, h, s);
   if (ev) cudaEventRecordWithFlags(ev[1], s, cudaEventRecordExternal);
-  if (h) k_loop<R><<<1, 32, 0, s>>>(v, cur, 1, *h);
-  else k_tail<R><<<1, 32, 0, s>>>(v, cur, 1);
-  if (ev) cudaEventRecordWithFlags(ev[2], s, cudaEventRecordExternal);
 }
 
 // A run whose electrons never fill the GPU (about one more per 100 eV of a primary's energy is alive at the
@@ -1486,7 +1537,7 @@ static bool starts_in_tail(unsigned long long total, double emax_eV, int tail_be
 }
 
 // One graph for a whole run: a gate, a WHILE loop of queue iterations, a gate, a WHILE loop of tail
-// iterations (CUDA conditional nodes; k_loop decides on the device whether a loop goes on).  Its kernels
+// iterations (CUDA conditional nodes; end_iteration decides on the device whether a loop goes on).  Its kernels
 // read the run's inputs through v.io, so the instantiated graph is kept in the buffers and serves every
 // later run with the same key; the host launches it once per run and reads the counters once.
 template <typename R>
@@ -1533,7 +1584,7 @@ static int build_loop_graph(cm_context* ctx, RunBuffers<R>& rb, const RunView<R>
       return bail(e, "cudaStreamBeginCaptureToGraph");
     for (int it = 0; it < (loop == 0 ? kQueueBody : kTailBody); ++it) {
       if (loop == 0) launch_queue_iteration<R>(ctx, v, vs, it & 1, grid, smem, ctx->cap_stream, &hh, nullptr);
-      else launch_tail_iteration<R>(ctx, v, it & 1, grid, tail_steps, ctx->cap_stream, &hh, nullptr);
+      else launch_tail_iteration<R>(ctx, v, it & 1, tail_steps, ctx->cap_stream, &hh, nullptr);
     }
     cudaGraph_t captured = nullptr;
     if ((e = cudaStreamEndCapture(ctx->cap_stream, &captured)) != cudaSuccess) return bail(e, "cudaStreamEndCapture");
@@ -1591,7 +1642,7 @@ static int run_device_once(cm_context* ctx, const cm_run_desc* d, uint32_t* back
   int rc;
   DevScene<R>& ds = scene_of<R>(ctx);
   if ((rc = build_scene<R>(ctx, ds))) return rc;
-  const cm_tuning tu = resolved_tuning<R>(ctx);
+  const cm_tuning tu = resolved_tuning<R>(ctx, ds.view.depth);
   const int W = d->wave > 0 ? d->wave : tu.wave;
   RunBuffers<R>& rb0 = buffers_of<R>(ctx);
   const int poolWant = std::max(pool_records(W, emax_eV, tu.pool), rb0.cap == W ? rb0.poolCap : 0);
@@ -1686,7 +1737,7 @@ static int run_device_once(cm_context* ctx, const cm_run_desc* d, uint32_t* back
     // profiled: the host replays captured iterations (events between the kernels) and reads the
     // counters after each replay
     const int K = kLoopBody;
-    std::vector<cudaEvent_t> pev((size_t)K * 6 + 1), tev((size_t)K * 3 + 1);
+    std::vector<cudaEvent_t> pev((size_t)K * 5 + 1), tev((size_t)K * 2 + 1);
     for (auto& ev : pev) CM_CUDA(cudaEventCreate(&ev));
     for (auto& ev : tev) CM_CUDA(cudaEventCreate(&ev));
     cudaGraph_t graph[2] = {nullptr, nullptr};
@@ -1696,8 +1747,8 @@ static int run_device_once(cm_context* ctx, const cm_run_desc* d, uint32_t* back
       std::vector<cudaEvent_t>& ev = loop == 0 ? pev : tev;
       cudaEventRecordWithFlags(ev[0], stream, cudaEventRecordExternal);
       for (int it = 0; it < K; ++it) {
-        if (loop == 0) launch_queue_iteration<R>(ctx, v, vs, it & 1, grid, smem, stream, nullptr, &pev[(size_t)it * 6 + 1]);
-        else launch_tail_iteration<R>(ctx, v, it & 1, grid, tu.tail_steps, stream, nullptr, &tev[(size_t)it * 3 + 1]);
+        if (loop == 0) launch_queue_iteration<R>(ctx, v, vs, it & 1, grid, smem, stream, nullptr, &pev[(size_t)it * 5 + 1]);
+        else launch_tail_iteration<R>(ctx, v, it & 1, tu.tail_steps, stream, nullptr, &tev[(size_t)it * 2 + 1]);
       }
       CM_CUDA(cudaStreamEndCapture(stream, &graph[loop]));
       CM_CUDA(cudaGraphInstantiate(&exec[loop], graph[loop], 0));
@@ -1710,16 +1761,15 @@ static int run_device_once(cm_context* ctx, const cm_run_desc* d, uint32_t* back
       CM_CUDA(cudaMemcpyAsync(ctx->counters_host, ctx->counters, sizeof(Counters), cudaMemcpyDeviceToHost, stream));
       CM_CUDA(cudaStreamSynchronize(stream));
       for (int it = 0; it < K; ++it) {
-        float ms[6] = {0, 0, 0, 0, 0, 0};
+        float ms[5] = {0, 0, 0, 0, 0};
         if (!tail) {
-          for (int k = 0; k < 6; ++k) cudaEventElapsedTime(&ms[k], pev[(size_t)it * 6 + k], pev[(size_t)it * 6 + k + 1]);
-          static const int order[6] = {CM_K_FLIGHT, CM_K_INELASTIC, CM_K_MISC, CM_K_ELASTIC, CM_K_SPAWN, CM_K_TAIL};
-          for (int k = 0; k < 6; ++k) kms[order[k]] += ms[k];
+          static const int order[5] = {CM_K_FLIGHT, CM_K_INELASTIC, CM_K_MISC, CM_K_ELASTIC, CM_K_SPAWN};
+          for (int k = 0; k < 5; ++k) cudaEventElapsedTime(&ms[k], pev[(size_t)it * 5 + k], pev[(size_t)it * 5 + k + 1]);
+          for (int k = 0; k < 5; ++k) kms[order[k]] += ms[k];
         } else {
-          for (int k = 0; k < 3; ++k) cudaEventElapsedTime(&ms[k], tev[(size_t)it * 3 + k], tev[(size_t)it * 3 + k + 1]);
+          for (int k = 0; k < 2; ++k) cudaEventElapsedTime(&ms[k], tev[(size_t)it * 2 + k], tev[(size_t)it * 2 + k + 1]);
           step_ms += ms[0];
           kms[CM_K_SPAWN] += ms[1];
-          kms[CM_K_TAIL] += ms[2];
         }
       }
       const Counters& hc = *ctx->counters_host;
@@ -1768,7 +1818,8 @@ static int run_device_once(cm_context* ctx, const cm_run_desc* d, uint32_t* back
     st->device_ms = ms;
     for (int k = 0; k < 6; ++k) {
       st->kernel_ms[k] = kms[k];
-      st->kernel_launches[k] = (int64_t)(k < 4 ? qslots : qslots + tslots);
+      // (the end of an iteration, CM_K_TAIL, is the last block of the refill's)
+      st->kernel_launches[k] = (int64_t)(k == CM_K_TAIL ? 0 : k < 4 ? qslots : qslots + tslots);
     }
     for (int k = 0; k < 4; ++k) st->units[k] = (int64_t)c.units[k];
     st->step_launches = tslots;
@@ -3185,8 +3236,7 @@ again:
       const RunView<R> v = view_at(v0, cur);
       if (blocks) {
         launch_block(v, cur, ctx->nsm, CM_TAIL_STEPS, s);
-        launch_spawn<R>(v, cur, grid, s);
-        k_tail<R><<<1, 32, 0, s>>>(v, cur, 1);
+        launch_spawn<R>(v, cur, ctx->nsm, kEndSteps, nullptr, s);
         continue;
       }
       launch_flight(v, cur, grid, s);
@@ -3194,8 +3244,7 @@ again:
       k_elastic<R><<<grid, 256, 0, s>>>(v, cur);
       k_inelastic<R><<<grid, 256, 0, s>>>(v, cur);
       launch_misc<R>(v, cur, grid, s);
-      launch_spawn<R>(v, cur, grid, s);
-      k_tail<R><<<1, 32, 0, s>>>(v, cur, 0);
+      launch_spawn<R>(v, cur, ctx->nsm, 0, nullptr, s);
     }
     CM_CUDA(cudaGetLastError());
     CM_CUDA(cudaMemcpyAsync(&hc, c, sizeof(Counters), cudaMemcpyDeviceToHost, s));
@@ -3234,7 +3283,7 @@ again:
     st->device_ms = ms;
     st->ended_zero_energy = (int64_t)hc.ended_zero;
     st->ended_step_limit = (int64_t)hc.ended_limit;
-    for (int k = 0; k < 6; ++k) st->kernel_launches[k] = blocks && k < 4 ? 0 : it;
+    for (int k = 0; k < 6; ++k) st->kernel_launches[k] = k == CM_K_TAIL || (blocks && k < 4) ? 0 : it;
     st->step_launches = blocks ? it : 0;
     st->step_units = (int64_t)hc.step_units;
     for (int k = 0; k < 4; ++k) st->units[k] = (int64_t)hc.units[k];

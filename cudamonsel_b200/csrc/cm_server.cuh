@@ -371,7 +371,7 @@ static int batch_round(Batcher& b) {
   DevScene<R>& ds = scene_of<R>(ctx);
   int rc;
   if ((rc = build_scene<R>(ctx, ds))) return rc;
-  const cm_tuning tu = resolved_tuning<R>(ctx);
+  const cm_tuning tu = resolved_tuning<R>(ctx, ds.view.depth);
   const int W = tu.wave;
   RunBuffers<R>& rb0 = buffers_of<R>(ctx);
   if (b.counters_live) {
@@ -455,7 +455,7 @@ static int batch_round(Batcher& b) {
     CM_CUDA(cudaStreamBeginCapture(ctx->cap_stream, cudaStreamCaptureModeThreadLocal));
     for (int it = 0; it < (tail ? kTailRound : kLoopBody); ++it) {
       if (loop == 0) launch_queue_iteration<R>(ctx, v, vs, it & 1, grid, smem, ctx->cap_stream, nullptr, nullptr);
-      else launch_tail_iteration<R>(ctx, v, it & 1, grid, tu.tail_steps, ctx->cap_stream, nullptr, nullptr);
+      else launch_tail_iteration<R>(ctx, v, it & 1, tu.tail_steps, ctx->cap_stream, nullptr, nullptr);
     }
     CM_CUDA(cudaStreamEndCapture(ctx->cap_stream, &b.round_graph[loop]));
     CM_CUDA(cudaGraphInstantiate(&b.round_exec[loop], b.round_graph[loop], 0));

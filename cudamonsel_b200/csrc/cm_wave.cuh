@@ -66,6 +66,7 @@ struct Counters {
   Line q[3];
   Line deferred;  // fast flights handed on to the next iteration's full flights
   Line pool;
+  Line ticket;  // blocks of the refill that are done
   Line claim;  // wave electrons taken by the blocks of the resident-steps kernel beyond their first share
   int n[2];       // electrons in each wave
   int error;
@@ -181,7 +182,7 @@ struct RunIO {
   uint32_t *elev, *azim;       // per-pixel angle histograms (182 and 362 counts), or null
   cm_escape_record* log;       // escape log, or null
   long long logCap;
-  // the device-driven loop (k_loop): iteration slots allowed, the tail threshold, queue kernels only to
+  // the device-driven loop (end_iteration): iteration slots allowed, the tail threshold, queue kernels only to
   // the end, and a flag in host memory that cancels the run (null: not cancellable)
   long long max_slots;
   int tail_below;
@@ -535,12 +536,6 @@ CM_D int flight_one(const RunView<R>& v, int i, Sink& sink, StepCounts& sc) {
   return queue;
 }
 
-CM_D int survivors(const Counters* c, int nxt) {
-  int n = 0;
-  for (int k = 0; k < kWaveSegments; ++k) n += c->nc[nxt][k];
-  return n;
-}
-
 // a record appended to the secondary pool; false (and CM_EOVERFLOW) when the pool is full
 template <typename R, typename Sink> CM_D bool pool_push(const RunView<R>& v, const El<R>& se, Sink& sink) {
   const int slot = sink.append(&v.c->pool.v);
@@ -656,8 +651,8 @@ CM_D int misc_one(const RunView<R>& v, int j, El<R>& e, Sink& sink, StepCounts& 
 // refill plan of the next wave: secondaries from the pool first; new primaries
 // only once the pool is empty, and at most W/32 per iteration so that the
 // cascades of one batch of primaries do not all peak together
-CM_D void refill_plan(const Counters* c, int nxt, int W, int poolCap, int& nn, int& take_se, int& take_p) {
-  nn = survivors(c, nxt);
+// (nn: the next wave's survivors)
+CM_D void refill_plan(const Counters* c, int nn, int W, int poolCap, int& take_se, int& take_p) {
   const int cap = c->fill > 0 && c->fill < W ? c->fill : W;
   const int room = cap - nn > 0 ? cap - nn : 0;
   const int pool = c->pool < poolCap ? c->pool : poolCap;  // an overflowed pool holds poolCap valid entries
@@ -707,38 +702,6 @@ CM_D int spawn_one(const RunView<R>& v, int j, int take_se, int poolTop, unsigne
   e.h[0] = e.h[1] = e.h[2] = 0;
   job_start(v, px, sink);
   return wave_segment(v.s, e);
-}
-
-// end of an iteration: counters of the next wave, reset of this one (steps: the iteration ran k_block)
-CM_D void tail_update(Counters* c, int cur, int W, int poolCap, bool steps) {
-  const int nxt = cur ^ 1;
-  int nn, take_se, take_p;
-  refill_plan(c, nxt, W, poolCap, nn, take_se, take_p);
-  if (c->pool > poolCap) c->pool = poolCap;
-  if (!c->done) {
-    if (steps) c->step_units += (unsigned long long)c->n[cur];
-    else c->units[0] += (unsigned long long)(c->n[cur] - c->deferred);
-    c->units[1] += (unsigned long long)c->q[0];
-    c->units[2] += (unsigned long long)c->q[1];
-    c->units[3] += (unsigned long long)c->q[2];
-    c->iterations += 1;
-  }
-  (void)nn;
-  int appended = 0;  // survivors and refills as appended (a stopped job's primaries are not)
-  for (int k = 0; k < kWaveSegments; ++k) {
-    c->nc[nxt][k] += c->ns[k];
-    c->ns[k] = 0;
-    c->nc[cur][k] = 0;
-    appended += c->nc[nxt][k];
-  }
-  c->n[nxt] = appended;
-  c->pool -= take_se;
-  c->next_primary += (unsigned long long)take_p;
-  c->n[cur] = 0;
-  for (int k = 0; k < 3; ++k) c->q[k] = 0;
-  c->deferred = 0;
-  c->claim = 0;
-  c->done = (c->n[nxt] == 0 && c->pool == 0 && c->next_primary == c->total_primaries) ? 1 : 0;
 }
 
 }  // namespace cm

@@ -68,7 +68,8 @@ int cm_set_options(cm_context* ctx, int options);
  * each electron's random stream is keyed by its lineage, so they change only the speed. */
 typedef struct {
   int wave;                    /* electrons per wave segment (default 2^21; 1024 .. 2^24) */
-  int tail_below;              /* k_block runs the tail once fewer electrons are left (default 262144) */
+  int tail_below;              /* k_block runs the tail once fewer electrons are left (default 262144;
+                                  131072 for scenes with unions, or in FP64 intersections) */
   int tail_steps;              /* iterations per launch of the tail kernel (default 64) */
   int blocks_per_sm;           /* grid = SMs x blocks_per_sm blocks of 256 threads (default 8) */
   double ms;                   /* cm_autotune: device time of the transport loop under these settings */
