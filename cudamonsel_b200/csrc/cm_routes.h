@@ -1,0 +1,126 @@
+// cm_routes.h -- what the host derives from a scene so that the kernels can take a short route: the inside
+// of each shape (FastRegion) and the search guides of the table axes (AxisGuide).  Plain C++ over the
+// scene's structs, so that a CPU test can compare the routes with the general searches.
+#pragma once
+#include <cmath>
+#include <cstring>
+#include <vector>
+
+#include "cm_device.cuh"
+
+namespace cm {
+
+// The half-spaces and cylinders whose common part lies strictly (by kFastMarginNm) inside a shape,
+// appended to fp and fc; false when the shape has no such description.  A step with both ends in there
+// crosses nothing as the boundary search sees it: its plane solves find u outside (0, 1] by a margin far
+// above rounding, and an intersection or a union of shapes (one part of it holding the step) reports none.
+static bool inside_of(const std::vector<Shape>& shapes, const std::vector<Plane>& planes, int id,
+                      std::vector<FastPlane>& fp, std::vector<FastCyl>& fc) {
+  const Shape& sh = shapes[id];
+  auto half_space = [&](const double* n, double d) {
+    const double len = sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+    if (!(len > 0) || !std::isfinite(len) || !std::isfinite(d)) return false;
+    fp.push_back(FastPlane{{n[0] / len, n[1] / len, n[2] / len}, d / len - kFastMarginNm});
+    return true;
+  };
+  switch (sh.kind) {
+    case SHAPE_PLANES:
+      for (int i = 0; i < sh.np; ++i) {
+        const Plane& p = planes[sh.plane0 + i];
+        if (!half_space(p.n, p.n[0] * p.p[0] + p.n[1] * p.p[1] + p.n[2] * p.p[2])) return false;
+      }
+      return true;
+    case SHAPE_INTERSECTION:
+      return inside_of(shapes, planes, sh.a, fp, fc) && inside_of(shapes, planes, sh.b, fp, fc);
+    case SHAPE_UNION: {
+      const size_t np = fp.size(), nc = fc.size();
+      if (inside_of(shapes, planes, sh.a, fp, fc) && fc.size() == nc) return true;
+      fp.resize(np);
+      fc.resize(nc);
+      if (inside_of(shapes, planes, sh.b, fp, fc)) return true;
+      fp.resize(np);
+      fc.resize(nc);
+      return false;
+    }
+    case SHAPE_CYLINDER: {
+      // only a cylinder whose axis is normalised is ever struck (see cm_shape_cylinder)
+      const double u = sh.nax[0] * sh.nax[0] + sh.nax[1] * sh.nax[1] + sh.nax[2] * sh.nax[2];
+      const double rad = sqrt(sh.rad2), m = 1e-3 + 1e-9 * sh.len;
+      if (!(fabs(u - 1.0) < 1e-9) || !(rad > 2 * m) || !(sh.len > 4 * m)) return false;
+      const double back[3] = {-sh.nax[0], -sh.nax[1], -sh.nax[2]};
+      const double a0 = sh.nax[0] * sh.e0[0] + sh.nax[1] * sh.e0[1] + sh.nax[2] * sh.e0[2];
+      if (!half_space(sh.nax, a0 + sh.len - m) || !half_space(back, -a0 - m)) return false;
+      fc.push_back(FastCyl{{sh.e0[0], sh.e0[1], sh.e0[2]}, {sh.nax[0], sh.nax[1], sh.nax[2]}, (rad - m) * (rad - m)});
+      return true;
+    }
+    default:
+      return false;  // spheres: the full form
+  }
+}
+
+// The search guide of an ascending axis: linear buckets or the leading bits of the argument, whichever
+// leaves at most one node in every bucket of at most 4096; kind 0 (bisection) when neither does.
+static AxisGuide make_guide(const double* x, int n, std::vector<GuideEntry>& out) {
+  AxisGuide g;
+  memset(&g, 0, sizeof(g));
+  if (n < 4 || n > 60000) return g;
+  for (int i = 0; i < n; ++i)
+    if (!std::isfinite(x[i]) || (i > 0 && !(x[i] > x[i - 1]))) return g;
+  auto bucket = [&](double v) -> int {  // as guide_below does
+    if (g.kind == 1) {
+      const double t = (v - g.x0) * g.scale;
+      return t > 0.0 ? (t < (double)(g.n - 1) ? (int)t : g.n - 1) : 0;
+    }
+    long long bits;
+    memcpy(&bits, &v, 8);
+    const int b = ((int)(bits >> 32) >> g.shift) - g.base;
+    return b < 0 ? 0 : b > g.n - 1 ? g.n - 1 : b;
+  };
+  auto fits = [&]() {
+    for (int i = 1; i < n; ++i)
+      if (bucket(x[i]) == bucket(x[i - 1])) return false;
+    return true;
+  };
+  bool ok = false;
+  g.kind = 1;
+  g.x0 = x[0];
+  for (int per = 1; per <= 8 && !ok; per *= 2) {
+    g.n = (n - 1) * per + 1;
+    if (g.n > 4096) break;
+    g.scale = (double)(g.n - 1) / (x[n - 1] - x[0]);
+    ok = std::isfinite(g.scale) && fits();
+  }
+  if (!ok && x[0] > 0) {
+    g.kind = 2;
+    for (g.shift = 20; g.shift >= 10 && !ok; --g.shift) {
+      long long b0, b1;
+      memcpy(&b0, &x[0], 8);
+      memcpy(&b1, &x[n - 1], 8);
+      g.base = (int)(b0 >> 32) >> g.shift;
+      const long long cells = (((long long)(int)(b1 >> 32)) >> g.shift) - g.base + 1;
+      if (cells > 4096) break;
+      g.n = (int)cells;
+      if ((ok = fits())) break;
+    }
+  }
+  if (!ok) {
+    memset(&g, 0, sizeof(g));
+    return g;
+  }
+  // the order-3 window of an argument with k nodes below it, from the reference's own search
+  auto first3 = [&](int k) {
+    const double v = k == 0 ? x[0] : k == n ? x[n - 1] * 2 + 1 : x[k];  // x[k] has exactly k nodes below it
+    int first, nearest;
+    nu_locate<double>(v, x, n, 3, first, nearest);
+    return (unsigned short)first;
+  };
+  g.off = (int)out.size();
+  int k = 0;
+  for (int b = 0; b < g.n; ++b) {
+    while (k < n && bucket(x[k]) < b) ++k;
+    out.push_back(GuideEntry{(unsigned short)k, first3(k), first3(std::min(k + 1, n)), 0});
+  }
+  return g;
+}
+
+}  // namespace cm
