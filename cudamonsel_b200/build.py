@@ -17,7 +17,7 @@ DEPS = ["cm_engine.cu", "cm_device.cuh", "cm_physics.cuh", "cm_scene.h", "cm_wav
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",
-         "-shared", "-diag-suppress", "20050", "-split-compile", "0"]
+         "-shared", "-diag-suppress", "20050"]
 
 
 def stale():

@@ -18,8 +18,11 @@
 
 namespace cm {
 
+// Threads: 512 (128 registers) in FP32, 384 (168) in FP64, where 128 registers spill 430 bytes a step (one
+// B200, 384 against 512 threads: 10 k primaries FP64 7.5 / 8.1 ms, FP64 line scan 32.9 / 33.4 ms; in FP32
+// the phonon scan 19.6 / 18.8 ms, the others within 2 %).
 #ifndef CM_BLOCK_THREADS
-#define CM_BLOCK_THREADS 512
+#define CM_BLOCK_THREADS (sizeof(R) == 8 ? 384 : 512)
 #endif
 #ifndef CM_BLOCK_MINB
 #define CM_BLOCK_MINB 1
@@ -28,14 +31,20 @@ namespace cm {
 #define CM_BLOCK_SLOTS 1024
 #endif
 
-constexpr int kBlockThreads = CM_BLOCK_THREADS;
+template <typename R> constexpr int kBlockThreads = CM_BLOCK_THREADS;
 constexpr int kBlockSlots = CM_BLOCK_SLOTS;
 constexpr int kBlockPerSm = CM_BLOCK_MINB;
 // lists a slot can be in: the flights of each wave segment, the inelastic and the misc events, the flights
 // that need the full form
-constexpr int kListSlow = kSlowSegment, kListTab = kWaveSegments, kListMisc = kWaveSegments + 1, kListDead = kWaveSegments + 2;
+constexpr int kListSlow = kSlowSegment, kListOpen = kOpenSegment, kListTab = kWaveSegments, kListMisc = kWaveSegments + 1, kListDead = kWaveSegments + 2;
 constexpr int kLists = kWaveSegments + 3;
 constexpr int kListNone = kLists;
+// The list of a wave segment's electrons.  Over leaf shapes both kinds of full flights share one (a block has
+// few of them; two lists: 8 % slower for the quick line scan), over trees, whose walks are long and unlike,
+// each has its own (one list: 2 % slower for the FP64 image).
+template <int D> __device__ __forceinline__ int block_list(int segment) {
+  return D == 0 && segment == kOpenSegment ? kListSlow : segment;
+}
 // iterations after which a block passes what is left of the wave on to the next one instead of taking it
 constexpr int kBlockHardLimit = 4096;
 
@@ -97,7 +106,7 @@ struct BlockMem {
 };
 
 // secondaries take a free slot of the block, or go to the run's pool when there is none
-template <typename R>
+template <typename R, int D>
 struct BlockSink : DeviceSink {
   int par;  // parity of the lists being filled
   __device__ __forceinline__ explicit BlockSink(int p) : par(p) {}
@@ -108,7 +117,7 @@ struct BlockSink : DeviceSink {
     const int slot = B::free_slot(avail - 1 - k);
     B::store(slot, se);
     B::born(slot) = 1;
-    B::put(par, wave_segment(v.s, se), slot);
+    B::put(par, block_list<D>(wave_segment(v.s, se)), slot);
     return true;
   }
 };
@@ -116,15 +125,15 @@ struct BlockSink : DeviceSink {
 // One task: up to 32 electrons of one list through their flight (with the elastic event it ends in) or
 // their queued event.  Every lane of the warp calls it; lanes without an electron have slot < 0.
 template <typename R, int D>
-__device__ __forceinline__ void block_task(const RunView<R>& v, int l, int slot, BlockSink<R>& sink, StepCounts& sc) {
+__device__ __forceinline__ void block_task(const RunView<R>& v, int l, int slot, BlockSink<R, D>& sink, StepCounts& sc) {
   using B = BlockMem<R>;
   int dest = kListNone;
   if (slot >= 0) {
     El<R> e = B::load(slot);
     bool alive;
     dest = kListDead;
-    if (l <= kListSlow) {
-      const int q = l == kListSlow ? flight_apply<R, D>(v, e, sink, sc) : flight_fast(v, e, sc, [](El<R>&) {});
+    if (l <= kListOpen) {
+      const int q = l >= kListSlow ? flight_apply<R, D>(v, e, sink, sc) : flight_fast(v, e, sc, [](El<R>&) {});
       alive = q >= 0;
       if (q == Q_EL) alive = elastic_apply(v, e);
       if (q == Q_SLOW) {
@@ -142,7 +151,7 @@ __device__ __forceinline__ void block_task(const RunView<R>& v, int l, int slot,
           if (aux_kind(e.aux) == AUX_BARRIER)
             for (int a = 0; a < 3; ++a) B::r(5 + a, slot) = e.h[a];
         }
-        dest = q == Q_EL ? segment_after(v.s, e) : q == Q_TAB ? kListTab : kListMisc;
+        dest = q == Q_EL ? block_list<D>(segment_after(v.s, e)) : q == Q_TAB ? kListTab : kListMisc;
       }
     } else {
       e.Ep = B::r(4, slot);
@@ -160,7 +169,7 @@ __device__ __forceinline__ void block_task(const RunView<R>& v, int l, int slot,
       if (alive) {
         for (int a = 0; a < 3; ++a) B::r(a, slot) = e.d[a];
         B::r(3, slot) = e.E;
-        dest = segment_after(v.s, e);
+        dest = block_list<D>(segment_after(v.s, e));
       }
     }
     if (!alive) job_end(v, e.pixel, e.step, sink);
@@ -179,30 +188,29 @@ __device__ __forceinline__ void block_task(const RunView<R>& v, int l, int slot,
 // The tasks of an iteration: 32 entries of one list each, events first (they take longest).  events_only:
 // the flights stay in their lists.
 template <typename R, int D>
-__device__ __forceinline__ void block_stage(const RunView<R>& v, int par, bool events_only, BlockSink<R>& sink,
+__device__ __forceinline__ void block_stage(const RunView<R>& v, int par, bool events_only, BlockSink<R, D>& sink,
                                             StepCounts& sc) {
   using B = BlockMem<R>;
+  // Lane k holds the k-th list in the order they are worked off (the longest tasks first), its entries and the
+  // tasks up to its end; a task's list is then one ballot away.
   const int lane = threadIdx.x & 31;
+  const int mine = lane == 0 ? kListTab : lane == 1 ? kListMisc : lane == 2 ? kListOpen : lane == 3 ? kListSlow : lane - 4;
+  const int n = lane < kSegments + 4 && !(events_only && lane > 1) ? B::ctl().cnt[par][mine] : 0;
+  int end = (n + 31) >> 5;
+  for (int off = 1; off < 16; off <<= 1) {
+    const int up = __shfl_up_sync(0xffffffffu, end, off);
+    if (lane >= off) end += up;
+  }
+  const int begin = end - ((n + 31) >> 5);
   for (;;) {
     int t = 0;
     if (lane == 0) t = atomicAdd(&B::ctl().task, 1);
     t = __shfl_sync(0xffffffffu, t, 0);
-    int l = kListTab, n;
-    for (;;) {  // the list this task falls in: inelastic, misc, full flights, then the segments
-      n = B::ctl().cnt[par][l];
-      const int k = (n + 31) >> 5;
-      if (t < k) break;
-      t -= k;
-      if (l == kListTab) l = kListMisc;
-      else if (l == kListMisc) {
-        if (events_only) return;
-        l = kListSlow;
-      } else if (l == kListSlow) {
-        l = 0;
-      } else if (++l == kSegments) return;
-    }
-    const int i = 32 * t + lane;
-    const int slot = i < n ? (int)B::list(par, l, i) : -1;
+    const unsigned after = __ballot_sync(0xffffffffu, t < end && lane < kSegments + 4);
+    if (!after) return;
+    const int k = __ffs(after) - 1;
+    const int l = __shfl_sync(0xffffffffu, mine, k), i = 32 * (t - __shfl_sync(0xffffffffu, begin, k)) + lane;
+    const int slot = i < __shfl_sync(0xffffffffu, n, k) ? (int)B::list(par, l, i) : -1;
     block_task<R, D>(v, l, slot, sink, sc);
   }
 }
@@ -210,11 +218,11 @@ __device__ __forceinline__ void block_stage(const RunView<R>& v, int par, bool e
 // Electrons of wave `cur` through about `iters` iterations (a flight with its elastic event, or a queued
 // event, per electron and iteration), survivors kept in the next wave.  cap: slots a block may use.
 template <typename R, int D>
-__global__ void __launch_bounds__(kBlockThreads, kBlockPerSm) k_block(const __grid_constant__ RunView<R> v, int cur, int iters, int cap) {
+__global__ void __launch_bounds__(kBlockThreads<R>, kBlockPerSm) k_block(const __grid_constant__ RunView<R> v, int cur, int iters, int cap) {
   using B = BlockMem<R>;
   BlockCtl& c = B::ctl();
   const int n = v.c->n[cur];
-  const int grid = gridDim.x, tid = threadIdx.x, T = kBlockThreads;
+  const int grid = gridDim.x, tid = threadIdx.x, T = kBlockThreads<R>;
   if (n == 0) return;
   __shared__ int first[kWaveSegments + 1];
   segment_starts(v.c, cur, first);
@@ -242,7 +250,7 @@ __global__ void __launch_bounds__(kBlockThreads, kBlockPerSm) k_block(const __gr
     const El<R> e = load_live(v.now, k * v.W + (i - first[k]));
     B::store(slot, e);
     B::born(slot) = 0;
-    B::put(par, k, slot);
+    B::put(par, block_list<D>(k), slot);
   };
   for (int j = tid; j < mine; j += T) take((j / run * grid + (int)blockIdx.x) * run + j % run, j, 0);
   if (tid == 0) {
@@ -259,7 +267,7 @@ __global__ void __launch_bounds__(kBlockThreads, kBlockPerSm) k_block(const __gr
     // the last iteration runs the queued events only, so that every electron ends between two steps
     const bool out = c.exhausted != 0;
     const bool last = (c.nfree == cap && out) || (it >= iters && out) || it >= kBlockHardLimit;
-    BlockSink<R> sink(par ^ 1);
+    BlockSink<R, D> sink(par ^ 1);
     block_stage<R, D>(v, par, last, sink, sc);
     __syncthreads();
     if (last) break;
@@ -327,21 +335,25 @@ __global__ void __launch_bounds__(kBlockThreads, kBlockPerSm) k_block(const __gr
 
 // Slots per block: all of them, or fewer for a small wave, so that the blocks together hold about a wave of
 // electrons at most: the secondary pool is sized by the wave, and what the blocks hold may end in it.
-static int block_cap(int W, int grid) {
-  const int cap = W / grid;
+static int block_cap(int held, int grid) {
+  const int cap = held / grid;
   return cap > kBlockSlots ? kBlockSlots : cap < 1 ? 1 : cap;
 }
 
-template <typename R, int D> static void launch_block_d(const RunView<R>& v, int cur, int nsm, int iters, cudaStream_t s) {
+template <typename R, int D>
+static void launch_block_d(const RunView<R>& v, int cur, int nsm, int iters, cudaStream_t s, int held) {
   const int grid = nsm * kBlockPerSm;
   cudaFuncSetAttribute(k_block<R, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, BlockMem<R>::kBytes);
-  k_block<R, D><<<grid, kBlockThreads, BlockMem<R>::kBytes, s>>>(v, cur, iters, block_cap(v.W, grid));
+  k_block<R, D><<<grid, kBlockThreads<R>, BlockMem<R>::kBytes, s>>>(v, cur, iters, block_cap(held, grid));
 }
 
-template <typename R> static void launch_block(const RunView<R>& v, int cur, int nsm, int iters, cudaStream_t s) {
-  if (v.s.depth == 0) launch_block_d<R, 0>(v, cur, nsm, iters, s);
-  else if (v.s.depth <= 2) launch_block_d<R, 2>(v, cur, nsm, iters, s);
-  else launch_block_d<R, kMaxShapeDepth>(v, cur, nsm, iters, s);
+// held: electrons the blocks may hold together (0: a wave)
+template <typename R>
+static void launch_block(const RunView<R>& v, int cur, int nsm, int iters, cudaStream_t s, int held = 0) {
+  if (held <= 0) held = v.W;
+  if (v.s.depth == 0) launch_block_d<R, 0>(v, cur, nsm, iters, s, held);
+  else if (v.s.depth <= 2) launch_block_d<R, 2>(v, cur, nsm, iters, s, held);
+  else launch_block_d<R, kMaxShapeDepth>(v, cur, nsm, iters, s, held);
 }
 
 }  // namespace cm

@@ -688,6 +688,9 @@ CM_D NV planes_first_normal(const Plane* pl, int np, const double* p0, const dou
       if ((num < 0) || ((num == 0) && tie_break(P.n))) continue;
       return nv_none();
     }
+    // From inside the plane, moving inwards (u < 0) or not reaching it (u > 1, by a margin far above
+    // rounding): such a u changes no outcome below, whatever the other planes give, and is not divided out.
+    if (num < 0 && (den < 0 || -num > den * 1.000001)) continue;
     const double u = -num / den;
     if (den > 0) {
       if (u < umax) {

@@ -983,7 +983,7 @@ __device__ __forceinline__ int segment_of(const int* first, int i) {
 template <typename R> __device__ __forceinline__ void flight_fast_loop(const RunView<R>& v, int cur) {
   DeviceSink sink;
   StepCounts sc;
-  const int n = v.c->n[cur] - v.c->nc[cur][kSlowSegment];
+  const int n = v.c->n[cur] - v.c->nc[cur][kSlowSegment] - v.c->nc[cur][kOpenSegment];
   if ((int)(blockIdx.x * blockDim.x) >= n) return;
   __shared__ int first[kWaveSegments + 1];
   segment_starts(v.c, cur, first);
@@ -1020,19 +1020,21 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? CM_MINB_FLIGHT32 : CM_MI
   flight_fast_loop(v, cur);
 }
 
-// the full form of the flights in the wave's slow segment
-template <typename R, int D> __global__ void __launch_bounds__(256) k_flight(const __grid_constant__ RunView<R> v, int cur) {
+// the full form of the flights in the wave's last two segments
+template <typename R, int D> __global__ void __launch_bounds__(256, D == 0 ? 2 : 1) k_flight(const __grid_constant__ RunView<R> v, int cur) {
   DeviceSink sink;
   StepCounts sc;
-  const int n = v.c->nc[cur][kSlowSegment];
+  // both segments, the second from a warp of its own on
+  const int ns = v.c->nc[cur][kSlowSegment], no = (ns + 31) & ~31, n = no + v.c->nc[cur][kOpenSegment];
   if ((int)(blockIdx.x * blockDim.x) >= n) return;
   __shared__ BlockAppend<3> app;
   append_init(app);
   int par = 0;
   for (int j0 = blockIdx.x * blockDim.x; j0 < n; j0 += gridDim.x * blockDim.x, par ^= 1) {
-    const int w = kSlowSegment * v.W + j0 + threadIdx.x;
+    const int j = j0 + (int)threadIdx.x;
+    const int w = j < no ? kSlowSegment * v.W + j : kOpenSegment * v.W + j - no;
     int dest = -1;
-    if (j0 + (int)threadIdx.x < n) dest = flight_one<R, D, false>(v, w, sink, sc);
+    if (j < ns || (j >= no && j < n)) dest = flight_one<R, D, false>(v, w, sink, sc);
     const int slot = append_slot(app, par, dest, [&](int k) { return &v.c->q[k].v; });
     if (dest >= 0) v.q[dest][slot] = w;
   }
@@ -1105,7 +1107,7 @@ __global__ void CM_LB_INELASTIC k_inelastic(const __grid_constant__ RunView<R> v
 }
 
 template <typename R, int D>
-__global__ void __launch_bounds__(256) k_misc(const __grid_constant__ RunView<R> v, int cur) {
+__global__ void __launch_bounds__(256, D == 0 ? (sizeof(R) == 4 ? 4 : 3) : 2) k_misc(const __grid_constant__ RunView<R> v, int cur) {
   DeviceSink sink;
   StepCounts sc;
   const int n = v.c->q[Q_MISC];
@@ -1187,7 +1189,7 @@ __device__ __forceinline__ void end_iteration(const RunView<R>& v, int cur, int 
   __syncwarp();
   if (lane != 0) return;
   int take_se, take_p;
-  refill_plan(c, nn, v.W, v.poolCap, take_se, take_p);
+  refill_plan(c, nn, v.W, v.poolCap, (end & kEndSteps) != 0, take_se, take_p);
   int pool = c->pool < v.poolCap ? (int)c->pool : v.poolCap;
   const unsigned long long next = c->next_primary + (unsigned long long)take_p, total = c->total_primaries;
   const int was = c->n[cur], error0 = c->error;
@@ -1228,7 +1230,7 @@ __global__ void __launch_bounds__(256) k_spawn(const __grid_constant__ RunView<R
   int nn = 0, take_se, take_p;
 #pragma unroll
   for (int k = 0; k < kWaveSegments; ++k) nn += v.c->nc[nxt][k];
-  refill_plan(v.c, nn, v.W, v.poolCap, take_se, take_p);
+  refill_plan(v.c, nn, v.W, v.poolCap, (end & kEndSteps) != 0, take_se, take_p);
   const int poolTop = v.c->pool < v.poolCap ? (int)v.c->pool : v.poolCap;
   const unsigned long long first = v.c->next_primary;
   const int n = take_se + take_p;
@@ -3067,10 +3069,12 @@ static int run_noalloc(cm_context* ctx, const cm_run_desc* d, uint32_t* back, ui
   const size_t rec = 3 * 8 + 8 * sizeof(R) + 4 * 4 + 8;
   const size_t pad = 3 * Wave<R>::kTile + 6 * 256;  // worst-case rounding of the 6 pieces below
   const size_t left = kNoAllocScratchBytes - a.off;
-  long long W = (long long)((left > pad ? left - pad : 0) / ((2 * kWaveSegments + 8) * rec + 3 * 4));
+  const size_t room = left > pad ? left - pad : 0;
+  // a third of the room to the pool (its capacity decides which runs fit), the rest to the waves and queues
+  const int poolCap = (int)(8 * (room / (24 * rec + 12)));
+  long long W = (long long)((room - (size_t)poolCap * rec) / (2 * kWaveSegments * rec + 3 * 4));
   if (d->wave > 0 && d->wave < W) W = d->wave;
   if (W < 1024) return fail(CM_EINVAL, "cm_run_noalloc: no room for a wave of 1024 electrons");
-  const int poolCap = (int)(8 * W);
   RunView<R> v;
 #ifdef CM_TRACE
   v.trace = nullptr;
@@ -3123,7 +3127,8 @@ again:
       const int cur = it & 1;
       const RunView<R> v = view_at(v0, cur);
       if (blocks) {
-        launch_block(v, cur, ctx->nsm, CM_TAIL_STEPS, s);
+        // (secondaries the blocks still hold at a launch's end fit half the pool)
+        launch_block(v, cur, ctx->nsm, CM_TAIL_STEPS, s, (int)W + poolCap / 2);
         launch_spawn<R>(v, cur, ctx->nsm, kEndSteps, nullptr, s);
         continue;
       }

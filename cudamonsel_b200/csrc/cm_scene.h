@@ -86,10 +86,10 @@ constexpr int kClasses = 4;
 // a warp's threads mostly run the same branches
 constexpr int kSegments = 2 * kClasses;
 constexpr double kSegmentSplitEv = 50.0;
-// and one more for the electrons whose next step may meet a boundary or needs no mechanism (those in regions
-// without a FastRegion description, at a boundary just met, or handed back by the fast flight): the full
-// flight takes these
-constexpr int kSlowSegment = kSegments, kWaveSegments = kSegments + 1;
+// and two more for the full flight: kSlowSegment for electrons that may meet a boundary of their region (at
+// one just met, or handed back by the fast flight), kOpenSegment for those in a region without a FastRegion
+// description (vacuum, a region with children), whose steps run through other code
+constexpr int kSlowSegment = kSegments, kOpenSegment = kSegments + 1, kWaveSegments = kSegments + 2;
 constexpr int kMaxWave = 1 << 27;  // electrons per wave segment: kWaveSegments x and 8 x (the pool) stay within int
 
 // The structs the transport kernels read are in the compute precision R, rounded once when the scene is

@@ -141,17 +141,18 @@ CM_HD int aux_kind(int a) { return (a >> 24) & 15; }
 CM_HD int aux_val(int a) { return a & 0xffffff; }
 
 // Wave segment of an electron: its material's class, split at kSegmentSplitEv, when it is strictly inside
-// its region (which the fast flight takes as given), else the slow segment.  inside: known to be.
+// its region (which the fast flight takes as given), else one of the full flight's.  inside: known to be.
 template <typename R> CM_D int wave_segment(const SceneView<R>& s, const El<R>& e, bool inside = false) {
-  if (e.region < 0) return kSlowSegment;
+  if (e.region < 0) return kOpenSegment;
   const FastRegion f = s.fast[e.region];
-  if (!inside && (f.np < 0 || !point_inside(s, f, e.p))) return kSlowSegment;
+  if (f.np < 0) return kOpenSegment;
+  if (!inside && !point_inside(s, f, e.p)) return kSlowSegment;
   return 2 * f.cls + (e.E < (R)kSegmentSplitEv ? 1 : 0);
 }
 
-// the segment after an event: an electron at a boundary just met is within the margin of it
+// the segment after an event
 template <typename R> CM_D int segment_after(const SceneView<R>& s, const El<R>& e) {
-  return aux_kind(e.aux) == AUX_BARRIER ? kSlowSegment : wave_segment(s, e, (e.aux & AUX_INSIDE) != 0);
+  return wave_segment(s, e, (e.aux & AUX_INSIDE) != 0);
 }
 
 #ifdef CM_TRACE
@@ -649,17 +650,18 @@ CM_D int misc_one(const RunView<R>& v, int j, El<R>& e, Sink& sink, StepCounts& 
 }
 
 // refill plan of the next wave: secondaries from the pool first; new primaries
-// only once the pool is empty, and at most W/32 per iteration so that the
-// cascades of one batch of primaries do not all peak together
+// only once the pool is empty, and at most W/32 per iteration (W/4 per launch of
+// k_block, which takes many steps) so that the cascades of one batch of primaries do
+// not all peak together
 // (nn: the next wave's survivors)
-CM_D void refill_plan(const Counters* c, int nn, int W, int poolCap, int& take_se, int& take_p) {
+CM_D void refill_plan(const Counters* c, int nn, int W, int poolCap, bool steps, int& take_se, int& take_p) {
   const int cap = c->fill > 0 && c->fill < W ? c->fill : W;
   const int room = cap - nn > 0 ? cap - nn : 0;
   const int pool = c->pool < poolCap ? c->pool : poolCap;  // an overflowed pool holds poolCap valid entries
   take_se = pool < room ? pool : room;
   const unsigned long long rem = c->total_primaries - c->next_primary;
   int left = pool > take_se ? 0 : room - take_se;
-  const int ramp = W / 32 > 1 ? W / 32 : 1;
+  const int batch = steps ? W / 4 : W / 32, ramp = batch > 1 ? batch : 1;
   if (left > ramp) left = ramp;
   take_p = rem < (unsigned long long)left ? (int)rem : left;
 }

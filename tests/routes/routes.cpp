@@ -170,6 +170,74 @@ static void check_boxes() {
   }
 }
 
+// NormalMultiPlaneShape::getFirstNormal with every quotient formed
+static NV first_normal_plain(const std::vector<Plane>& pl, const double* p0, const double* p1) {
+  double umin = -INFINITY, umax = INFINITY;
+  int lo = -1, hi = -1;
+  for (int i = 0; i < (int)pl.size(); ++i) {
+    double num = 0, den = 0;
+    for (int a = 0; a < 3; ++a) {
+      num += (p0[a] - pl[i].p[a]) * pl[i].n[a];
+      den += (p1[a] - p0[a]) * pl[i].n[a];
+    }
+    if (den == 0) {
+      if (num < 0 || (num == 0 && tie_break(pl[i].n))) continue;
+      return nv_none();
+    }
+    const double u = -num / den;
+    if (den > 0) {
+      if (u < umax) {
+        if (u < 0 || u <= umin) return nv_none();
+        umax = u;
+        hi = i;
+      }
+    } else if (u > umin) {
+      if (u > 1 || u >= umax) return nv_none();
+      umin = u;
+      lo = i;
+    }
+  }
+  NV r = nv_none();
+  const int k = umin > 0 ? lo : umax <= 1 && umax > 0 ? hi : -1;
+  if (k < 0) return r;
+  r.u = umin > 0 ? umin : umax;
+  for (int a = 0; a < 3; ++a) r.n[a] = pl[k].n[a];
+  return r;
+}
+
+static void check_planes() {
+  std::mt19937_64 r(23);
+  std::uniform_real_distribution<double> u(-1.0, 1.0);
+  long hits = 0;
+  for (int k = 0; k < 400000; ++k) {
+    const int np = 1 + k % 8;
+    std::vector<Plane> pl;
+    double p0[3], p1[3];
+    const double len = pow(10.0, 4 * u(r));
+    for (int a = 0; a < 3; ++a) {
+      p0[a] = 30 * u(r);
+      p1[a] = p0[a] + len * u(r);
+    }
+    for (int i = 0; i < np; ++i) {
+      Plane P;
+      double m = 0;
+      for (int a = 0; a < 3; ++a) {
+        P.n[a] = k % 3 == 0 ? (double)(int)(2.5 * u(r)) : u(r);
+        P.p[a] = k % 3 == 0 ? (double)(int)(30 * u(r)) : 30 * u(r);
+        m += P.n[a] * P.n[a];
+      }
+      if (m == 0) P.n[2] = 1;
+      if (k % 5 == 0)  // a plane through an end of the step
+        for (int a = 0; a < 3; ++a) P.p[a] = i % 2 ? p0[a] : p1[a];
+      pl.push_back(P);
+    }
+    const NV a = planes_first_normal(pl.data(), np, p0, p1), b = first_normal_plain(pl, p0, p1);
+    hits += b.u <= 1;
+    CHECK(a.u == b.u && (a.u > 1 || (a.n[0] == b.n[0] && a.n[1] == b.n[1] && a.n[2] == b.n[2])), "planes: u %.17g %.17g", a.u, b.u);
+  }
+  CHECK(hits > 10000, "planes: only %ld crossings", hits);
+}
+
 int main() {
   auto axis = [](int n, auto f) {
     std::vector<double> x;
@@ -234,6 +302,7 @@ int main() {
   check_shape("union with an unnormalised cylinder", s, ghosts, 60, true);
   check_shape("sphere", s, sphere, 60, false);
   check_boxes();
+  check_planes();
   printf("%ld checks, %d failures\n", checks, failures);
   return failures ? 1 : 0;
 }
