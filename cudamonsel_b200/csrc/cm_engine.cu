@@ -1426,6 +1426,17 @@ static bool starts_in_tail(unsigned long long total, double emax_eV, int tail_be
   return (double)total * (1.0 + emax_eV / 100.0) < (double)tail_below;
 }
 
+// the side streams of a captured iteration, made when a context first captures one
+static int ensure_side(cm_context* ctx) {
+  if (ctx->fork_ev) return 0;
+  for (int k = 0; k < 2; ++k) {
+    if (!ctx->side[k]) CM_CUDA(cudaStreamCreateWithFlags(&ctx->side[k], cudaStreamNonBlocking));
+    if (!ctx->join_ev[k]) CM_CUDA(cudaEventCreateWithFlags(&ctx->join_ev[k], cudaEventDisableTiming));
+  }
+  CM_CUDA(cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming));
+  return 0;
+}
+
 // One graph for a whole run: a gate, a WHILE loop of queue iterations, a gate, a WHILE loop of tail
 // iterations (CUDA conditional nodes; end_iteration decides on the device whether a loop goes on).  Its kernels
 // read the run's inputs through v.io, so the instantiated graph is kept in the buffers and serves every
@@ -1435,6 +1446,7 @@ static int build_loop_graph(cm_context* ctx, RunBuffers<R>& rb, const RunView<R>
                             size_t smem, int tail_steps) {
   NvtxRange range("cm launch graph");
   rb.drop_graph();
+  if (const int rc = ensure_side(ctx)) return rc;
   cudaGraph_t g = nullptr;
   CM_CUDA(cudaGraphCreate(&g, 0));
   auto bail = [&](cudaError_t e, const char* what) -> int {
@@ -1959,11 +1971,6 @@ int cm_context_create(int device, cm_context** out) {
   if (stack < 8192) CM_CUDA(cudaDeviceSetLimit(cudaLimitStackSize, 8192));
   CM_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   CM_CUDA(cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking));
-  CM_CUDA(cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming));
-  for (int k = 0; k < 2; ++k) {
-    CM_CUDA(cudaStreamCreateWithFlags(&c->side[k], cudaStreamNonBlocking));
-    CM_CUDA(cudaEventCreateWithFlags(&c->join_ev[k], cudaEventDisableTiming));
-  }
   CM_CUDA(cudaMalloc(&c->counters, sizeof(Counters)));
   CM_CUDA(cudaMallocHost(&c->counters_host, sizeof(Counters)));
   CM_CUDA(cudaMallocHost(&c->io_host, sizeof(RunIO)));

@@ -452,6 +452,7 @@ static int batch_round(Batcher& b) {
   }
   const int loop = tail ? 1 : 0;
   if (!b.round_exec[loop]) {  // each kind of round is captured when the batch first needs it
+    if ((rc = ensure_side(ctx))) return rc;
     CM_CUDA(cudaStreamBeginCapture(ctx->cap_stream, cudaStreamCaptureModeThreadLocal));
     for (int it = 0; it < (tail ? kTailRound : kLoopBody); ++it) {
       if (loop == 0) launch_queue_iteration<R>(ctx, v, vs, it & 1, grid, smem, ctx->cap_stream, nullptr, nullptr);

@@ -214,7 +214,7 @@ typedef struct cm_escape_record {
 #define CM_K_INELASTIC 2
 #define CM_K_MISC 3
 #define CM_K_SPAWN 4
-#define CM_K_TAIL 5
+#define CM_K_TAIL 5 /* the end of an iteration: part of CM_K_SPAWN, its time and launches are 0 */
 
 typedef struct {
   int64_t primaries, steps, scatter_events, barrier_events, escapes, secondaries, iterations;
