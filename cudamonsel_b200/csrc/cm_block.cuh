@@ -7,12 +7,13 @@
 // appends is the next one's lists, so a warp runs one kind of work at a time although a thread sees every
 // kind, and secondaries start at once in the slots of electrons that ended.
 //
-// It runs where few electrons are left: there the queue kernels cost ~55 us an iteration (six launches and
-// their serial latency) however few electrons they move, and one electron per thread through whole steps
-// leaves a warp's lanes in different events (measured before this kernel: 26 M steps of a 3 keV scan with
-// phonons 61 ms, now 20 ms; the last 256 k electrons of a 500 eV line scan 12.3 -> 7.7 ms in FP32, 42 ->
-// 23 ms in FP64).  With the GPU full the queue kernels move 3.8 G electron-steps/s and this kernel 2.3 G
-// (16 warps per SM against their 24 and more), so they keep the full waves.
+// What bounds it: instruction fetch (the warps run different code), the barriers of an iteration, whose pace
+// is the longest task's, and in small runs the serial latency of a step (~9 us).  It runs where few electrons
+// are left: there the queue kernels take ~55 us an iteration however few electrons they move, and one
+// electron per thread through whole steps, which this kernel replaced, left a warp's lanes in different
+// events (one B200: 26 M steps of a 3 keV scan with phonons 62 -> 18.7 ms, 10 k primaries of 1 keV in FP64
+// 17.3 -> 7.8 ms, the last 256 k electrons of a 500 eV line scan 12.3 -> 6.2 ms).  With the GPU full the queue
+// kernels move 5.5 G electron-steps/s and this kernel about 2 G, so they keep the full waves.
 //
 #pragma once
 
