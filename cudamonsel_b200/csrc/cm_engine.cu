@@ -712,7 +712,9 @@ static int build_scene(cm_context* ctx, DevScene<R>& ds) {
     r.shape = hr.shape;
     r.child0 = (int)children.size();
     r.nchild = (int)hr.children.size();
-    r.cls = hr.msm < kClasses ? hr.msm : kClasses - 1;
+    int rank = 0;  // among the models with mechanisms
+    for (int k = 0; k < hr.msm; ++k) rank += msms[k].nmech > 0;
+    r.cls = std::min(rank, kClasses - 1);
     // the box in nm, widened so that rounding never excludes a crossing or a point on the surface
     const Box bx = shape_box(ctx, hr.shape);
     for (int a = 0; a < 3; ++a) {

@@ -80,7 +80,8 @@ constexpr double kFastMarginNm = 1e-4;
 
 // electrons are kept in one wave segment per material class, so that the
 // threads of a warp mostly run the same material's code
-constexpr int kClasses = 4;
+// (of the models with mechanisms: vacuum has none and takes no fast flight)
+constexpr int kClasses = 3;
 // a wave has two segments per class: electrons at or above kSegmentSplitEv and below it (the low band
 // takes the Browning branch of the elastic cross sections and the low-energy secondary paths), so that
 // a warp's threads mostly run the same branches
