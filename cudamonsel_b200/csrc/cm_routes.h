@@ -109,7 +109,7 @@ static AxisGuide make_guide(const double* x, int n, std::vector<GuideEntry>& out
   }
   // the order-3 window of an argument with k nodes below it, from the reference's own search
   auto first3 = [&](int k) {
-    const double v = k == 0 ? x[0] : k == n ? x[n - 1] * 2 + 1 : x[k];  // x[k] has exactly k nodes below it
+    const double v = k == n ? INFINITY : x[k];  // has exactly k nodes below it
     int first, nearest;
     nu_locate<double>(v, x, n, 3, first, nearest);
     return (unsigned short)first;

@@ -1,0 +1,37 @@
+"""The kernels' short routes at the ends of their ranges, through the public entry points."""
+import numpy as np
+import pytest
+
+FP64, FP32 = 0, 1
+pytestmark = pytest.mark.gpu
+
+
+def cubic(xs, f, x):
+    """The cubic through four nodes at x, in 64 bits."""
+    return sum(f[i] * np.prod([(x - xs[j]) / (xs[i] - xs[j]) for j in range(4) if j != i]) for i in range(4))
+
+
+@pytest.mark.parametrize("prec", [FP64, FP32], ids=["fp64", "fp32"])
+def test_tables_beyond_an_axis_that_ends_below_zero(prec):
+    """2-D and 3-D tables whose first axis runs from -20 to -5.57: an argument above its last node is
+    extrapolated from the last four nodes.  The values are random, so another window is off by about one.
+    FP64: 15 (the weights' sum one interval beyond) times rounding, with room.  FP32: an abscissa's rounding of
+    1e-6 in an interval of 0.37, times the weights' slope of about 30, is 1e-4, with room."""
+    from cudamonsel_b200 import capi
+    rng = np.random.default_rng(3)
+    a = -20.0 + 0.37 * np.arange(40)
+    b, c = np.linspace(0.0, 1.0, 9), np.linspace(0.0, 1.0, 7)
+    v2, v3 = rng.random((40, 9)), rng.random((40, 9, 7))
+    e = capi.Engine(0)
+    e.set_options(1)  # 3-D tables with the window's own abscissae in every step
+    t2, t3 = e.table(2, [40, 9], [a, b], v2), e.table(3, [40, 9, 7], [a, b, c], v3)
+    xs = a[-1] + 0.37 * np.array([0.001, 0.25, 0.5, 1.0])
+    x = np.stack([xs, np.full(4, b[4]), np.full(4, c[3])], axis=1)
+    got2, got3 = e.eval_table(t2, x, 3, prec), e.eval_table(t3, x, 3, prec)
+    first = e.eval_locate(t2, x, 3, prec)[:, 0]
+    e.close()
+    assert (first == 36).all()
+    tol = 1e-11 if prec == FP64 else 2e-3
+    for k in range(4):
+        assert abs(got2[k] - cubic(a[-4:], v2[-4:, 4], xs[k])) < tol
+        assert abs(got3[k] - cubic(a[-4:], v3[-4:, 4, 3], xs[k])) < tol
