@@ -10,24 +10,30 @@
 
 namespace cm {
 
-// The half-spaces and cylinders whose common part lies strictly (by kFastMarginNm) inside a shape,
+// The half-spaces and cylinders whose common part lies strictly (by kFastMarginNm or more) inside a shape,
 // appended to fp and fc; false when the shape has no such description.  A step with both ends in there
 // crosses nothing as the boundary search sees it: its plane solves find u outside (0, 1] by a margin far
 // above rounding, and an intersection or a union of shapes (one part of it holding the step) reports none.
+// The margin grows with what the searches round: by 1e-14 of the distance of the point a plane or cylinder
+// is given by (their dot products round to a few 1e-16 of it), and in a cylinder so that the squared
+// distance from the wall, 2 rad m, stays above 1e-14 len^2 (the search takes it as the difference of squares
+// of the length, rounded to at most 7e-15 len^2).
 static bool inside_of(const std::vector<Shape>& shapes, const std::vector<Plane>& planes, int id,
                       std::vector<FastPlane>& fp, std::vector<FastCyl>& fc) {
   const Shape& sh = shapes[id];
-  auto half_space = [&](const double* n, double d) {
+  auto rounding = [](const double* p) { return 1e-14 * (fabs(p[0]) + fabs(p[1]) + fabs(p[2])); };
+  // n . p < d, given by a point at
+  auto half_space = [&](const double* n, double d, const double* at) {
     const double len = sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
     if (!(len > 0) || !std::isfinite(len) || !std::isfinite(d)) return false;
-    fp.push_back(FastPlane{{n[0] / len, n[1] / len, n[2] / len}, d / len - kFastMarginNm});
+    fp.push_back(FastPlane{{n[0] / len, n[1] / len, n[2] / len}, d / len - kFastMarginNm - rounding(at)});
     return true;
   };
   switch (sh.kind) {
     case SHAPE_PLANES:
       for (int i = 0; i < sh.np; ++i) {
         const Plane& p = planes[sh.plane0 + i];
-        if (!half_space(p.n, p.n[0] * p.p[0] + p.n[1] * p.p[1] + p.n[2] * p.p[2])) return false;
+        if (!half_space(p.n, p.n[0] * p.p[0] + p.n[1] * p.p[1] + p.n[2] * p.p[2], p.p)) return false;
       }
       return true;
     case SHAPE_INTERSECTION:
@@ -45,11 +51,11 @@ static bool inside_of(const std::vector<Shape>& shapes, const std::vector<Plane>
     case SHAPE_CYLINDER: {
       // only a cylinder whose axis is normalised is ever struck (see cm_shape_cylinder)
       const double u = sh.nax[0] * sh.nax[0] + sh.nax[1] * sh.nax[1] + sh.nax[2] * sh.nax[2];
-      const double rad = sqrt(sh.rad2), m = 1e-3 + 1e-9 * sh.len;
+      const double rad = sqrt(sh.rad2), m = 1e-3 + 1e-9 * sh.len + 1e-14 * sh.len2 / rad + rounding(sh.e0);
       if (!(fabs(u - 1.0) < 1e-9) || !(rad > 2 * m) || !(sh.len > 4 * m)) return false;
       const double back[3] = {-sh.nax[0], -sh.nax[1], -sh.nax[2]};
       const double a0 = sh.nax[0] * sh.e0[0] + sh.nax[1] * sh.e0[1] + sh.nax[2] * sh.e0[2];
-      if (!half_space(sh.nax, a0 + sh.len - m) || !half_space(back, -a0 - m)) return false;
+      if (!half_space(sh.nax, a0 + sh.len - m, sh.e0) || !half_space(back, -a0 - m, sh.e0)) return false;
       fc.push_back(FastCyl{{sh.e0[0], sh.e0[1], sh.e0[2]}, {sh.nax[0], sh.nax[1], sh.nax[2]}, (rad - m) * (rad - m)});
       return true;
     }

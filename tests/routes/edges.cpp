@@ -51,9 +51,115 @@ static void check_axis_ends() {
       }
 }
 
+// ---- the inside of shapes far larger than they are wide, or given by points far away: a step with both ends
+// strictly inside is one the boundary search finds no boundary for
+struct OneShape {
+  std::vector<Shape> shapes;
+  std::vector<Plane> planes;
+};
+
+static OneShape cylinder(const double* e0, const double* ax, double rad) {
+  Shape s;
+  memset(&s, 0, sizeof(s));
+  s.kind = SHAPE_CYLINDER;
+  s.len2 = ax[0] * ax[0] + ax[1] * ax[1] + ax[2] * ax[2];
+  s.len = sqrt(s.len2);
+  for (int k = 0; k < 3; ++k) {
+    s.e0[k] = e0[k];
+    s.ax[k] = ax[k];
+    s.nax[k] = ax[k] / s.len;
+  }
+  s.rad2 = rad * rad;
+  return OneShape{{s}, {}};
+}
+
+// steps from at(a point) to at(another), kept when both ends are strictly inside
+template <typename F> static void check_inside(const char* name, const OneShape& sh, F at) {
+  std::vector<FastPlane> fp;
+  std::vector<FastCyl> fc;
+  if (!inside_of(sh.shapes, sh.planes, 0, fp, fc)) return;  // not described: the full flight
+  SceneView<double> v;
+  memset(&v, 0, sizeof(v));
+  v.shapes = sh.shapes.data();
+  v.planes = sh.planes.data();
+  v.fast_planes = fp.data();
+  v.fast_cyls = fc.data();
+  const FastRegion f{0, 0, 0, (int)fp.size(), fc.empty() ? -1 : 0, {0, 0, 0}};
+  for (int k = 0; k < 200000; ++k) {
+    double p0[3], p1[3];
+    at(k, p0, p1);
+    if (!point_inside(v, f, p0) || !point_inside(v, f, p1)) continue;
+    CHECK((shape_contains<double, 0>(v, 0, p0)), "%s: start not contained", name);
+    const NV nv = shape_first_normal<double, 0>(v, 0, p0, p1);
+    CHECK(!(nv.u <= 1.0), "%s: boundary at u = %.17g", name, nv.u);
+  }
+}
+
+static void check_far_shapes() {
+  std::mt19937_64 r(11);
+  std::uniform_real_distribution<double> u(-1.0, 1.0);
+  const double dir[2][3] = {{0, 1, 0}, {0.48, 0.6, 0.64}};
+  for (double len : {1e3, 1e5, 1e6, 1e7, 1e8, 2e8})
+    for (double rad : {0.5, 2.0, 5.0, 100.0, 1e4, 1e6})
+      for (const double* n : dir) {
+        double e0[3], ax[3], side[2][3];
+        for (int a = 0; a < 3; ++a) {
+          ax[a] = len * n[a];
+          e0[a] = -0.5 * ax[a];
+          side[0][a] = a == 0 ? (n[0] > 0 ? 0.8 : 1.0) : a == 1 && n[0] > 0 ? -0.64 : 0.0;
+        }
+        const double m = sqrt(side[0][0] * side[0][0] + side[0][1] * side[0][1]), dot = side[0][0] * n[0] + side[0][1] * n[1];
+        for (int a = 0; a < 3; ++a) side[0][a] = (side[0][a] - dot * n[a]) / m;
+        for (int a = 0; a < 3; ++a)
+          side[1][a] = n[(a + 1) % 3] * side[0][(a + 2) % 3] - n[(a + 2) % 3] * side[0][(a + 1) % 3];
+        const double margin = 1e-3 + 1e-9 * len;
+        char name[64];
+        snprintf(name, sizeof(name), "cylinder %g x %g", len, rad);
+        check_inside(name, cylinder(e0, ax, rad), [&](int k, double* p0, double* p1) {
+          const double w0 = 0.5 * len * u(r), w1 = k % 2 ? w0 + 3 * rad * u(r) : 0.5 * len * u(r);
+          for (int e = 0; e < 2; ++e) {
+            // from the axis to within a few margins of the wall
+            const double rr = k % 3 ? rad - margin * (1 + 3 * fabs(u(r))) : rad * fabs(u(r)), th = 3.14159265358979 * u(r);
+            for (int a = 0; a < 3; ++a)
+              (e ? p1 : p0)[a] = n[a] * (e ? w1 : w0) + rr * (cos(th) * side[0][a] + sin(th) * side[1][a]);
+          }
+        });
+      }
+  // a slab whose planes are given by points far from it
+  for (double far : {0.0, 1e8, 1e9, 1e10, 1e12, 1e14})
+    for (int tilted = 0; tilted < 2; ++tilted) {
+      const double n[3] = {tilted ? 0.48 : 0.0, tilted ? 0.6 : 0.0, tilted ? 0.64 : 1.0};
+      const double t[3] = {tilted ? 0.8 : 1.0, 0.0, tilted ? -0.6 : 0.0};  // along the slab
+      OneShape s;
+      Shape sh;
+      memset(&sh, 0, sizeof(sh));
+      sh.kind = SHAPE_PLANES;
+      sh.np = 2;
+      s.shapes.push_back(sh);
+      for (int sg = -1; sg <= 1; sg += 2) {
+        Plane P;
+        for (int a = 0; a < 3; ++a) {
+          P.n[a] = sg * n[a];
+          P.p[a] = sg * 10 * n[a] + far * t[a];
+        }
+        s.planes.push_back(P);
+      }
+      char name[64];
+      snprintf(name, sizeof(name), "slab through points %g away", far);
+      check_inside(name, s, [&](int k, double* p0, double* p1) {
+        for (int e = 0; e < 2; ++e) {
+          const double h = k % 3 ? (10 - 3 * kFastMarginNm * fabs(u(r))) * (u(r) > 0 ? 1 : -1) : 10 * u(r);
+          const double x = 1e3 * u(r), off = far * (n[0] * t[0] + n[1] * t[1] + n[2] * t[2]);
+          for (int a = 0; a < 3; ++a) (e ? p1 : p0)[a] = n[a] * (h + off) + t[a] * x;
+        }
+      });
+    }
+}
+
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   if (what == "axis_ends") check_axis_ends();
+  else if (what == "far_shapes") check_far_shapes();
   else return 2;
   printf("%s: %ld checks, %d failures\n", what.c_str(), checks, failures);
   return failures ? 1 : 0;
