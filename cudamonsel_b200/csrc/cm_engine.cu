@@ -778,14 +778,14 @@ static int build_scene(cm_context* ctx, DevScene<R>& ds) {
     r.grid = (int)grids.size();
     grids.push_back(g);
   }
-  // what lies strictly inside each childless region (FastRegion): its shape's half-spaces and at most one
-  // cylinder; of a union one part is enough
+  // what lies strictly inside each region the fast flight serves (FastRegion): its shape's half-spaces and at
+  // most one cylinder; of a union one part is enough
   std::vector<FastRegion> fast;
   std::vector<FastPlane> fplanes;
   std::vector<FastCyl> fcyls;
   for (const Region& r : regions) {
     FastRegion f{r.msm, r.cls, (int)fplanes.size(), -1, -1, {0, 0, 0}};
-    if (r.nchild == 0 && msms[r.msm].nmech <= 4) {  // the fast flight picks among at most four mechanisms
+    if (fast_model(r, msms[r.msm])) {
       const size_t c0 = fcyls.size();
       if (inside_of(shapes, planes, r.shape, fplanes, fcyls) && fcyls.size() - c0 <= 1) {
         f.np = (int)fplanes.size() - f.plane0;

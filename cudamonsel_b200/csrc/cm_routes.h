@@ -64,6 +64,13 @@ static bool inside_of(const std::vector<Shape>& shapes, const std::vector<Plane>
   }
 }
 
+// Whether the steps of a region may take the fast flight: it has no children and its model has mechanisms,
+// at most the four the fast flight picks among.  In a region without mechanisms (vacuum) every step ends at
+// a boundary, so a fast flight would only hand it on to the next iteration's full flight.
+template <typename R> static bool fast_model(const Region& r, const Msm<R>& m) {
+  return r.nchild == 0 && m.nmech > 0 && m.nmech <= 4;
+}
+
 // The search guide of an ascending axis: linear buckets or the leading bits of the argument, whichever
 // leaves at most one node in every bucket of at most 4096; kind 0 (bisection) when neither does.
 static AxisGuide make_guide(const double* x, int n, std::vector<GuideEntry>& out) {

@@ -156,10 +156,25 @@ static void check_far_shapes() {
     }
 }
 
+// ---- which regions take the fast flight: childless ones whose model has one to four mechanisms
+static void check_fast_models() {
+  for (int nmech = 0; nmech <= kMaxMech; ++nmech)
+    for (int nchild = 0; nchild < 3; ++nchild) {
+      Region r;
+      Msm<float> m;
+      memset(&r, 0, sizeof(r));
+      memset(&m, 0, sizeof(m));
+      r.nchild = nchild;
+      m.nmech = nmech;
+      CHECK(fast_model(r, m) == (nchild == 0 && nmech >= 1 && nmech <= 4), "%d mechanisms, %d children", nmech, nchild);
+    }
+}
+
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   if (what == "axis_ends") check_axis_ends();
   else if (what == "far_shapes") check_far_shapes();
+  else if (what == "fast_models") check_fast_models();
   else return 2;
   printf("%s: %ld checks, %d failures\n", what.c_str(), checks, failures);
   return failures ? 1 : 0;

@@ -35,3 +35,43 @@ def test_tables_beyond_an_axis_that_ends_below_zero(prec):
     for k in range(4):
         assert abs(got2[k] - cubic(a[-4:], v2[-4:, 4], xs[k])) < tol
         assert abs(got3[k] - cubic(a[-4:], v3[-4:, 4, 3], xs[k])) < tol
+
+
+@pytest.mark.parametrize("prec", [FP64, FP32], ids=["fp64", "fp32"])
+def test_vacuum_steps_take_one_iteration(prec):
+    """A primary that starts inside a vacuum box and flies through a stack of them takes one step per wall, and
+    each step one iteration of the queue kernels: as many iterations whether or not the boxes have children
+    (a region with children takes the full flight), one more than steps for the start.  The resident-steps
+    kernel gives the same tallies."""
+    from cudamonsel_b200 import capi, scenes
+
+    def box(s, c, h):
+        n, p = [], []
+        for a in range(3):
+            for sg in (-1.0, 1.0):
+                n += [sg * (a == k) for k in range(3)]
+                p += [c[k] + sg * h[k] * (a == k) for k in range(3)]
+        return s.planes(n, p)
+
+    def run(children, options):
+        s = scenes.SceneSpec()
+        vac = scenes.vacuum(s)
+        ch = s.region(None, vac, s.sphere([0.0, 0.0, 0.0], 0.1))
+        for k in range(8):
+            r = s.region(ch, vac, box(s, [0.0, 0.0, 40e-9 * k], [50e-9, 50e-9, 10e-9]))
+            if children:  # a child that the beam misses
+                s.region(r, vac, box(s, [45e-9, 45e-9, 40e-9 * k], [1e-9, 1e-9, 1e-9]))
+        e = capi.Engine(0)
+        h = scenes.replay(s, scenes.EngineBackend(e))
+        e.set_options(options)
+        b, f, st = e.run(h[ch.idx], np.array([[0.0, 0.0, 1e-9]]), scenes.eV(500.0), 1, 50, 0.0, 3, precision=prec)
+        e.close()
+        return b, f, st
+
+    b0, f0, s0 = run(False, capi.OPT_QUEUE_STEPS)
+    b1, f1, s1 = run(True, capi.OPT_QUEUE_STEPS)
+    b2, f2, s2 = run(False, 0)
+    print("steps %d, iterations %d, with children %d" % (s0.steps, s0.iterations, s1.iterations))
+    assert s0.steps == s1.steps == s2.steps and s0.escapes == 1 and s0.steps == 16
+    assert s0.iterations == s1.iterations == s0.steps + 1
+    assert np.array_equal(b0, b1) and np.array_equal(f0, f1) and np.array_equal(b0, b2) and np.array_equal(f0, f2)
