@@ -134,7 +134,7 @@ __device__ __forceinline__ void block_task(const RunView<R>& v, int l, int slot,
     bool alive;
     dest = kListDead;
     if (l <= kListOpen) {
-      const int q = l >= kListSlow ? flight_apply<R, D>(v, e, sink, sc) : flight_fast(v, e, sc, [](El<R>&) {});
+      const int q = l >= kListSlow ? flight_apply<R, D>(v, e, sink, sc) : flight_fast(v, e, sink, sc, [](El<R>&) {});
       alive = q >= 0;
       if (q == Q_EL) alive = elastic_apply(v, e);
       if (q == Q_SLOW) {

@@ -459,7 +459,8 @@ CM_D int flight_apply(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc,
 // them (flight_apply then takes it from the start: the random stream is keyed by the step).  e holds the
 // energy, step, key and region; rest(e) reads the position and direction, which the rates do not need
 // (read with the others they would spill).
-template <typename R, typename Rest> CM_D int flight_fast(const RunView<R>& v, El<R>& e, StepCounts& sc, Rest rest) {
+template <typename R, typename Sink, typename Rest>
+CM_D int flight_fast(const RunView<R>& v, El<R>& e, Sink& sink, StepCounts& sc, Rest rest) {
   const SceneView<R>& s = v.s;
   const FastRegion f = s.fast[e.region];
   const Msm<R>& m = s.msms[f.msm];
@@ -491,7 +492,13 @@ template <typename R, typename Rest> CM_D int flight_fast(const RunView<R>& v, E
   const int kind = (m.kinds >> (4 * idx)) & 15;
   if (kind == MECH_POLARON) return -1;  // GanachaudMokraniPolaronTrapSM::scatter: trapped, E = 0
   e.aux = aux_pack(AUX_MECH, idx) | AUX_INSIDE;
-  return kind == MECH_NISTMOTT ? Q_EL : kind == MECH_TABULATED ? Q_TAB : Q_MISC;
+  const int queue = kind == MECH_NISTMOTT ? Q_EL : kind == MECH_TABULATED ? Q_TAB : Q_MISC;
+#ifdef CM_TRACE
+  cm_trace(v, e, e.region, queue * 100 + aux_kind(e.aux) * 10 + aux_val(e.aux) % 10, sink);
+#else
+  (void)sink;
+#endif
+  return queue;
 }
 
 // append an electron to segment k of the next wave
@@ -518,7 +525,7 @@ CM_D int flight_one(const RunView<R>& v, int i, Sink& sink, StepCounts& sc) {
   };
   int queue;
   if (FAST) {
-    queue = flight_fast(v, e, sc, rest);
+    queue = flight_fast(v, e, sink, sc, rest);
   } else {
     rest(e);
     queue = flight_apply<R, D>(v, e, sink, sc, &w.pixel());  // the pixel is read only on escape

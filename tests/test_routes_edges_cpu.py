@@ -21,3 +21,13 @@ def test_short_routes_at_the_ends_of_their_ranges(edges, what):
     r = subprocess.run([edges, what], capture_output=True, text=True, timeout=300)
     print(r.stdout)
     assert r.returncode == 0, r.stdout
+
+
+def test_fast_flights_are_recorded_like_full_ones(tmp_path):
+    """tests/routes/trace.cpp: the build that records steps (CM_TRACE)."""
+    exe = str(tmp_path / "trace")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-w", "-I", os.path.join(ROOT, "cudamonsel_b200", "csrc"),
+                    "-o", exe, os.path.join(HERE, "routes", "trace.cpp")], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
+    print(r.stdout)
+    assert r.returncode == 0, r.stdout
