@@ -1291,7 +1291,7 @@ CM_D int find_end_of_step(const SceneView<R>& s, int reg, const double* p0, doub
       tlo = fmax(tlo, fmin(u, w));
       thi = fmin(thi, fmax(u, w));
     }
-    if (ex == 0.0) hit = p0[0] >= g.x0 && p0[0] <= X1;
+    if (ex == 0.0) hit = hit && p0[0] >= g.x0 && p0[0] <= X1;
     else {
       double a0 = (g.x0 - p0[0]) / ex, a1 = (X1 - p0[0]) / ex;
       if (a0 > a1) { const double q = a0; a0 = a1; a1 = q; }

@@ -730,51 +730,8 @@ static int build_scene(cm_context* ctx, DevScene<R>& ds) {
   std::vector<ChildGrid> grids;
   std::vector<int> cell_start, grid_items;
   for (Region& r : regions) {
-    if (r.nchild < kGridMinChildren || (ctx->options & CM_OPT_SCAN_CHILDREN)) continue;
-    std::vector<int> bounded, unbounded;
-    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int i = 0; i < r.nchild; ++i) {
-      const double* bb = regions[children[r.child0 + i]].bb;
-      if (std::isinf(bb[0]) || std::isinf(bb[1]) || std::isinf(bb[3]) || std::isinf(bb[4]) || bb[0] > bb[3] ||
-          bb[1] > bb[4]) {
-        unbounded.push_back(i);
-        continue;
-      }
-      bounded.push_back(i);
-      for (int a = 0; a < 3; ++a) {
-        lo[a] = std::min(lo[a], bb[a]);
-        hi[a] = std::max(hi[a], bb[3 + a]);
-      }
-    }
-    if ((int)bounded.size() < kGridMinChildren) continue;
     ChildGrid g;
-    const double wx = std::max(hi[0] - lo[0], 1e-3), wy = std::max(hi[1] - lo[1], 1e-3);
-    const double cells = std::min(65536.0, std::max(16.0, 2.0 * bounded.size()));
-    g.nx = std::max(1, std::min(4096, (int)ceil(sqrt(cells * wx / wy))));
-    g.ny = std::max(1, std::min(4096, (int)ceil(cells / g.nx)));
-    g.x0 = lo[0];
-    g.y0 = lo[1];
-    g.dx = wx / g.nx;
-    g.dy = wy / g.ny;
-    g.z0 = lo[2];
-    g.z1 = hi[2];
-    std::vector<std::vector<int>> lists((size_t)g.nx * g.ny);
-    for (int i : bounded) {  // ascending positions, so every cell list is ascending
-      const double* bb = regions[children[r.child0 + i]].bb;
-      const int ix0 = std::max(0, (int)floor((bb[0] - g.x0) / g.dx)), ix1 = std::min(g.nx - 1, (int)floor((bb[3] - g.x0) / g.dx));
-      const int iy0 = std::max(0, (int)floor((bb[1] - g.y0) / g.dy)), iy1 = std::min(g.ny - 1, (int)floor((bb[4] - g.y0) / g.dy));
-      for (int iy = iy0; iy <= iy1; ++iy)
-        for (int ix = ix0; ix <= ix1; ++ix) lists[(size_t)iy * g.nx + ix].push_back(i);
-    }
-    g.cell0 = (int)cell_start.size();
-    for (auto& l : lists) {
-      cell_start.push_back((int)grid_items.size());
-      grid_items.insert(grid_items.end(), l.begin(), l.end());
-    }
-    cell_start.push_back((int)grid_items.size());
-    g.unb0 = (int)grid_items.size();
-    g.nunb = (int)unbounded.size();
-    grid_items.insert(grid_items.end(), unbounded.begin(), unbounded.end());
+    if ((ctx->options & CM_OPT_SCAN_CHILDREN) || !child_grid(regions, children, r, g, cell_start, grid_items)) continue;
     r.grid = (int)grids.size();
     grids.push_back(g);
   }

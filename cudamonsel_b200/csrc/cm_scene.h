@@ -59,11 +59,11 @@ struct ChildGrid {
   int unb0, nunb;         // the unbounded children: grid_items[unb0 .. unb0 + nunb)
 };
 
-// The part of a childless region of a model with mechanisms that lies strictly inside its shape, as half-spaces (FastPlane) and at
-// most one cylinder wall.  A step whose two ends are both in there meets no boundary, and the region test
-// and the boundary search need not run: kFastMarginNm is far above the rounding of either evaluation (at
-// most ~1e-6 nm for coordinates below 1e9 nm; shapes given by larger ones keep a wider margin, see
-// inside_of), so both decide alike.
+// The part of a region that lies strictly inside its shape, for the childless regions of models with
+// mechanisms, as half-spaces (FastPlane) and at most one cylinder wall.  A step whose two ends are both in
+// there meets no boundary, and the region test and the boundary search need not run: kFastMarginNm is far
+// above the rounding of either evaluation (at most ~1e-6 nm for coordinates below 1e9 nm; shapes given by
+// larger ones keep a wider margin, see inside_of), so both decide alike.
 struct alignas(16) FastRegion {
   int msm, cls;          // as the Region's
   int plane0, np;        // half-spaces fast_planes[plane0, plane0 + np); np < 0: no such description

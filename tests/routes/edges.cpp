@@ -170,11 +170,141 @@ static void check_fast_models() {
     }
 }
 
+// ---- the walk through a child grid
+struct GridScene {
+  std::vector<Shape> shapes;
+  std::vector<Plane> planes;
+  std::vector<Region> regions;
+  std::vector<int> children, cell_start, grid_items;
+  std::vector<ChildGrid> grids;
+  SceneView<double> v;
+
+  int region(int parent, const Shape& sh, const double* lo, const double* hi) {
+    Region r;
+    memset(&r, 0, sizeof(r));
+    r.parent = parent;
+    r.shape = (int)shapes.size();
+    r.grid = -1;
+    for (int a = 0; a < 3; ++a) {
+      r.bb[a] = lo[a] - 1e-3;
+      r.bb[3 + a] = hi[a] + 1e-3;
+    }
+    shapes.push_back(sh);
+    regions.push_back(r);
+    return (int)regions.size() - 1;
+  }
+  GridScene() {  // the chamber
+    Shape s;
+    memset(&s, 0, sizeof(s));
+    s.kind = SHAPE_SPHERE;
+    s.r = 1e8;
+    const double lo[3] = {-1e8, -1e8, -1e8}, hi[3] = {1e8, 1e8, 1e8};
+    region(-1, s, lo, hi);
+  }
+  void box(const double* lo, const double* hi) {
+    Shape s;
+    memset(&s, 0, sizeof(s));
+    s.kind = SHAPE_PLANES;
+    s.plane0 = (int)planes.size();
+    s.np = 6;
+    for (int a = 0; a < 3; ++a)
+      for (int k = 0; k < 2; ++k) {
+        Plane P{{0, 0, 0}, {0, 0, 0}};
+        P.n[a] = k ? 1 : -1;
+        P.p[a] = k ? hi[a] : lo[a];
+        planes.push_back(P);
+      }
+    children.push_back(region(0, s, lo, hi));
+  }
+  // the chamber's grid; its cells list the children by their boxes
+  ChildGrid& finish() {
+    regions[0].nchild = (int)children.size();
+    ChildGrid g;
+    CHECK(child_grid(regions, children, regions[0], g, cell_start, grid_items), "no grid over %zu children", children.size());
+    grids.push_back(g);
+    regions[0].grid = 0;
+    memset(&v, 0, sizeof(v));
+    v.shapes = shapes.data();
+    v.planes = planes.data();
+    v.regions = regions.data();
+    v.children = children.data();
+    v.grids = grids.data();
+    v.cell_start = cell_start.data();
+    v.grid_items = grid_items.data();
+    return grids[0];
+  }
+};
+
+static void check_grid_walk() {
+  std::mt19937_64 r(29);
+  std::uniform_real_distribution<double> u(-1.0, 1.0);
+  GridScene s;
+  for (int k = 0; k < 90; ++k) {  // boxes of unlike sizes, some of them overlapping, in a layer of 300 nm
+    double lo[3], hi[3];
+    for (int a = 0; a < 3; ++a) {
+      const double c = (a == 2 ? 100 : 500) * u(r), w = (a == 2 ? 50 : 40) * fabs(u(r)) + 0.5;
+      lo[a] = c - w;
+      hi[a] = c + w;
+    }
+    s.box(lo, hi);
+  }
+  const ChildGrid g = s.finish();
+  long hits = 0, down = 0;
+  for (int k = 0; k < 400000; ++k) {
+    double p0[3], d[3];
+    for (int a = 0; a < 3; ++a) {
+      p0[a] = (a == 2 ? 300 : 600) * u(r);
+      d[a] = u(r);
+    }
+    const double len = k % 4 == 0 ? 2e8 : k % 4 == 1 ? 1000 * fabs(u(r)) : k % 4 == 2 ? 5 * fabs(u(r)) : 300;
+    if (k % 5 < 3) d[k % 5] = 0;              // within a plane across an axis
+    if (k % 7 < 3) d[(k + 1) % 3] = d[(k + 2) % 3] = 0;  // along an axis
+    if (k % 11 == 0) p0[0] = g.x0 + g.dx * (int)(g.nx * fabs(u(r)));  // on a cell's border
+    if (k % 13 == 0) p0[2] = k % 2 ? g.z0 : g.z1;             // on the layer's
+    double a1[3], b1[3], an[3], bn[3];
+    bool ac = false, bc = false;
+    for (int a = 0; a < 3; ++a) a1[a] = b1[a] = p0[a] + len * d[a];
+    down += d[0] == 0 && d[1] == 0 && d[2] != 0;
+    s.regions[0].grid = 0;
+    const int ra = find_end_of_step<double, 0>(s.v, 0, p0, a1, an, &ac);
+    s.regions[0].grid = -1;
+    const int rb = find_end_of_step<double, 0>(s.v, 0, p0, b1, bn, &bc);
+    hits += rb > 0;
+    CHECK(ra == rb && ac == bc && !memcmp(a1, b1, sizeof(a1)) && (!ac || !memcmp(an, bn, sizeof(an))),
+          "step %d from %g %g %g: region %d through the grid, %d by the scan", k, p0[0], p0[1], p0[2], ra, rb);
+  }
+  CHECK(hits > 10000 && down > 10000, "only %ld hits, %ld steps straight down", hits, down);
+}
+
+// a step that stays out of the children's layer visits no cell: a child put outside the layer that the grid
+// states is struck only by steps that do visit its cell
+static void check_grid_layer() {
+  GridScene s;
+  for (int iy = 0; iy < 6; ++iy)
+    for (int ix = 0; ix < 6; ++ix) {
+      const double lo[3] = {20.0 * ix, 20.0 * iy, 20}, hi[3] = {20.0 * ix + 15, 20.0 * iy + 15, 30};
+      s.box(lo, hi);
+    }
+  ChildGrid& g = s.finish();
+  g.z0 = 0;
+  g.z1 = 10;
+  for (double ex : {0.0, 1e-3, 2.0})
+    for (double ey : {0.0, 1e-3, 2.0})
+      for (int layer = 0; layer < 2; ++layer) {
+        const double p0[3] = {42, 42, layer ? 5.0 : 15.0};
+        double p1[3] = {p0[0] + ex, p0[1] + ey, 28}, n[3];
+        const int reg = find_end_of_step<double, 0>(s.v, 0, p0, p1, n);
+        CHECK((reg > 0) == (layer == 1), "ex %g ey %g from z %g: region %d", ex, ey, p0[2], reg);
+      }
+}
+
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   if (what == "axis_ends") check_axis_ends();
   else if (what == "far_shapes") check_far_shapes();
   else if (what == "fast_models") check_fast_models();
+  else if (what == "grid_walk") check_grid_walk();
+  else if (what == "grid_layer") check_grid_layer();
   else return 2;
   printf("%s: %ld checks, %d failures\n", what.c_str(), checks, failures);
   return failures ? 1 : 0;

@@ -16,7 +16,7 @@ def edges(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["axis_ends", "far_shapes", "fast_models"])
+@pytest.mark.parametrize("what", ["axis_ends", "far_shapes", "fast_models", "grid_walk", "grid_layer"])
 def test_short_routes_at_the_ends_of_their_ranges(edges, what):
     r = subprocess.run([edges, what], capture_output=True, text=True, timeout=300)
     print(r.stdout)
