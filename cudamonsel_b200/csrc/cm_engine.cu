@@ -3066,6 +3066,9 @@ static int run_noalloc(cm_context* ctx, const cm_run_desc* d, uint32_t* back, ui
   // iterations (the queue kernels') or wants the queue kernels; a pool overflow there, where a launch takes
   // many steps before the refill empties the pool, repeats the run with them.
   bool blocks = d->max_iterations <= 0 && !(ctx->options & CM_OPT_QUEUE_STEPS);
+  // the time, launches and electrons of an attempt given up
+  double ms = 0;
+  int64_t given_up = 0, given_up_units = 0;
 again:
   CM_CUDA(cudaMemsetAsync(c, 0, sizeof(Counters), s));
   CM_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), s));
@@ -3110,6 +3113,9 @@ again:
     CM_CUDA(cudaStreamSynchronize(s));
     if (hc.error == CM_EOVERFLOW && blocks) {
       blocks = false;
+      ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+      given_up = it;
+      given_up_units = (int64_t)hc.step_units;
       goto again;
     }
     if (hc.error) {
@@ -3129,7 +3135,7 @@ again:
       break;
     }
   }
-  const double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+  ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   if (st) {
     memset(st, 0, sizeof(*st));
     st->primaries = (int64_t)hc.next_primary;
@@ -3142,9 +3148,11 @@ again:
     st->device_ms = ms;
     st->ended_zero_energy = (int64_t)hc.ended_zero;
     st->ended_step_limit = (int64_t)hc.ended_limit;
-    for (int k = 0; k < 6; ++k) st->kernel_launches[k] = k == CM_K_TAIL || (blocks && k < 4) ? 0 : it;
-    st->step_launches = blocks ? it : 0;
-    st->step_units = (int64_t)hc.step_units;
+    for (int k = 0; k < 6; ++k)
+      st->kernel_launches[k] = k == CM_K_TAIL || (blocks && k < 4) ? 0 : it + (k == CM_K_SPAWN ? given_up : 0);
+    st->step_launches = blocks ? it : given_up;
+    st->step_units = (int64_t)hc.step_units + given_up_units;
+    st->pool_restarts = given_up > 0;
     for (int k = 0; k < 4; ++k) st->units[k] = (int64_t)hc.units[k];
   }
   return status;

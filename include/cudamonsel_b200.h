@@ -232,8 +232,9 @@ typedef struct {
   int64_t ended_step_limit;    /* electrons ended by the reference's 10^6-step limit
                                   (MONSEL_MaterialScatterModel.cu:86-90) */
   int64_t pool_restarts;       /* times the run (a job: its batch) overflowed the secondary pool and was
-                                  run again from its start with twice the pool; the tallies are those of
-                                  a run with a large enough pool */
+                                  run again from its start with twice the pool (cm_run_noalloc, whose pool
+                                  is fixed: once, with the queue kernels, which need less of it); the
+                                  tallies are those of a run with a large enough pool */
 } cm_run_stats;
 
 /* back/fwd: [npix * hist_stride] counts, index = histogram bin + 1 (0 = underflow,
@@ -261,8 +262,9 @@ int cm_autotune(cm_context* ctx, const cm_run_desc* desc, cm_tuning* best);
  * arguments, same tallies as cm_run_device (stream 0 = the legacy default
  * stream; stats->kernel_ms stays zero).  Limits: npix <= 65536; the wave is
  * capped by the scratch (about 17 k electrons in FP32, 12 k in FP64), so a run
- * whose secondaries overflow the fixed pool returns CM_EOVERFLOW instead of
- * growing it.  The scene must already be on the device for desc->precision
+ * whose secondaries overflow the fixed pool is run again with the queue kernels
+ * (stats->pool_restarts 1; device_ms and the launches count both runs) and
+ * returns CM_EOVERFLOW when they overflow it too, instead of growing it.  The scene must already be on the device for desc->precision
  * (uploading it allocates): after the last scene change, make one cm_run,
  * cm_run_device or cm_eval_* call with that precision first, else CM_ESTATE.
  * The first call on a device looks up the array's device address; make that
