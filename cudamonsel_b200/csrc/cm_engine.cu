@@ -1100,7 +1100,7 @@ namespace cm {
 // shape trees enters the tail at half as many electrons: k_block's tree walks spill at its 128 registers
 // (one B200, 131072 against 262144: rounded features 66.5 / 69.4 ms, FP64 line scan 34.8 / 37.0 ms, FP64
 // image 111.5 / 110.7 ms; leaf scenes: FP32 line scan 46.3 / 45.3 ms, deep 131.9 / 126.1 ms).
-template <typename R> static cm_tuning resolved_tuning(const cm_context* ctx, int depth = 0) {
+template <typename R> static cm_tuning resolved_tuning(const cm_context* ctx, int depth) {
   cm_tuning t = ctx->tune[sizeof(R) == 8 ? CM_PREC_FP64 : CM_PREC_FP32];
   if (t.wave <= 0) t.wave = 1 << 21;
   if (t.tail_below <= 0) t.tail_below = depth > 0 ? CM_TAIL_BELOW / 2 : CM_TAIL_BELOW;
@@ -2666,6 +2666,14 @@ int cm_run_device(cm_context* ctx, const cm_run_desc* d, uint32_t* back, uint32_
   return rc;
 }
 
+static int scene_for(cm_context* ctx, int precision) {
+  if (!ctx) return fail(CM_EINVAL, "null context");
+  CM_CUDA(cudaSetDevice(ctx->device));
+  if (precision == CM_PREC_FP64) return build_scene<double>(ctx, ctx->d64);
+  if (precision == CM_PREC_FP32) return build_scene<float>(ctx, ctx->d32);
+  return fail(CM_EINVAL, "bad precision");
+}
+
 // Coordinate descent over the launch settings from the defaults, one cm_run per candidate.
 int cm_autotune(cm_context* ctx, const cm_run_desc* d, cm_tuning* best) {
   int rc = check_desc(ctx, d);
@@ -2689,13 +2697,16 @@ int cm_autotune(cm_context* ctx, const cm_run_desc* d, cm_tuning* best) {
     ms = st.device_ms;
     return r;
   };
-  cm_tuning cur = d->precision == CM_PREC_FP64 ? cm::resolved_tuning<double>(ctx) : cm::resolved_tuning<float>(ctx);
+  // from the settings an untuned run of this scene would use
+  if ((rc = scene_for(ctx, d->precision))) return rc;
+  cm_tuning cur = d->precision == CM_PREC_FP64 ? cm::resolved_tuning<double>(ctx, ctx->d64.view.depth)
+                                               : cm::resolved_tuning<float>(ctx, ctx->d32.view.depth);
   double cur_ms = 0, ms = 0;
-  if ((rc = trial(cur, cur_ms)) || (rc = trial(cur, cur_ms))) {  // the first run also builds the scene
+  if ((rc = trial(cur, cur_ms)) || (rc = trial(cur, cur_ms))) {  // the first run warms up
     slot = saved;
     return rc;
   }
-  const int belows[] = {65536, 131072, 524288};
+  const int belows[] = {65536, 131072, 262144, 524288};
   const int steps[] = {32, 128};
   auto sweep = [&](int cm_tuning::*field, const int* vals, int n) -> int {
     for (int k = 0; k < n; ++k) {
@@ -2718,7 +2729,7 @@ int cm_autotune(cm_context* ctx, const cm_run_desc* d, cm_tuning* best) {
     const cm_tuning before = cur;
     const int waves[] = {std::max(1024, cur.wave / 2), std::min(1 << 24, cur.wave * 2)};
     const int blocks[] = {std::max(2, cur.blocks_per_sm / 2), std::min(32, cur.blocks_per_sm * 2)};
-    if ((rc = sweep(&cm_tuning::wave, waves, 2)) || (rc = sweep(&cm_tuning::tail_below, belows, 3)) ||
+    if ((rc = sweep(&cm_tuning::wave, waves, 2)) || (rc = sweep(&cm_tuning::tail_below, belows, 4)) ||
         (rc = sweep(&cm_tuning::tail_steps, steps, 2)) || (rc = sweep(&cm_tuning::blocks_per_sm, blocks, 2))) {
       slot = saved;
       return rc;
@@ -2757,14 +2768,6 @@ static int eval_launch(cm_context* ctx, int n, const double* in, size_t in_per, 
   return 0;
 }
 
-}
-
-static int scene_for(cm_context* ctx, int precision) {
-  if (!ctx) return fail(CM_EINVAL, "null context");
-  CM_CUDA(cudaSetDevice(ctx->device));
-  if (precision == CM_PREC_FP64) return build_scene<double>(ctx, ctx->d64);
-  if (precision == CM_PREC_FP32) return build_scene<float>(ctx, ctx->d32);
-  return fail(CM_EINVAL, "bad precision");
 }
 
 static int mech_index(cm_context* ctx, int msm, int mech, int kind) {

@@ -75,3 +75,26 @@ def test_vacuum_steps_take_one_iteration(prec):
     assert s0.steps == s1.steps == s2.steps and s0.escapes == 1 and s0.steps == 16
     assert s0.iterations == s1.iterations == s0.steps + 1
     assert np.array_equal(b0, b1) and np.array_equal(f0, f1) and np.array_equal(b0, b2) and np.array_equal(f0, f2)
+
+
+@pytest.mark.parametrize("prec", [FP64, FP32], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("scene,below", [("features", 131072), ("halfspace", 262144)])
+def test_autotuner_starts_from_the_scene_s_own_settings(scene, below, prec):
+    """cm_autotune starts from the settings an untuned run of the scene would use; a scene with shape trees
+    enters the tail at half as many electrons.  Under CM_OPT_QUEUE_STEPS the tail settings change nothing, so
+    the tuner keeps that start unless two runs of one kind differ by its 1 % (three tries)."""
+    from cudamonsel_b200 import capi, scenes
+    sc = scenes.features() if scene == "features" else scenes.halfspace()
+    got = []
+    for _ in range(3):
+        e = capi.Engine(0)
+        h = scenes.build_engine(sc, e)
+        e.set_options(capi.OPT_QUEUE_STEPS | sc.spec.options)
+        t = e.autotune(h["chamber"], scenes.linescan_pixels(64), scenes.eV(500.0), 300 if prec == FP32 else 100, 50,
+                       1e-9, 9, precision=prec)
+        e.close()
+        got.append((t.tail_below, round(t.ms, 2)))
+        if t.tail_below == below:
+            break
+    print(scene, got)
+    assert got[-1][0] == below
