@@ -340,11 +340,12 @@ def main():
     d2h = 2 * NPIX * stride * 4
 
     steps_total = sum(s.steps for s in stats)
-    # the queue kernels, spawn and loop kernel of every iteration, the tail kernel, and the run's two gates
+    # the five queue kernels of an iteration (two flights, three kinds of events), the refill that ends every
+    # iteration, the resident-steps kernel, and the run's two gates
     launches = sum(sum(int(x) for x in s.kernel_launches) + int(s.step_launches) + 2 for s in stats)
     # roofline of the dominant kernel: one more step of the same workload with CUDA events
     # between the kernels of every iteration (event nodes inside the captured graphs); the tail
-    # iterations run k_block ("steps" in the shares), the others the six queue kernels
+    # iterations run k_block ("steps" in the shares), the others the queue kernels
     flush.zero_()
     prof = [step(prec, profile=1)]
     torch.cuda.synchronize()
@@ -357,7 +358,8 @@ def main():
         step_ms += s.step_ms
     names = capi.RunStats.KERNELS
     dom = int(np.argmax(kms[:4]))
-    nlaunch = sum(int(s.kernel_launches[dom]) for s in prof)
+    # (the two flights of an iteration share its electrons and are timed as one)
+    nlaunch = sum(int(s.kernel_launches[dom]) for s in prof) // (2 if names[dom] == "flight" else 1)
     per_launch_units = units[dom] / max(1, nlaunch)
     avg_ms = kms[dom] / max(1, nlaunch)
     achieved = units[dom] * BYTES_PER_STEP / (kms[dom] / 1000.0) / 1e9

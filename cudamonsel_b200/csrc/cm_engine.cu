@@ -1679,8 +1679,8 @@ static int run_device_once(cm_context* ctx, const cm_run_desc* d, uint32_t* back
     st->device_ms = ms;
     for (int k = 0; k < 6; ++k) {
       st->kernel_ms[k] = kms[k];
-      // (the end of an iteration, CM_K_TAIL, is the last block of the refill's)
-      st->kernel_launches[k] = (int64_t)(k == CM_K_TAIL ? 0 : k < 4 ? qslots : qslots + tslots);
+      // (the end of an iteration, CM_K_TAIL, is the last block of the refill's; the flights are two kernels)
+      st->kernel_launches[k] = (int64_t)(k == CM_K_TAIL ? 0 : k == CM_K_FLIGHT ? 2 * qslots : k < 4 ? qslots : qslots + tslots);
     }
     for (int k = 0; k < 4; ++k) st->units[k] = (int64_t)c.units[k];
     st->step_launches = tslots;
@@ -3152,7 +3152,10 @@ again:
     st->ended_zero_energy = (int64_t)hc.ended_zero;
     st->ended_step_limit = (int64_t)hc.ended_limit;
     for (int k = 0; k < 6; ++k)
-      st->kernel_launches[k] = k == CM_K_TAIL || (blocks && k < 4) ? 0 : it + (k == CM_K_SPAWN ? given_up : 0);
+      st->kernel_launches[k] = k == CM_K_TAIL || (blocks && k < 4) ? 0
+                               : k == CM_K_FLIGHT                  ? 2 * it
+                               : k == CM_K_SPAWN                   ? it + given_up
+                                                                   : it;
     st->step_launches = blocks ? it : given_up;
     st->step_units = (int64_t)hc.step_units + given_up_units;
     st->pool_restarts = given_up > 0;

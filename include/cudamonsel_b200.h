@@ -220,7 +220,7 @@ typedef struct {
   int64_t primaries, steps, scatter_events, barrier_events, escapes, secondaries, iterations;
   double device_ms;            /* time of the transport loop on the device */
   double kernel_ms[6];         /* per kernel, summed over launches (profile != 0 only) */
-  int64_t kernel_launches[6];
+  int64_t kernel_launches[6];  /* CM_K_FLIGHT: the fast and the full flight of every iteration, two launches */
   int64_t units[4];            /* electrons handled by flight, elastic, inelastic, misc */
   int64_t step_launches;       /* launches of the resident-steps kernel (k_block) that runs the tail of a
                                   run (when fewer electrons are left than fill the GPU); the queue kernels

@@ -98,3 +98,19 @@ def test_autotuner_starts_from_the_scene_s_own_settings(scene, below, prec):
             break
     print(scene, got)
     assert got[-1][0] == below
+
+
+@pytest.mark.parametrize("profile", [0, 1])
+def test_launch_counts_hold_both_flights(profile):
+    """An iteration of the queue kernels launches the fast and the full flight, three event kernels and the
+    refill; a tail iteration the resident-steps kernel and the refill."""
+    from cudamonsel_b200 import capi, scenes
+    e = capi.Engine(0)
+    h = scenes.build_engine(scenes.lines(), e)
+    _, _, st = e.run(h["chamber"], scenes.linescan_pixels(64), scenes.eV(500.0), 1000, 50, 1e-9, seed=9,
+                     precision=FP32, profile=profile)
+    e.close()
+    n = list(st.kernel_launches)
+    print(n, st.step_launches)
+    assert n[1] > 0 and n[1] == n[2] == n[3] and n[0] == 2 * n[1]
+    assert n[4] == n[1] + st.step_launches and n[5] == 0

@@ -45,9 +45,10 @@ def test_noalloc_overflow_is_repeated_and_reported(prec):
     rc2, s2, b2, f2 = call(e.L.cm_run_noalloc, 1000.0, 100)
     e.close()
     print("overflow: restarts %d, resident-steps launches %d, queue launches %d, %.1f ms" % (
-        s1.pool_restarts, s1.step_launches, s1.kernel_launches[0], s1.device_ms))
+        s1.pool_restarts, s1.step_launches, s1.kernel_launches[1], s1.device_ms))
     assert rc0 == 0 and rc1 == capi.EOVERFLOW and rc2 == 0
     assert s1.pool_restarts == 1 and s1.step_launches > 0 and s1.step_units > 0 and s1.kernel_launches[0] > 0
-    assert s1.kernel_launches[4] == s1.step_launches + s1.kernel_launches[0]
+    assert s1.kernel_launches[4] == s1.step_launches + s1.kernel_launches[1]
+    assert s1.kernel_launches[0] == 2 * s1.kernel_launches[1]
     assert s2.pool_restarts == 0 and s2.step_launches > 0 and s2.kernel_launches[0] == 0
     assert s2.steps == s0.steps and np.array_equal(b2, b0) and np.array_equal(f2, f0)
