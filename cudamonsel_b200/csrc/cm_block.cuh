@@ -13,15 +13,18 @@
 // electron per thread through whole steps, which this kernel replaced, left a warp's lanes in different
 // events (one B200: 26 M steps of a 3 keV scan with phonons 62 -> 18.7 ms, 10 k primaries of 1 keV in FP64
 // 17.3 -> 7.8 ms, the last 256 k electrons of a 500 eV line scan 12.3 -> 6.2 ms).  With the GPU full the queue
-// kernels move 5.5 G electron-steps/s and this kernel about 2 G, so they keep the full waves.
+// kernels are 2 to 3.6 times faster, so they keep the full waves (whole runs through the queue kernels and
+// their tail / through this kernel alone: FP32 line scan 44 / 144 ms, image 209 / 759, deep 120 / 223, FP64
+// line scan 32 / 63; 5.5 / 1.7 G electron-steps/s in the first).
 //
 #pragma once
 
 namespace cm {
 
-// Threads: 512 (128 registers) in FP32, 384 (168) in FP64, where 128 registers spill 430 bytes a step (one
-// B200, 384 against 512 threads: 10 k primaries FP64 7.5 / 8.1 ms, FP64 line scan 32.9 / 33.4 ms; in FP32
-// the phonon scan 19.6 / 18.8 ms, the others within 2 %).
+// Threads: 512 (128 registers) in FP32, 384 (168) in FP64, where 128 registers spill 430 bytes a step over
+// leaf shapes and 168 spill 32 (one B200, 384 against 512 threads: 10 k primaries FP64 7.5 / 8.1 ms, FP64
+// line scan 32.9 / 33.4 ms; in FP32 the phonon scan 19.6 / 18.8 ms, the others within 2 %).  Over shape trees
+// of depth 2 both still spill about 1450 bytes of stores and 1700 (FP32) or 2200 (FP64) of loads.
 #ifndef CM_BLOCK_THREADS
 #define CM_BLOCK_THREADS (sizeof(R) == 8 ? 384 : 512)
 #endif

@@ -2,19 +2,21 @@
 //
 // Replaces MonteCarloSS::runMultipleTrajectories (NISTMonte/MonteCarloSS.cu:
 // 107-231) for a batch of beam landing points.  One "wave" of live electrons
-// is kept as structure-of-arrays in HBM.  Each iteration runs
+// is kept in HBM, in tiles of 32 records.  Each iteration runs
 //
-//   flight   : region check, scatter rates, free path, boundary search, CSD
-//              loss, escape tally; classifies every electron's step end and
-//              appends it (warp-aggregated) to one event queue
+//   flight   : scatter rates, free path, CSD loss; where the step may meet a
+//              boundary also the region check, boundary search and escape
+//              tally (the fast and the full flight, two kernels); appends
+//              every electron's step end to one event queue
 //   elastic  : SelectableElasticSM/NISTMottRS events
 //   inelastic: TabulatedInelasticSM events (secondaries -> pool)
 //   misc     : barrier crossings, FittedInelSM, phonon, pass-through
-//   spawn    : refill the next wave from the secondary pool, then primaries
-//   tail     : swap counters
+//   spawn    : refill the next wave from the secondary pool, then primaries;
+//              its last block ends the iteration
 //
-// Survivors of every event kernel are appended compactly into the other wave
-// buffer, so the next flight reads fully coalesced SoA.  Every electron draws
+// Appends are block-wide: one global atomic per block and list.  Survivors of
+// every event kernel are appended compactly into their segments of the other
+// wave buffer.  Every electron draws
 // from its own Philox stream (key = primary or parent lineage, counter =
 // step), so results do not depend on scheduling or on what else is in the wave.
 #include <cooperative_groups.h>
@@ -1013,22 +1015,12 @@ template <typename R, int D> __global__ void __launch_bounds__(256, D == 0 ? 2 :
 #endif
 
 // Resident CTAs per SM the kernels are compiled for (register caps 65536 / (256 x n)); a build may set
-// them with -DCM_MINB_FLIGHT32=n and so on.  CM_MINB_INELASTIC unset: the compiler chooses.
+// them with -DCM_MINB_FLIGHT32=n and so on.
 #ifndef CM_MINB_ELASTIC
 #define CM_MINB_ELASTIC 4
 #endif
-#if defined(CM_MINB_ELASTIC)
-#define CM_LB_ELASTIC __launch_bounds__(256, CM_MINB_ELASTIC)
-#else
-#define CM_LB_ELASTIC __launch_bounds__(256)
-#endif
 #ifndef CM_MINB_INELASTIC
 #define CM_MINB_INELASTIC 2
-#endif
-#if defined(CM_MINB_INELASTIC)
-#define CM_LB_INELASTIC __launch_bounds__(256, CM_MINB_INELASTIC)
-#else
-#define CM_LB_INELASTIC __launch_bounds__(256)
 #endif
 
 // the events of a queue's n entries, survivors appended to their segments of the next wave
@@ -1048,7 +1040,7 @@ __device__ __forceinline__ void event_loop(const RunView<R>& v, int cur, int n, 
 
 // k_elastic runs at 4 CTAs per SM (64 registers, a few spills): linescan +2 %.
 template <typename R>
-__global__ void CM_LB_ELASTIC k_elastic(const __grid_constant__ RunView<R> v, int cur) {
+__global__ void __launch_bounds__(256, CM_MINB_ELASTIC) k_elastic(const __grid_constant__ RunView<R> v, int cur) {
   DeviceSink sink;
   const int n = v.c->q[Q_EL];
   if ((int)(blockIdx.x * blockDim.x) >= n || !stage_tables(v)) return;
@@ -1056,7 +1048,7 @@ __global__ void CM_LB_ELASTIC k_elastic(const __grid_constant__ RunView<R> v, in
 }
 
 template <typename R>
-__global__ void CM_LB_INELASTIC k_inelastic(const __grid_constant__ RunView<R> v, int cur) {
+__global__ void __launch_bounds__(256, CM_MINB_INELASTIC) k_inelastic(const __grid_constant__ RunView<R> v, int cur) {
   DeviceSink sink;
   StepCounts sc;
   const int n = v.c->q[Q_TAB];
@@ -1075,8 +1067,8 @@ __global__ void __launch_bounds__(256, D == 0 ? (sizeof(R) == 4 ? 4 : 3) : 2) k_
   flush_counts(v.c, sc);
 }
 
-// the kernels are compiled for the intersection nestings 0 (leaf shapes only), 2 and 4
-// smem: bytes of staged tables (v.s.nstaged elements), 0 when the view stages none
+// the full flights; like k_misc, k_spawn and k_block compiled for the intersection nestings 0 (leaf shapes
+// only), 2 and 4
 template <typename R> static void launch_flight(const RunView<R>& v, int cur, int grid, cudaStream_t s) {
   if (v.s.depth == 0) k_flight<R, 0><<<grid, 256, 0, s>>>(v, cur);
   else if (v.s.depth <= 2) k_flight<R, 2><<<grid, 256, 0, s>>>(v, cur);
@@ -1314,9 +1306,9 @@ static int pool_records(int W, double emax_eV, int factor) {
   return (int)std::min<double>(f * (double)W, (double)(1 << 30));
 }
 
-// iterations of a replayed or served round (an even number: the waves alternate), and of the bodies of the
-// device-driven loops: a body runs to its end, so the iterations after a loop's last are idle launches
-// (~3 us each), and each turn of a loop costs ~8 us
+// iterations of a profiled run's replay and of a served round of queue iterations (even numbers: the waves
+// alternate), and of the bodies of the device-driven loops: a body runs to its end, so the iterations after
+// a loop's last are idle launches (~3 us each), and each turn of a loop costs ~8 us
 constexpr int kLoopBody = 16;
 constexpr int kQueueBody = 16, kTailBody = 2;
 
@@ -1419,7 +1411,7 @@ static int build_loop_graph(cm_context* ctx, RunBuffers<R>& rb, const RunView<R>
       return bail(e, "cudaGraphConditionalHandleCreate");
   cudaGraphNode_t prev = nullptr;
   for (int loop = 0; loop < 2; ++loop) {
-    // the gate kernel, then the WHILE node whose body holds kLoopBody iterations
+    // the gate kernel, then the WHILE node whose body holds kQueueBody or kTailBody iterations
     const Counters* cp = v.c;
     cudaGraphConditionalHandle hh = h[loop];
     const RunIO* iop = v.io;
@@ -1559,8 +1551,8 @@ static int run_device_once(cm_context* ctx, const cm_run_desc* d, uint32_t* back
   c0.total_primaries = total;
   CM_CUDA(cudaMemcpyAsync(ctx->counters, &c0, sizeof(c0), cudaMemcpyHostToDevice, stream));
   const int grid = ctx->nsm * tu.blocks_per_sm;
-  // the kernels that read tables (flight, elastic, inelastic, steps) stage the blob's small-table prefix
-  // into shared memory unless CM_OPT_GLOBAL_TABLES; the others get a view without it
+  // the kernels that stage tables (CM_STAGE_KERNELS: k_inelastic) copy the blob's small-table prefix into
+  // shared memory unless CM_OPT_GLOBAL_TABLES; the others get a view without it
   v.s.nstaged = 0;
   RunView<R> vs = v;
   if (!(ctx->options & CM_OPT_GLOBAL_TABLES)) vs.s.nstaged = v.s.nstage;

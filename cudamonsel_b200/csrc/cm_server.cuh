@@ -362,8 +362,8 @@ constexpr int kTailRound = 4;
 // rounds a batch runs between two reads of its counters while its wave is full and no job waits
 constexpr int kRoundRepeats = 4;
 
-// one round of the batch: kLoopBody iterations of the queue kernels, or of the tail kernels once every
-// primary has started and fewer electrons are left than the tail threshold
+// one round of the batch: kLoopBody iterations of the queue kernels, or kTailRound of the tail kernels while
+// fewer electrons are left than the tail threshold
 template <typename R>
 static int batch_round(Batcher& b) {
   NvtxRange range("cm server round");

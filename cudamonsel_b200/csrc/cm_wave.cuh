@@ -2,8 +2,9 @@
 // work of each event kernel.
 //
 // Every function here handles one electron and is host-callable; the kernels
-// in cm_engine.cu are grid-stride loops over them with a DeviceSink that does
-// warp-aggregated appends.  Reference paths relative to
+// in cm_engine.cu are grid-stride loops over them, whose results are appended
+// to queues and segments by whole blocks (secondaries go to the pool through
+// a sink, one atomic per converged warp).  Reference paths relative to
 // CudaMONSEL/CudaMONSEL/gov/nist/.
 #pragma once
 #include "cm_physics.cuh"
@@ -219,7 +220,7 @@ struct RunView {
   const RunIO* io;
 };
 
-// per-thread event counts, reduced once per warp by the kernels
+// per-thread event counts, summed once per block by the kernels
 struct StepCounts {
   unsigned int steps = 0, scat = 0, bar = 0, esc = 0, sec = 0, zero = 0, limit = 0;
 };
