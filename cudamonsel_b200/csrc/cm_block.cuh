@@ -155,7 +155,13 @@ __device__ __forceinline__ void block_task(const RunView<R>& v, int l, int slot,
           if (aux_kind(e.aux) == AUX_BARRIER)
             for (int a = 0; a < 3; ++a) B::r(5 + a, slot) = e.h[a];
         }
-        dest = q == Q_EL ? block_list<D>(segment_after(v.s, e)) : q == Q_TAB ? kListTab : kListMisc;
+        // A step without mechanisms that stayed in its region has no event: its next flight, one iteration a
+        // step.  (An electron in a vacuum region without a far end flies on to the limit of 10^6 steps: one B200,
+        // 5.0 s through the misc list, 3.0 s so.)
+        dest = q == Q_EL ? block_list<D>(segment_after(v.s, e))
+               : q == Q_TAB ? kListTab
+               : aux_kind(e.aux) == AUX_PASS ? block_list<D>(kOpenSegment)
+                                             : kListMisc;
       }
     } else {
       e.Ep = B::r(4, slot);

@@ -114,3 +114,21 @@ def test_launch_counts_hold_both_flights(profile):
     print(n, st.step_launches)
     assert n[1] > 0 and n[1] == n[2] == n[3] and n[0] == 2 * n[1]
     assert n[4] == n[1] + st.step_launches and n[5] == 0
+
+
+def test_steps_that_stay_in_vacuum_take_one_iteration_each():
+    """An electron that enters a vacuum region without a far end flies on, staying in the region, to the
+    reference's limit of 10^6 steps: the resident-steps kernel takes it through one step per iteration (64 a
+    launch), as no such step has an event."""
+    from cudamonsel_b200 import capi, scenes
+    s = scenes.SceneSpec()
+    vac = scenes.vacuum(s)
+    ch = s.region(None, vac, s.sphere([0.0, 0.0, 0.0], 0.1))
+    s.region(ch, vac, s.planes([0.0, 0.0, -1.0], [0.0, 0.0, 0.0]))
+    e = capi.Engine(0)
+    h = scenes.replay(s, scenes.EngineBackend(e))
+    _, _, st = e.run(h[ch.idx], np.array([[0.0, 0.0, -20e-9]]), scenes.eV(500.0), 1, 50, 0.0, 3, precision=FP32)
+    e.close()
+    print("steps %d, launches %d, %.0f ms" % (st.steps, st.iterations, st.device_ms))
+    assert st.ended_step_limit == 1 and st.escapes == 0 and 1000000 < st.steps < 1000010
+    assert st.iterations < st.steps / 64 + 8
