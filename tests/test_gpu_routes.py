@@ -82,11 +82,11 @@ def test_vacuum_steps_take_one_iteration(prec):
 def test_autotuner_starts_from_the_scene_s_own_settings(scene, below, prec):
     """cm_autotune starts from the settings an untuned run of the scene would use; a scene with shape trees
     enters the tail at half as many electrons.  Under CM_OPT_QUEUE_STEPS the tail settings change nothing, so
-    the tuner keeps that start unless two runs of one kind differ by its 1 % (three tries)."""
+    the tuner keeps that start unless two runs of one kind differ by its 1 % (six tries)."""
     from cudamonsel_b200 import capi, scenes
     sc = scenes.features() if scene == "features" else scenes.halfspace()
     got = []
-    for _ in range(3):
+    for _ in range(6):
         e = capi.Engine(0)
         h = scenes.build_engine(sc, e)
         e.set_options(capi.OPT_QUEUE_STEPS | sc.spec.options)
